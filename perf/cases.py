@@ -197,3 +197,96 @@ def tolerance(case):
     room for sums in another order."""
     return {"bf16": {"rel": 1e-2, "max": 0.1}, "fp16": {"rel": 2e-3, "max": 2e-2},
             "fp32": {"rel": 5e-6, "max": 1e-4}}[case["dtype"]]
+
+
+def _tiles(case):
+    """Raster index of every tile-order token of the (T, H, W) grid, -1 for padding, and the tiles' sizes: tiles in
+    raster order, the tokens of a clipped tile packed to its front."""
+    (T, H, W), (a, b, c) = [case[n] for n in ("grid_t", "grid_h", "grid_w")], BLOCKS[case["block"]]
+    ids = torch.arange(T * H * W, device="cuda").view(T, H, W)
+    rows, sizes = [], []
+    for t in range(0, T, a):
+        for h in range(0, H, b):
+            for w in range(0, W, c):
+                live = ids[t:t + a, h:h + b, w:w + c].reshape(-1)
+                rows.append(torch.nn.functional.pad(live, (0, case["block"] - live.numel()), value=-1))
+                sizes.append(live.numel())
+    return torch.stack(rows).view(-1), torch.tensor(sizes, device="cuda")
+
+
+def _exact_slice(case, x, sizes, routes):
+    """One (batch, head) slice in float64.  ``x``: q, k, v (and gate, dout) ``[tokens, dim]`` in tile order."""
+    be, D, dtype = case["block"], case["dim"], DTYPES[case["dtype"]]
+    x = {n: t.double() for n, t in x.items()}
+    blocks, scale = sizes.numel(), 1.0 / math.sqrt(D)
+    live = torch.arange(be, device="cuda")[None, :] < sizes[:, None]
+    blocked = {n: t.reshape(blocks, be, D) for n, t in x.items()}
+    grads, pooled, share = {}, case["op"] != "routes", None
+    if pooled:
+        share = live.double() / sizes.clamp(min=1)[:, None]
+        qc, kc, vc = ((blocked[n] * share[..., None]).sum(1) for n in "qkv")
+        # the routes are those of scores in the operator's own type (rounded after the product and after the scale),
+        # equal scores to the lower block
+        rounded = ((qc.to(dtype).double() @ kc.to(dtype).double().T).to(dtype).double() * scale).to(dtype)
+        routes = rounded.float().sort(dim=-1, descending=True, stable=True).indices[:, :case["topk"]]
+        probs = (qc @ kc.T * scale).softmax(-1)
+        out_c = probs @ vc
+    out, dq, dk, dv = (torch.zeros_like(blocked["q"]) for _ in range(4))
+    step = max(1, int(3e8 / (case["topk"] * be * D * 8)))
+    for at in range(0, blocks, step):
+        sel = routes[at:at + step].long()
+        q, n = blocked["q"][at:at + step], sel.shape[0]
+        k, v = (blocked[m][sel].reshape(n, -1, D) for m in "kv")
+        s = (q @ k.transpose(1, 2) * scale).masked_fill_(~live[sel].reshape(n, 1, -1), -math.inf)
+        p = s.softmax(-1)
+        out[at:at + step] = o = p @ v
+        if case["train"]:
+            do = blocked["dout"][at:at + step]
+            ds = p * (do @ v.transpose(1, 2) - (do * o).sum(-1, keepdim=True)) * scale
+            dq[at:at + step] = ds @ k
+            dk.index_add_(0, sel.reshape(-1), (ds.transpose(1, 2) @ q).reshape(-1, be, D))
+            dv.index_add_(0, sel.reshape(-1), (p.transpose(1, 2) @ do).reshape(-1, be, D))
+    if pooled:
+        gate = blocked.get("gate", torch.ones((), device="cuda", dtype=torch.float64))
+        out = out + out_c[:, None] * gate
+        if case["train"]:
+            do_c = (blocked["dout"] * gate).sum(1)
+            ds = probs * (do_c @ vc.T - (do_c * out_c).sum(-1, keepdim=True)) * scale
+            dq += (ds @ kc)[:, None] * share[..., None]
+            dk += (ds.T @ qc)[:, None] * share[..., None]
+            dv += (probs.T @ do_c)[:, None] * share[..., None]
+            if case["gate"]:
+                grads["dgate"] = blocked["dout"] * out_c[:, None]
+    if case["train"]:
+        grads.update(dq=dq, dk=dk, dv=dv)
+    return {"out": out.reshape(-1, D), **{n: g.reshape(-1, D) for n, g in grads.items()}}
+
+
+def exact(case, seed):
+    """``run``'s outputs in float64, slice by slice; the two largest shapes would take too long."""
+    if work(case)["flops"] > 2.5e13:
+        return None
+    state = prepare(case, seed)
+    tensors = {n: t.detach() for n, t in state["tensors"].items()}
+    if case["train"]:
+        tensors["dout"] = state["dout"]
+    raster = case["op"] == "raster"
+    if raster:
+        rows, sizes = _tiles(case)
+    else:
+        sizes = state["sizes"]
+    names = ["out"] + (["dq", "dk", "dv"] + ["dgate"] * case["gate"] if case["train"] else [])
+    result = {n: torch.zeros(tensors["q"].shape, device="cuda", dtype=torch.float64) for n in names}
+    for b in range(case["batch"]):
+        for h in range(case["heads"]):
+            if raster:
+                x = {n: t[b, :, h][rows.clamp(min=0)].masked_fill_((rows < 0)[:, None], 0) for n, t in tensors.items()}
+            else:
+                x = {n: t[b, h] for n, t in tensors.items()}
+            got = _exact_slice(case, x, sizes, state["routes"][b, h] if case["op"] == "routes" else None)
+            for n, t in got.items():
+                if raster:
+                    result[n][b, rows[rows >= 0], h] = t[rows >= 0]
+                else:
+                    result[n][b, h] = t
+    return result
