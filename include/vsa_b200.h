@@ -327,10 +327,11 @@ int vsa_sparse_bwd_dkdv_sharded(const void* dout, const void* q, const void* k_s
 int vsa_gather_rows(const void* src, const int32_t* map, void* dst,
                     int64_t batch, int64_t src_rows, int64_t dst_rows, int64_t row_bytes, void* stream);
 
-/* Which kernels the fine-attention entry points run for a shape in this process (environment switches included):
- * 2 = tcgen05/TMA (bf16 or fp16, D = 128, be = 64, 128 or 256, topk*ceil(be/64) <= 1024), 1 = warp-level mma.sync
- * (bf16 or fp16, D = 64 or 128, be = 64, 128 or 256), 0 = CUDA-core kernels (everything else the reference accepts,
- * and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
+/* What the fine-attention entry points run on for a shape in this process (environment switches included):
+ * 2 = tcgen05/TMA with every option of this header (bf16 or fp16, D = 128, be = 64, 128 or 256, topk*ceil(be/64) <= 1024),
+ * 1 = tensor cores for the ordinary layout only, without shard-major K/V, raster-order stores and stored dS (bf16 or fp16,
+ * D = 64 or 128, be = 64, 128 or 256: warp-level mma.sync, or tcgen05 for D = 64 and be = 128 or 256), 0 = CUDA-core
+ * kernels (everything else the reference accepts, and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
 int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
 
 /* ---- raster-order activations: the tiling front end folded into the kernels --------------------------------

@@ -46,6 +46,11 @@ static bool mma_forced() {
   return e && std::strcmp(e, "mma") == 0;
 }
 
+// The fine kernels of an ordinary call on the tcgen05 path: head dim 128, or head dim 64 with blocks of 128 or 256 tokens.
+static bool on_umma(int D, int be, int dtype, int topk) {
+  return !scalar_forced() && !mma_forced() && (sparse_umma_eligible(D, be, dtype, topk) || sparse_wide64_eligible(D, be, dtype, topk));
+}
+
 static int check_dtype(int dtype) {
   if (dtype != VSA_BF16 && dtype != VSA_F32 && dtype != VSA_F16)
     return fail(VSA_ERR_UNSUPPORTED, "dtype %d is not bf16 (0), fp32 (1) or fp16 (2)", dtype);
@@ -170,8 +175,8 @@ static int sparse_fwd_dispatch(const void* q, const void* k, const void* v, cons
                                void* out_comb, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk,
                                float scale, int dtype, cudaStream_t st) {
   int rc;
-  if (lse2 && !scalar_forced() && !mma_forced() && sparse_umma_eligible(D, be, dtype, topk)) {
-    rc = sparse_fwd_umma(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, dtype, st, out_c, gate,
+  if (lse2 && on_umma(D, be, dtype, topk)) {
+    rc = sparse_fwd_umma(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st, out_c, gate,
                          out_comb);
     if (rc) return rc;
     // exact recomputation of the (normally zero) tiles the fixed-shift softmax marked as out of range
@@ -228,8 +233,8 @@ int vsa_sparse_bwd_dq(const void* dout, const void* q, const void* k, const void
   int rc = check_sparse(BH, Lq, Lkv, D, be, topk, dtype);
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && out_s && lse2 && selected && kv_sizes && delta && dq, "sparse dQ: null pointer");
-  if (!scalar_forced() && !mma_forced() && sparse_umma_eligible(D, be, dtype, topk))
-    return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale,
+  if (on_umma(D, be, dtype, topk))
+    return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream);
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
     return sparse_dq_tc(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
@@ -246,8 +251,8 @@ int vsa_sparse_bwd_dkdv(const void* dout, const void* q, const void* k, const vo
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && lse2 && delta && counts && offsets && inverse && kv_sizes && dk && dv,
               "sparse dK/dV: null pointer");
-  if (!scalar_forced() && !mma_forced() && sparse_umma_eligible(D, be, dtype, topk))
-    return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be,
+  if (on_umma(D, be, dtype, topk))
+    return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream);
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
     return sparse_dkdv_tc(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
@@ -268,8 +273,8 @@ int vsa_sparse_bwd_dq_fused(const void* dout, const void* q, const void* k, cons
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && out_s && lse2 && selected && kv_sizes && delta && dq && dq_mean && q_sizes,
               "sparse dQ (fused): null pointer");
-  if (!scalar_forced() && !mma_forced() && sparse_umma_eligible(D, be, dtype, topk))
-    return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale,
+  if (on_umma(D, be, dtype, topk))
+    return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream, dq_mean, q_sizes);
   rc = vsa_sparse_bwd_dq(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                          dtype, stream);
@@ -286,8 +291,8 @@ int vsa_sparse_bwd_dkdv_fused(const void* dout, const void* q, const void* k, co
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && lse2 && delta && counts && offsets && inverse && kv_sizes && dk && dv &&
                   dk_mean && dv_mean, "sparse dK/dV (fused): null pointer");
-  if (!scalar_forced() && !mma_forced() && sparse_umma_eligible(D, be, dtype, topk))
-    return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be,
+  if (on_umma(D, be, dtype, topk))
+    return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean);
   rc = vsa_sparse_bwd_dkdv(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                            topk, scale, dtype, stream);
@@ -340,7 +345,7 @@ int vsa_sparse_bwd_dkdv_ds(const void* dout, const void* q, const void* k, const
   VSA_REQUIRE((dk_mean == nullptr) == (dv_mean == nullptr), "sparse dK/dV (dS stored): give both pooled gradients or neither");
   if (!vsa_sparse_bwd_ds_supported(D, be, topk, dtype))
     return fail(VSA_ERR_UNSUPPORTED, "sparse dK/dV (dS stored): needs bf16 or fp16, head dim 128, block volume 64, 128 or 256");
-  return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse_edges, kv_sizes, dk, dv, BH, Lq, Lkv, be,
+  return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse_edges, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                           topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean, ds_ws);
 }
 
@@ -384,7 +389,7 @@ int vsa_sparse_fwd_combine_sharded(const void* q, const void* k_sh, const void* 
   VSA_REQUIRE((out == nullptr) == (out_c == nullptr), "sparse forward (sharded): give out_c and out together, or neither");
   if ((rc = check_sharded(Lkv, kv_shard, D, be, topk, dtype, "sparse forward (sharded)"))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = sparse_fwd_umma(q, k_sh, v_sh, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, be, topk, scale, dtype, st, out_c, gate,
+  rc = sparse_fwd_umma(q, k_sh, v_sh, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st, out_c, gate,
                        out, kv_shard);
   if (rc) return rc;
   return sparse_fwd_tc(q, k_sh, v_sh, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, true, st, out_c,
@@ -402,7 +407,7 @@ int vsa_sparse_bwd_dq_sharded(const void* dout, const void* q, const void* k_sh,
               "sparse dQ (sharded): null pointer");
   VSA_REQUIRE((dq_mean == nullptr) == (q_sizes == nullptr), "sparse dQ (sharded): give the pooled gradient and the query sizes, or neither");
   if ((rc = check_sharded(Lkv, kv_shard, D, be, topk, dtype, "sparse dQ (sharded)"))) return rc;
-  return sparse_dq_umma(dout, q, k_sh, v_sh, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale,
+  return sparse_dq_umma(dout, q, k_sh, v_sh, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                         dtype, (cudaStream_t)stream, dq_mean, q_sizes, kv_shard);
 }
 
@@ -417,7 +422,7 @@ int vsa_sparse_bwd_dkdv_sharded(const void* dout, const void* q, const void* k_s
               "sparse dK/dV (sharded): null pointer");
   VSA_REQUIRE((dk_mean == nullptr) == (dv_mean == nullptr), "sparse dK/dV (sharded): give both pooled gradients or neither");
   if ((rc = check_sharded(Lkv, kv_shard, D, be, topk, dtype, "sparse dK/dV (sharded)"))) return rc;
-  return sparse_dkdv_umma(dout, q, k_sh, v_sh, lse2, delta, counts, offsets, inverse, kv_sizes, dk_sh, dv_sh, BH, Lq, Lkv, be,
+  return sparse_dkdv_umma(dout, q, k_sh, v_sh, lse2, delta, counts, offsets, inverse, kv_sizes, dk_sh, dv_sh, BH, Lq, Lkv, D, be,
                           topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean, nullptr, kv_shard);
 }
 
@@ -476,7 +481,7 @@ int vsa_sparse_fwd_combine_raster(const void* q, const void* k, const void* v, c
               "sparse forward (raster): null pointer");
   if ((rc = check_raster(q_map, raster_rows, heads, BH, D, be, topk, dtype, "sparse forward (raster)"))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  rc = sparse_fwd_umma(q, k, v, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, be, topk, scale, dtype, st, out_c,
+  rc = sparse_fwd_umma(q, k, v, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st, out_c,
                        gate_raster, out_raster, 0, q_map, raster_rows, heads);
   if (rc) return rc;
   return sparse_fwd_tc(q, k, v, selected, kv_sizes, out_s, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, true, st, out_c,
@@ -494,7 +499,7 @@ int vsa_sparse_bwd_dq_raster(const void* dout, const void* q, const void* k, con
               "sparse dQ (raster): null pointer");
   VSA_REQUIRE((dq_mean == nullptr) == (q_sizes == nullptr), "sparse dQ (raster): give the pooled gradient and the query sizes, or neither");
   if ((rc = check_raster(q_map, raster_rows, heads, BH, D, be, topk, dtype, "sparse dQ (raster)"))) return rc;
-  return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq_raster, BH, Lq, Lkv, be, topk, scale,
+  return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq_raster, BH, Lq, Lkv, D, be, topk, scale,
                         dtype, (cudaStream_t)stream, dq_mean, q_sizes, 0, q_map, raster_rows, heads);
 }
 
@@ -511,7 +516,7 @@ int vsa_sparse_bwd_dkdv_raster(const void* dout, const void* q, const void* k, c
   VSA_REQUIRE((dk_mean == nullptr) == (dv_mean == nullptr), "sparse dK/dV (raster): give both pooled gradients or neither");
   if ((rc = check_raster(kv_map, raster_rows, heads, BH, D, be, topk, dtype, "sparse dK/dV (raster)"))) return rc;
   return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk_raster, dv_raster, BH, Lq,
-                          Lkv, be, topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean, nullptr, 0, kv_map,
+                          Lkv, D, be, topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean, nullptr, 0, kv_map,
                           raster_rows, heads);
 }
 

@@ -69,8 +69,10 @@ int sparse_dkdv_tc(const void* dout, const void* q, const void* k, const void* v
 
 // ---- tcgen05 / TMA kernels, bf16 or fp16 by `dtype` (sparse_umma.cu) -----------------------------------------------------
 bool sparse_umma_eligible(int D, int be, int dtype, int topk);
+// head dim 64 on the 128-row tcgen05 kernels: ordinary layout only (no shard-major K/V, raster stores or stored dS)
+bool sparse_wide64_eligible(int D, int be, int dtype, int topk);
 int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes,
-                    void* out, float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale,
+                    void* out, float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale,
                     int dtype, cudaStream_t st, const void* out_c = nullptr, const void* gate = nullptr,
                     void* out_comb = nullptr, int64_t kv_shard = 0,   // kv_shard: tokens per shard of a shard-major K/V buffer (0 = ordinary layout)
                     const int32_t* comb_map = nullptr, int64_t comb_rows = 0, int comb_heads = 1);
@@ -78,12 +80,12 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
 // the raster layout [B, comb_rows, comb_heads, D] (BH = B * comb_heads) instead of tile order
 int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v, const void* out_s,
                    const float* lse2, const int32_t* selected, const int32_t* kv_sizes, float* delta, void* dq,
-                   int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale, int dtype,
+                   int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale, int dtype,
                    cudaStream_t st, const void* dq_mean = nullptr, const int32_t* q_sizes = nullptr,
                    int64_t kv_shard = 0, const int32_t* out_map = nullptr, int64_t out_rows = 0, int out_heads = 1);
 int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void* v, const float* lse2,
                      const float* delta, const int32_t* counts, const int32_t* offsets, const int32_t* inverse,
-                     const int32_t* kv_sizes, void* dk, void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk,
+                     const int32_t* kv_sizes, void* dk, void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk,
                      float scale, int dtype, cudaStream_t st, const void* dk_mean = nullptr,
                      const void* dv_mean = nullptr, void* ds_ws = nullptr, int64_t kv_shard = 0,
                      const int32_t* out_map = nullptr, int64_t out_rows = 0, int out_heads = 1);

@@ -30,6 +30,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -73,16 +74,16 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [rows, cols] row-major of a 16-bit element type (cols = 128: q/k/v-like tensors; cols = 64: stored dS tiles), boxes of 64 rows x 64
-// columns, 128-byte swizzle.
-int make_map_of(CUtensorMap* map, CUtensorMapDataType elem, const void* ptr, int64_t rows, const char* what, int cols = kD) {
+// [rows, cols] row-major of a 16-bit element type (cols = 128: q/k/v-like tensors; cols = 64: stored dS tiles), boxes of box_rows
+// rows x 64 columns, 128-byte swizzle.
+int make_map_of(CUtensorMap* map, CUtensorMapDataType elem, const void* ptr, int64_t rows, const char* what, int cols = kD, int box_rows = 64) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(VSA_ERR_LAUNCH, "%s: cuTensorMapEncodeTiled is not available from the driver", what);
   if (reinterpret_cast<uintptr_t>(ptr) % 16) return fail(VSA_ERR_BAD_ARGUMENT, "%s: pointer is not 16-byte aligned", what);
   if (rows > 0x7fffffffLL) return fail(VSA_ERR_UNSUPPORTED, "%s: %lld rows exceed the TMA coordinate range", what, (long long)rows);
   const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t gstride[1] = {(cuuint64_t)cols * 2};
-  const cuuint32_t box[2] = {64, 64};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(map, elem, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -242,7 +243,8 @@ int check_kv_shard(int64_t Lkv, int be, int64_t* kv_shard, const char* what) {
 
 }  // namespace
 
-// A logical block of 64, 128 or 256 tokens is walked as 1, 2 or 4 tiles of 64 tokens (the kernels' SUB parameter).
+// The stored-dS backward walks a block of 64, 128 or 256 tokens as 1, 2 or 4 tiles of 64 tokens (its kernels' SUB parameter);
+// otherwise blocks that are multiples of 128 run on the 128-row kernels (sparse_wide.inl).
 #define VSA_BY_BLOCK_VOLUME(be_, launch_, kernel_) \
   return (be_) == 64 ? launch_(kernel_<1>) : (be_) == 128 ? launch_(kernel_<2>) : launch_(kernel_<4>)
 
@@ -279,38 +281,42 @@ bool sparse_umma_eligible(int D, int be, int dtype, int topk) {
   return false;
 }
 
+bool sparse_wide64_eligible(int D, int be, int dtype, int topk) {
+  return D == 64 && (be == 128 || be == 256) && (dtype == VSA_BF16 || dtype == VSA_F16) && topk * (be / kTile) <= kMaxTiles;
+}
+
 int64_t sparse_ds_workspace_bytes(int64_t BH, int64_t Lq, int be, int topk) {
   const int64_t sub = be / kTile;
   return BH * (Lq / be) * topk * sub * sub * (int64_t)(kTile * kTile * 2);
 }
 
 int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes,
-                    void* out, float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale,
+                    void* out, float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale,
                     int dtype, cudaStream_t st, const void* out_c, const void* gate, void* out_comb, int64_t kv_shard,
                     const int32_t* comb_map, int64_t comb_rows, int comb_heads) {
   const RasterMap rm{comb_map, (long long)comb_rows, comb_heads > 0 ? comb_heads : 1};
-  return VSA_BY_DTYPE(dtype, sparse_fwd_umma(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st,
+  return VSA_BY_DTYPE(dtype, sparse_fwd_umma(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, st,
                                              out_c, gate, out_comb, kv_shard, rm));
 }
 
 int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v, const void* out_s,
                    const float* lse2, const int32_t* selected, const int32_t* kv_sizes, float* delta, void* dq,
-                   int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale, int dtype, cudaStream_t st,
+                   int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale, int dtype, cudaStream_t st,
                    const void* dq_mean, const int32_t* q_sizes, int64_t kv_shard, const int32_t* out_map,
                    int64_t out_rows, int out_heads) {
   const RasterMap rm{out_map, (long long)out_rows, out_heads > 0 ? out_heads : 1};
-  return VSA_BY_DTYPE(dtype, sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be,
+  return VSA_BY_DTYPE(dtype, sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be,
                                             topk, scale, st, dq_mean, q_sizes, kv_shard, rm));
 }
 
 int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void* v, const float* lse2,
                      const float* delta, const int32_t* counts, const int32_t* offsets, const int32_t* inverse,
-                     const int32_t* kv_sizes, void* dk, void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk,
+                     const int32_t* kv_sizes, void* dk, void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk,
                      float scale, int dtype, cudaStream_t st, const void* dk_mean, const void* dv_mean, void* ds_ws,
                      int64_t kv_shard, const int32_t* out_map, int64_t out_rows, int out_heads) {
   const RasterMap rm{out_map, (long long)out_rows, out_heads > 0 ? out_heads : 1};
   return VSA_BY_DTYPE(dtype, sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH,
-                                              Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, ds_ws, kv_shard, rm));
+                                              Lq, Lkv, D, be, topk, scale, st, dk_mean, dv_mean, ds_ws, kv_shard, rm));
 }
 
 int sparse_dq_from_ds_umma(const void* k, const int32_t* selected, const int32_t* kv_sizes, const void* ds_ws, void* dq,
