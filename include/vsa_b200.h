@@ -128,6 +128,13 @@ int vsa_coarse_fwd(const void* q_mean, const void* k_mean, const void* v_mean,
                    int64_t BH, int Qb, int Kb, int D, float scale,
                    int dtype, void* stream);
 
+/* The same with the rows of probs `pitch` >= Kb elements apart (what lies between Kb and pitch is neither read nor
+ * written).  A pitch of a multiple of 8 lets 16-bit types use the tensor cores whatever the block counts are. */
+int vsa_coarse_fwd_pitched(const void* q_mean, const void* k_mean, const void* v_mean,
+                           void* scores, void* probs, void* out_c,
+                           int64_t BH, int Qb, int Kb, int pitch, int D, float scale,
+                           int dtype, void* stream);
+
 /* Top-K key blocks per query block from the pooled scores; ids are written in
  * ascending order, ties broken towards the lower id.
  * Replaces scores.topk(...).indices: vsa/torch_impl.py:85, vsa/triton_impl.py:1710. */
@@ -143,6 +150,14 @@ int vsa_coarse_bwd(const void* d_out_c, const void* out_c,
                    void* dq_mean, void* dk_mean, void* dv_mean,
                    int64_t BH, int Qb, int Kb, int D, float scale,
                    int dtype, void* stream);
+
+/* The same with the rows of probs and dscores_ws `pitch` elements apart, as vsa_coarse_fwd_pitched left them. */
+int vsa_coarse_bwd_pitched(const void* d_out_c, const void* out_c,
+                           const void* q_mean, const void* k_mean, const void* v_mean,
+                           const void* probs, void* dscores_ws, float* rowdot_ws,
+                           void* dq_mean, void* dk_mean, void* dv_mean,
+                           int64_t BH, int Qb, int Kb, int pitch, int D, float scale,
+                           int dtype, void* stream);
 
 /* Fine attention of each query block over the valid tokens of its selected key
  * blocks; lse2 (may be NULL, which selects the warp-level kernel instead of the tcgen05 one)

@@ -25,8 +25,10 @@ SIGNATURES = {
     "vsa_block_mean_bwd_accumulate": [P, P, P, L, L, I, I, I, P],
     "vsa_block_mean_bwd": [P, P, P, L, L, I, I, I, P],
     "vsa_coarse_fwd": [P, P, P, P, P, P, L, I, I, I, F, I, P],
+    "vsa_coarse_fwd_pitched": [P, P, P, P, P, P, L, I, I, I, I, F, I, P],
     "vsa_topk": [P, P, L, I, I, I, P],
     "vsa_coarse_bwd": [P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, F, I, P],
+    "vsa_coarse_bwd_pitched": [P, P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, F, I, P],
     "vsa_sparse_fwd": [P, P, P, P, P, P, P, L, L, L, I, I, I, F, I, P],
     "vsa_sparse_fwd_combine": [P, P, P, P, P, P, P, P, P, P, L, L, L, I, I, I, F, I, P],
     "vsa_route_invert": [P, P, P, P, P, L, I, I, I, P],

@@ -125,15 +125,30 @@ int vsa_block_mean_bwd(void* dx, const void* dmean, const int32_t* sizes, int64_
   return block_mean_bwd(dx, dmean, sizes, BH, L, D, be, dtype, false, (cudaStream_t)stream);
 }
 
-int vsa_coarse_fwd(const void* q_mean, const void* k_mean, const void* v_mean, void* scores, void* probs, void* out_c,
-                   int64_t BH, int Qb, int Kb, int D, float scale, int dtype, void* stream) {
+// Rows of probs and dS lie `pitch` elements apart.  Tensor cores take them when that is a multiple of 16 bytes; the dense
+// entry points keep to shapes whose two block counts are multiples of eight.
+static int coarse_fwd_any(const void* q_mean, const void* k_mean, const void* v_mean, void* scores, void* probs,
+                          void* out_c, int64_t BH, int Qb, int Kb, int pitch, int D, float scale, int dtype, bool tensor,
+                          cudaStream_t st) {
   int rc = check_dtype(dtype);
   if (rc) return rc;
-  VSA_REQUIRE(BH >= 0 && Qb >= 0 && Kb >= 1 && D >= 1, "coarse forward: bad extents");
+  VSA_REQUIRE(BH >= 0 && Qb >= 0 && Kb >= 1 && D >= 1 && pitch >= Kb, "coarse forward: bad extents");
   VSA_REQUIRE(q_mean && k_mean && v_mean && scores && probs && out_c, "coarse forward: null pointer");
-  if (!scalar_forced() && coarse_umma_eligible(Qb, Kb, D, dtype))
-    return coarse_fwd_umma(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, D, scale, dtype, (cudaStream_t)stream);
-  return coarse_fwd(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, D, scale, dtype, (cudaStream_t)stream);
+  if (tensor && !scalar_forced() && coarse_umma_eligible(Kb, pitch, D, dtype))
+    return coarse_fwd_umma(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, pitch, D, scale, dtype, st);
+  return coarse_fwd(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, pitch, D, scale, dtype, st);
+}
+
+int vsa_coarse_fwd(const void* q_mean, const void* k_mean, const void* v_mean, void* scores, void* probs, void* out_c,
+                   int64_t BH, int Qb, int Kb, int D, float scale, int dtype, void* stream) {
+  return coarse_fwd_any(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, Kb, D, scale, dtype,
+                        Qb % 8 == 0 && Kb % 8 == 0, (cudaStream_t)stream);
+}
+
+int vsa_coarse_fwd_pitched(const void* q_mean, const void* k_mean, const void* v_mean, void* scores, void* probs,
+                           void* out_c, int64_t BH, int Qb, int Kb, int pitch, int D, float scale, int dtype, void* stream) {
+  return coarse_fwd_any(q_mean, k_mean, v_mean, scores, probs, out_c, BH, Qb, Kb, pitch, D, scale, dtype, true,
+                        (cudaStream_t)stream);
 }
 
 int vsa_topk(const void* scores, int32_t* selected, int64_t rows, int Kb, int topk, int dtype, void* stream) {
@@ -145,19 +160,35 @@ int vsa_topk(const void* scores, int32_t* selected, int64_t rows, int Kb, int to
   return topk_select(scores, selected, rows, Kb, topk, dtype, (cudaStream_t)stream);
 }
 
+static int coarse_bwd_any(const void* d_out_c, const void* out_c, const void* q_mean, const void* k_mean,
+                          const void* v_mean, const void* probs, void* dscores_ws, float* rowdot_ws, void* dq_mean,
+                          void* dk_mean, void* dv_mean, int64_t BH, int Qb, int Kb, int pitch, int D, float scale, int dtype,
+                          bool tensor, cudaStream_t st) {
+  int rc = check_dtype(dtype);
+  if (rc) return rc;
+  VSA_REQUIRE(BH >= 0 && Qb >= 0 && Kb >= 1 && D >= 1 && pitch >= Kb, "coarse backward: bad extents");
+  VSA_REQUIRE(d_out_c && out_c && q_mean && k_mean && v_mean && probs && dscores_ws && rowdot_ws && dq_mean &&
+                  dk_mean && dv_mean, "coarse backward: null pointer");
+  if (tensor && !scalar_forced() && coarse_umma_eligible(Kb, pitch, D, dtype))
+    return coarse_bwd_umma(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean,
+                           dv_mean, BH, Qb, Kb, pitch, D, scale, dtype, st);
+  return coarse_bwd(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean, dv_mean,
+                    BH, Qb, Kb, pitch, D, scale, dtype, st);
+}
+
 int vsa_coarse_bwd(const void* d_out_c, const void* out_c, const void* q_mean, const void* k_mean, const void* v_mean,
                    const void* probs, void* dscores_ws, float* rowdot_ws, void* dq_mean, void* dk_mean, void* dv_mean,
                    int64_t BH, int Qb, int Kb, int D, float scale, int dtype, void* stream) {
-  int rc = check_dtype(dtype);
-  if (rc) return rc;
-  VSA_REQUIRE(BH >= 0 && Qb >= 0 && Kb >= 1 && D >= 1, "coarse backward: bad extents");
-  VSA_REQUIRE(d_out_c && out_c && q_mean && k_mean && v_mean && probs && dscores_ws && rowdot_ws && dq_mean &&
-                  dk_mean && dv_mean, "coarse backward: null pointer");
-  if (!scalar_forced() && coarse_umma_eligible(Qb, Kb, D, dtype))
-    return coarse_bwd_umma(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean,
-                           dv_mean, BH, Qb, Kb, D, scale, dtype, (cudaStream_t)stream);
-  return coarse_bwd(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean, dv_mean,
-                    BH, Qb, Kb, D, scale, dtype, (cudaStream_t)stream);
+  return coarse_bwd_any(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean, dv_mean, BH,
+                        Qb, Kb, Kb, D, scale, dtype, Qb % 8 == 0 && Kb % 8 == 0, (cudaStream_t)stream);
+}
+
+int vsa_coarse_bwd_pitched(const void* d_out_c, const void* out_c, const void* q_mean, const void* k_mean,
+                           const void* v_mean, const void* probs, void* dscores_ws, float* rowdot_ws, void* dq_mean,
+                           void* dk_mean, void* dv_mean, int64_t BH, int Qb, int Kb, int pitch, int D, float scale, int dtype,
+                           void* stream) {
+  return coarse_bwd_any(d_out_c, out_c, q_mean, k_mean, v_mean, probs, dscores_ws, rowdot_ws, dq_mean, dk_mean, dv_mean, BH,
+                        Qb, Kb, pitch, D, scale, dtype, true, (cudaStream_t)stream);
 }
 
 static int check_sparse(int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, int dtype) {

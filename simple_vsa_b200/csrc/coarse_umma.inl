@@ -36,7 +36,7 @@ enum GemmEpilogue { kEpiStore = 0, kEpiScores = 1, kEpiSoftmaxBwd = 2 };
 template <int A_MN, int B_MN, int EPI>
 __global__ void __launch_bounds__(192, 2)
 coarse_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                        elem_t* __restrict__ C, int M, int N, int K, float scale, const elem_t* __restrict__ probs,
+                        elem_t* __restrict__ C, int M, int N, int K, int ldc, float scale, const elem_t* __restrict__ probs,
                         const float* __restrict__ rowdot) {
   extern __shared__ uint8_t smem_raw[];
   if (*(volatile int*)&g_device_status != 0) return;
@@ -120,7 +120,7 @@ coarse_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     if (!ok && lane == 0) report_timeout(33);
     tc_fence_after();
     if (ok) {
-      const long long row_off = ((long long)batch * M + m) * N;
+      const long long row_off = ((long long)batch * M + m) * ldc;   // a multiple of 8: the wide stores are aligned
       const float rd = (EPI == kEpiSoftmaxBwd && m < M) ? rowdot[(long long)batch * M + m] : 0.f;
 #pragma unroll 1
       for (int c4 = 0; c4 < 4; ++c4) {

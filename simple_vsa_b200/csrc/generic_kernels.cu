@@ -280,7 +280,7 @@ template <typename T> struct EpiSoftmaxBwd {   // dS = P * (dP - rowdot) * scale
 template <typename T, typename Epi>
 __global__ void __launch_bounds__(256) gemm_kernel(const T* __restrict__ A, long long a_bs, int a_rs, int a_cs,
                                                    const T* __restrict__ B, long long b_bs, int b_rs, int b_cs,
-                                                   T* __restrict__ C, long long c_bs, int M, int N, int K, Epi epi) {
+                                                   T* __restrict__ C, int c_rs, int M, int N, int K, Epi epi) {
   __shared__ float As[16][68];
   __shared__ float Bs[16][68];
   const long long b = blockIdx.z;
@@ -327,27 +327,27 @@ __global__ void __launch_bounds__(256) gemm_kernel(const T* __restrict__ A, long
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      if (n < N) epi(C, b * c_bs + (long long)m * N + n, b, m, n, acc[i][j]);
+      if (n < N) epi(C, (b * M + m) * (long long)c_rs + n, b, m, n, acc[i][j]);
     }
   }
 }
 
 template <typename T, typename Epi>
 static int gemm(const T* A, long long a_bs, int a_rs, int a_cs, const T* B, long long b_bs, int b_rs, int b_cs,
-                T* C, int64_t batch, int M, int N, int K, Epi epi, cudaStream_t st, const char* what) {
+                T* C, int64_t batch, int M, int N, int K, Epi epi, cudaStream_t st, const char* what, int c_rs = 0) {
   if (batch == 0 || M == 0 || N == 0) return VSA_OK;
   if (batch > 65535) return fail(VSA_ERR_UNSUPPORTED, "%s: batch*heads %lld exceeds 65535", what, (long long)batch);
   dim3 grid((N + 63) / 64, (M + 63) / 64, (unsigned)batch);
-  gemm_kernel<T, Epi><<<grid, 256, 0, st>>>(A, a_bs, a_rs, a_cs, B, b_bs, b_rs, b_cs, C, (long long)M * N, M, N, K, epi);
+  gemm_kernel<T, Epi><<<grid, 256, 0, st>>>(A, a_bs, a_rs, a_cs, B, b_bs, b_rs, b_cs, C, c_rs ? c_rs : N, M, N, K, epi);
   return check_launch(what);
 }
 
 // Row softmax of the pooled scores: probs = round(softmax_fp32(scores)).
 template <typename T>
-__global__ void __launch_bounds__(128) softmax_rows_kernel(const T* __restrict__ scores, T* __restrict__ probs, int n) {
+__global__ void __launch_bounds__(128) softmax_rows_kernel(const T* __restrict__ scores, T* __restrict__ probs, int n, int pitch) {
   __shared__ float red[4];
   const T* s = scores + (long long)blockIdx.x * n;
-  T* p = probs + (long long)blockIdx.x * n;
+  T* p = probs + (long long)blockIdx.x * pitch;
   float mx = -INFINITY;
   for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmaxf(mx, Elem<T>::ld(s + i));
   mx = warp_max(mx);
@@ -369,12 +369,12 @@ __global__ void __launch_bounds__(128) softmax_rows_kernel(const T* __restrict__
 // element), reductions by shuffles only.  Same arithmetic as above: fp32 max, expf, fp32 sum, one rounding.
 template <typename T, int SLOTS>
 __global__ void __launch_bounds__(256) softmax_rows_warp_kernel(const T* __restrict__ scores, T* __restrict__ probs,
-                                                                long long rows, int n) {
+                                                                long long rows, int n, int pitch) {
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const T* s = scores + row * n;
-  T* p = probs + row * n;
+  T* p = probs + row * pitch;
   float x[SLOTS];
   float mx = -INFINITY;
 #pragma unroll
@@ -400,16 +400,16 @@ __global__ void __launch_bounds__(256) softmax_rows_warp_kernel(const T* __restr
 }
 
 template <typename T>
-static int launch_softmax_rows(const T* scores, T* probs, long long rows, int n, cudaStream_t st) {
+static int launch_softmax_rows(const T* scores, T* probs, long long rows, int n, int pitch, cudaStream_t st) {
   const unsigned grid = (unsigned)((rows + 7) / 8);
   if (n <= 512) {
-    softmax_rows_warp_kernel<T, 16><<<grid, 256, 0, st>>>(scores, probs, rows, n);
+    softmax_rows_warp_kernel<T, 16><<<grid, 256, 0, st>>>(scores, probs, rows, n, pitch);
   } else if (n <= 1536) {
-    softmax_rows_warp_kernel<T, 48><<<grid, 256, 0, st>>>(scores, probs, rows, n);
+    softmax_rows_warp_kernel<T, 48><<<grid, 256, 0, st>>>(scores, probs, rows, n, pitch);
   } else if (n <= 3072) {
-    softmax_rows_warp_kernel<T, 96><<<grid, 256, 0, st>>>(scores, probs, rows, n);
+    softmax_rows_warp_kernel<T, 96><<<grid, 256, 0, st>>>(scores, probs, rows, n, pitch);
   } else {
-    softmax_rows_kernel<T><<<(unsigned)rows, 128, 0, st>>>(scores, probs, n);
+    softmax_rows_kernel<T><<<(unsigned)rows, 128, 0, st>>>(scores, probs, n, pitch);
   }
   return check_launch("softmax_rows_kernel");
 }
@@ -425,12 +425,12 @@ __global__ void rowdot_kernel(const T* __restrict__ a, const T* __restrict__ b, 
   if ((threadIdx.x & 31) == 0) out[r] = s;
 }
 
-int softmax_rows(const void* scores, void* probs, int64_t rows, int n, int dtype, cudaStream_t st) {
+int softmax_rows(const void* scores, void* probs, int64_t rows, int n, int pitch, int dtype, cudaStream_t st) {
   if (rows == 0) return VSA_OK;
   if (rows > 0x7fffffffLL) return fail(VSA_ERR_UNSUPPORTED, "pooled softmax: too many rows");
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = VSA_TAG_TYPE(tag);
-    return launch_softmax_rows<T>((const T*)scores, (T*)probs, rows, n, st);
+    return launch_softmax_rows<T>((const T*)scores, (T*)probs, rows, n, pitch, st);
   });
 }
 
@@ -443,34 +443,47 @@ int rowdot_rows(const void* a, const void* b, float* out, int64_t rows, int D, i
   });
 }
 
+// scores[Qb,Kb] = qc[Qb,D] * kc[Kb,D]^T
+template <typename T>
+static int coarse_scores_t(const T* qc, const T* kc, T* scores, int64_t BH, int Qb, int Kb, int D, float scale, cudaStream_t st) {
+  return gemm<T>(qc, (long long)Qb * D, D, 1, kc, (long long)Kb * D, 1, D, scores, BH, Qb, Kb, D, EpiScores{scale}, st,
+                 "coarse scores");
+}
+
+int coarse_scores(const void* qc, const void* kc, void* scores, int64_t BH, int Qb, int Kb, int D, float scale, int dtype,
+                  cudaStream_t st) {
+  return dispatch_dtype(dtype, [&](auto* tag) {
+    using T = VSA_TAG_TYPE(tag);
+    return coarse_scores_t<T>((const T*)qc, (const T*)kc, (T*)scores, BH, Qb, Kb, D, scale, st);
+  });
+}
+
 template <typename T>
 static int coarse_fwd_t(const T* qc, const T* kc, const T* vc, T* scores, T* probs, T* out_c,
-                        int64_t BH, int Qb, int Kb, int D, float scale, cudaStream_t st) {
-  // scores[Qb,Kb] = qc[Qb,D] * kc[Kb,D]^T
-  int rc = gemm<T>(qc, (long long)Qb * D, D, 1, kc, (long long)Kb * D, 1, D, scores, BH, Qb, Kb, D,
-                   EpiScores{scale}, st, "coarse scores");
+                        int64_t BH, int Qb, int Kb, int pitch, int D, float scale, cudaStream_t st) {
+  int rc = coarse_scores_t<T>(qc, kc, scores, BH, Qb, Kb, D, scale, st);
   if (rc) return rc;
   const long long rows = BH * Qb;
   if (rows > 0x7fffffffLL) return fail(VSA_ERR_UNSUPPORTED, "coarse softmax: too many rows");
-  rc = launch_softmax_rows<T>(scores, probs, rows, Kb, st);
+  rc = launch_softmax_rows<T>(scores, probs, rows, Kb, pitch, st);
   if (rc) return rc;
   // out_c[Qb,D] = probs[Qb,Kb] * vc[Kb,D]
-  return gemm<T>(probs, (long long)Qb * Kb, Kb, 1, vc, (long long)Kb * D, D, 1, out_c, BH, Qb, D, Kb, EpiStore{}, st,
+  return gemm<T>(probs, (long long)Qb * pitch, pitch, 1, vc, (long long)Kb * D, D, 1, out_c, BH, Qb, D, Kb, EpiStore{}, st,
                  "coarse output");
 }
 
 int coarse_fwd(const void* qc, const void* kc, const void* vc, void* scores, void* probs, void* out_c, int64_t BH,
-               int Qb, int Kb, int D, float scale, int dtype, cudaStream_t st) {
+               int Qb, int Kb, int pitch, int D, float scale, int dtype, cudaStream_t st) {
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = VSA_TAG_TYPE(tag);
-    return coarse_fwd_t<T>((const T*)qc, (const T*)kc, (const T*)vc, (T*)scores, (T*)probs, (T*)out_c, BH, Qb, Kb, D,
+    return coarse_fwd_t<T>((const T*)qc, (const T*)kc, (const T*)vc, (T*)scores, (T*)probs, (T*)out_c, BH, Qb, Kb, pitch, D,
                            scale, st);
   });
 }
 
 template <typename T>
 static int coarse_bwd_t(const T* d_out_c, const T* out_c, const T* qc, const T* kc, const T* vc, const T* probs,
-                        T* ds, float* rowdot, T* dqc, T* dkc, T* dvc, int64_t BH, int Qb, int Kb, int D, float scale,
+                        T* ds, float* rowdot, T* dqc, T* dkc, T* dvc, int64_t BH, int Qb, int Kb, int pitch, int D, float scale,
                         cudaStream_t st) {
   const long long rows = BH * Qb;
   if (rows == 0) return VSA_OK;
@@ -478,29 +491,29 @@ static int coarse_bwd_t(const T* d_out_c, const T* out_c, const T* qc, const T* 
   int rc = check_launch("rowdot_kernel");
   if (rc) return rc;
   // dV_c[Kb,D] = probs^T[Kb,Qb] * d_out_c[Qb,D]
-  rc = gemm<T>(probs, (long long)Qb * Kb, 1, Kb, d_out_c, (long long)Qb * D, D, 1, dvc, BH, Kb, D, Qb, EpiStore{}, st,
+  rc = gemm<T>(probs, (long long)Qb * pitch, 1, pitch, d_out_c, (long long)Qb * D, D, 1, dvc, BH, Kb, D, Qb, EpiStore{}, st,
                "coarse dV");
   if (rc) return rc;
   // dS[Qb,Kb] = probs * (d_out_c[Qb,D] * vc[Kb,D]^T - rowdot) * scale
   rc = gemm<T>(d_out_c, (long long)Qb * D, D, 1, vc, (long long)Kb * D, 1, D, ds, BH, Qb, Kb, D,
-               EpiSoftmaxBwd<T>{probs, rowdot, scale, Qb}, st, "coarse dS");
+               EpiSoftmaxBwd<T>{probs, rowdot, scale, Qb}, st, "coarse dS", pitch);
   if (rc) return rc;
   // dQ_c[Qb,D] = dS[Qb,Kb] * kc[Kb,D]
-  rc = gemm<T>(ds, (long long)Qb * Kb, Kb, 1, kc, (long long)Kb * D, D, 1, dqc, BH, Qb, D, Kb, EpiStore{}, st,
+  rc = gemm<T>(ds, (long long)Qb * pitch, pitch, 1, kc, (long long)Kb * D, D, 1, dqc, BH, Qb, D, Kb, EpiStore{}, st,
                "coarse dQ");
   if (rc) return rc;
   // dK_c[Kb,D] = dS^T[Kb,Qb] * qc[Qb,D]
-  return gemm<T>(ds, (long long)Qb * Kb, 1, Kb, qc, (long long)Qb * D, D, 1, dkc, BH, Kb, D, Qb, EpiStore{}, st,
+  return gemm<T>(ds, (long long)Qb * pitch, 1, pitch, qc, (long long)Qb * D, D, 1, dkc, BH, Kb, D, Qb, EpiStore{}, st,
                  "coarse dK");
 }
 
 int coarse_bwd(const void* d_out_c, const void* out_c, const void* qc, const void* kc, const void* vc,
                const void* probs, void* ds, float* rowdot, void* dqc, void* dkc, void* dvc, int64_t BH, int Qb, int Kb,
-               int D, float scale, int dtype, cudaStream_t st) {
+               int pitch, int D, float scale, int dtype, cudaStream_t st) {
   return dispatch_dtype(dtype, [&](auto* tag) {
     using T = VSA_TAG_TYPE(tag);
     return coarse_bwd_t<T>((const T*)d_out_c, (const T*)out_c, (const T*)qc, (const T*)kc, (const T*)vc,
-                           (const T*)probs, (T*)ds, rowdot, (T*)dqc, (T*)dkc, (T*)dvc, BH, Qb, Kb, D, scale, st);
+                           (const T*)probs, (T*)ds, rowdot, (T*)dqc, (T*)dkc, (T*)dvc, BH, Qb, Kb, pitch, D, scale, st);
   });
 }
 

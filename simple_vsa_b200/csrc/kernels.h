@@ -10,12 +10,15 @@ int block_mean_fwd(const void* const* x, void* const* out, const int32_t* const*
                    int ntensors, int64_t BH, int D, int be, int dtype, cudaStream_t st);
 int block_mean_bwd(void* dx, const void* dmean, const int32_t* sizes, int64_t BH, int64_t L, int D, int be,
                    int dtype, bool accumulate, cudaStream_t st);
+// pitch: elements between rows of probs and ds (>= Kb)
 int coarse_fwd(const void* qc, const void* kc, const void* vc, void* scores, void* probs, void* out_c, int64_t BH,
-               int Qb, int Kb, int D, float scale, int dtype, cudaStream_t st);
+               int Qb, int Kb, int pitch, int D, float scale, int dtype, cudaStream_t st);
+int coarse_scores(const void* qc, const void* kc, void* scores, int64_t BH, int Qb, int Kb, int D, float scale, int dtype,
+                  cudaStream_t st);
 int coarse_bwd(const void* d_out_c, const void* out_c, const void* qc, const void* kc, const void* vc,
                const void* probs, void* ds, float* rowdot, void* dqc, void* dkc, void* dvc, int64_t BH, int Qb, int Kb,
-               int D, float scale, int dtype, cudaStream_t st);
-int softmax_rows(const void* scores, void* probs, int64_t rows, int n, int dtype, cudaStream_t st);
+               int pitch, int D, float scale, int dtype, cudaStream_t st);
+int softmax_rows(const void* scores, void* probs, int64_t rows, int n, int pitch, int dtype, cudaStream_t st);
 int rowdot_rows(const void* a, const void* b, float* out, int64_t rows, int D, int dtype, cudaStream_t st);
 int topk_select(const void* scores, int32_t* selected, int64_t rows, int Kb, int topk, int dtype, cudaStream_t st);
 // packed: rows hold (query block << 11) | slot of the key block in that query block's route, instead of query block ids
@@ -96,12 +99,12 @@ int64_t sparse_ds_workspace_bytes(int64_t BH, int64_t Lq, int be, int topk);
 int sparse_dq_from_ds_umma(const void* k, const int32_t* selected, const int32_t* kv_sizes, const void* ds_ws, void* dq,
                            int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale, int dtype,
                            cudaStream_t st, const void* dq_mean = nullptr, const int32_t* q_sizes = nullptr);
-bool coarse_umma_eligible(int Qb, int Kb, int D, int dtype);
+bool coarse_umma_eligible(int Kb, int pitch, int D, int dtype);
 int coarse_fwd_umma(const void* qc, const void* kc, const void* vc, void* scores, void* probs, void* out_c, int64_t BH,
-                    int Qb, int Kb, int D, float scale, int dtype, cudaStream_t st);
+                    int Qb, int Kb, int pitch, int D, float scale, int dtype, cudaStream_t st);
 int coarse_bwd_umma(const void* d_out_c, const void* out_c, const void* qc, const void* kc, const void* vc,
                     const void* probs, void* ds, float* rowdot, void* dqc, void* dkc, void* dvc, int64_t BH, int Qb,
-                    int Kb, int D, float scale, int dtype, cudaStream_t st);
+                    int Kb, int pitch, int D, float scale, int dtype, cudaStream_t st);
 int umma_selftest(const void* a, const void* b, float* out, int mode, cudaStream_t st);
 int wait_timeout_selftest(unsigned long long limit_ns, int* gave_up, cudaStream_t st);
 int device_status_fetch_and_clear(int* status);

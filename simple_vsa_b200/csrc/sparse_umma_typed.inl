@@ -9,8 +9,9 @@
 int make_map(CUtensorMap* map, const void* ptr, int64_t rows, const char* what, int cols = kD) {
   return make_map_of(map, kTmaElem, ptr, rows, what, cols);
 }
-int make_map3d(CUtensorMap* map, const void* ptr, int64_t batch, int64_t rows, int64_t cols, int box_rows, const char* what) {
-  return make_map3d_of(map, kTmaElem, ptr, batch, rows, cols, box_rows, what);
+int make_map3d(CUtensorMap* map, const void* ptr, int64_t batch, int64_t rows, int64_t cols, int box_rows, const char* what,
+               int64_t pitch = 0) {
+  return make_map3d_of(map, kTmaElem, ptr, batch, rows, cols, box_rows, what, pitch);
 }
 
 // 8 MMAs over the 128-wide reduction, both operands reduction-contiguous ("K-major").
@@ -499,52 +500,58 @@ int sparse_dq_from_ds_umma(const void* k, const int32_t* selected, const int32_t
   VSA_BY_BLOCK_VOLUME(be, launch, sparse_dq_from_ds_kernel);
 }
 
-// C[batch, M, N] = A * B.  a_rows/a_cols and b_rows/b_cols describe the operands as stored in memory.
+// C[batch, M, N] = A * B.  a_rows/a_cols and b_rows/b_cols describe the operands as stored in memory; a_pitch and c_pitch
+// (0: dense) are the row pitches of A and of C (and of `probs`).
 template <int A_MN, int B_MN, int EPI>
-int launch_gemm(const void* A, int64_t a_rows, int64_t a_cols, const void* B, int64_t b_rows, int64_t b_cols, void* C,
-                int64_t batch, int M, int N, int K, float scale, const void* probs, const float* rowdot,
-                cudaStream_t st, const char* what) {
+int launch_gemm(const void* A, int64_t a_rows, int64_t a_cols, int64_t a_pitch, const void* B, int64_t b_rows, int64_t b_cols,
+                void* C, int64_t c_pitch, int64_t batch, int M, int N, int K, float scale, const void* probs,
+                const float* rowdot, cudaStream_t st, const char* what) {
   if (batch == 0 || M == 0 || N == 0) return VSA_OK;
   if (batch > 65535) return fail(VSA_ERR_UNSUPPORTED, "%s: batch*heads %lld exceeds 65535", what, (long long)batch);
   CUtensorMap ma, mb;
   int rc;
-  if ((rc = make_map3d(&ma, A, batch, a_rows, a_cols, A_MN ? 64 : 128, what))) return rc;
+  if ((rc = make_map3d(&ma, A, batch, a_rows, a_cols, A_MN ? 64 : 128, what, a_pitch))) return rc;
   if ((rc = make_map3d(&mb, B, batch, b_rows, b_cols, B_MN ? 64 : 128, what))) return rc;
   const int smem = GemmSmem::total + 1024;
   auto kern = coarse_gemm_umma_kernel<A_MN, B_MN, EPI>;
   if ((rc = reserve_smem(kern, smem, what))) return rc;
   dim3 grid((unsigned)((N + 127) / 128), (unsigned)((M + 127) / 128), (unsigned)batch);
-  kern<<<grid, 192, smem, st>>>(ma, mb, (elem_t*)C, M, N, K, scale, (const elem_t*)probs, rowdot);
+  kern<<<grid, 192, smem, st>>>(ma, mb, (elem_t*)C, M, N, K, (int)(c_pitch ? c_pitch : N), scale, (const elem_t*)probs, rowdot);
   return check_launch(what);
 }
 
+// The scores keep the operator's dense layout.  With a row pitch that is not 16 bytes their product stays on the CUDA cores:
+// it is one of six, and a sum taken in another order can turn a rounding, and with it a tie at the edge of the Top-K.
 int coarse_fwd_umma(const void* qc, const void* kc, const void* vc, void* scores, void* probs, void* out_c, int64_t BH,
-                    int Qb, int Kb, int D, float scale, cudaStream_t st) {
-  int rc = launch_gemm<0, 0, kEpiScores>(qc, Qb, D, kc, Kb, D, scores, BH, Qb, Kb, D, scale, nullptr, nullptr, st,
-                                         "pooled scores");
+                    int Qb, int Kb, int pitch, int D, float scale, cudaStream_t st) {
+  int rc = Qb % 8 == 0 && Kb % 8 == 0
+               ? launch_gemm<0, 0, kEpiScores>(qc, Qb, D, 0, kc, Kb, D, scores, 0, BH, Qb, Kb, D, scale, nullptr, nullptr, st,
+                                               "pooled scores")
+               : coarse_scores(qc, kc, scores, BH, Qb, Kb, D, scale, kDtypeCode, st);
   if (rc) return rc;
-  if ((rc = softmax_rows(scores, probs, BH * Qb, Kb, kDtypeCode, st))) return rc;
-  return launch_gemm<0, 1, kEpiStore>(probs, Qb, Kb, vc, Kb, D, out_c, BH, Qb, D, Kb, 1.f, nullptr, nullptr, st,
+  if ((rc = softmax_rows(scores, probs, BH * Qb, Kb, pitch, kDtypeCode, st))) return rc;
+  return launch_gemm<0, 1, kEpiStore>(probs, Qb, Kb, pitch, vc, Kb, D, out_c, 0, BH, Qb, D, Kb, 1.f, nullptr, nullptr, st,
                                       "pooled output");
 }
 
 int coarse_bwd_umma(const void* d_out_c, const void* out_c, const void* qc, const void* kc, const void* vc,
                     const void* probs, void* ds, float* rowdot, void* dqc, void* dkc, void* dvc, int64_t BH, int Qb,
-                    int Kb, int D, float scale, cudaStream_t st) {
+                    int Kb, int pitch, int D, float scale, cudaStream_t st) {
   int rc = rowdot_rows(d_out_c, out_c, rowdot, BH * Qb, D, kDtypeCode, st);
   if (rc) return rc;
   // dV_c[Kb,D] = P^T dO_c : A = P stored [Qb rows (reduction), Kb cols (M)], B = dO_c stored [Qb rows, D cols]
-  if ((rc = launch_gemm<1, 1, kEpiStore>(probs, Qb, Kb, d_out_c, Qb, D, dvc, BH, Kb, D, Qb, 1.f, nullptr, nullptr, st,
-                                         "pooled dV")))
+  if ((rc = launch_gemm<1, 1, kEpiStore>(probs, Qb, Kb, pitch, d_out_c, Qb, D, dvc, 0, BH, Kb, D, Qb, 1.f, nullptr, nullptr,
+                                         st, "pooled dV")))
     return rc;
   // dS[Qb,Kb] = P * (dO_c v_c^T - rowdot) * scale
-  if ((rc = launch_gemm<0, 0, kEpiSoftmaxBwd>(d_out_c, Qb, D, vc, Kb, D, ds, BH, Qb, Kb, D, scale, probs, rowdot, st,
-                                              "pooled dS")))
+  if ((rc = launch_gemm<0, 0, kEpiSoftmaxBwd>(d_out_c, Qb, D, 0, vc, Kb, D, ds, pitch, BH, Qb, Kb, D, scale, probs, rowdot,
+                                              st, "pooled dS")))
     return rc;
   // dQ_c[Qb,D] = dS k_c
-  if ((rc = launch_gemm<0, 1, kEpiStore>(ds, Qb, Kb, kc, Kb, D, dqc, BH, Qb, D, Kb, 1.f, nullptr, nullptr, st,
+  if ((rc = launch_gemm<0, 1, kEpiStore>(ds, Qb, Kb, pitch, kc, Kb, D, dqc, 0, BH, Qb, D, Kb, 1.f, nullptr, nullptr, st,
                                          "pooled dQ")))
     return rc;
   // dK_c[Kb,D] = dS^T q_c
-  return launch_gemm<1, 1, kEpiStore>(ds, Qb, Kb, qc, Qb, D, dkc, BH, Kb, D, Qb, 1.f, nullptr, nullptr, st, "pooled dK");
+  return launch_gemm<1, 1, kEpiStore>(ds, Qb, Kb, pitch, qc, Qb, D, dkc, 0, BH, Kb, D, Qb, 1.f, nullptr, nullptr, st,
+                                      "pooled dK");
 }

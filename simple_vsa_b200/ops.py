@@ -245,6 +245,15 @@ def sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be: int, scal
     return dq, dk, dv
 
 
+def pooled_probs(scores_shape, like: Tensor) -> Tensor:
+    """Buffer ``[B,H,Qb,pitch]`` for the pooled probabilities or dS of ``Kb <= pitch`` key blocks.  In 16-bit types a row
+    starts on a 16-byte boundary, which TMA asks of a matrix operand: with dense rows, block counts that are not
+    multiples of eight kept the pooled products on the CUDA cores.  The columns from ``Kb`` on are never read."""
+    B, H, Qb, Kb = scores_shape
+    pitch = Kb if like.dtype == torch.float32 else -(-Kb // 8) * 8
+    return torch.empty((B, H, Qb, pitch), device=like.device, dtype=like.dtype)
+
+
 def pooled_forward(q, k, v, kv_sizes, q_sizes, be: int, scale: float, topk: int):
     """Block means, pooled scores/probabilities/output and the Top-K routing table."""
     B, H, Lq, D = q.shape
@@ -259,10 +268,10 @@ def pooled_forward(q, k, v, kv_sizes, q_sizes, be: int, scale: float, topk: int)
     call("vsa_block_mean3_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), q_sizes.data_ptr(), kv_sizes.data_ptr(),
          qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), B * H, Lq, Lkv, D, be, dt, st)
     scores = torch.empty((B, H, Qb, Kb), device=dev, dtype=ty)
-    probs = torch.empty_like(scores)
+    probs = pooled_probs(scores.shape, scores)
     out_c = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
-    call("vsa_coarse_fwd", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
-         out_c.data_ptr(), B * H, Qb, Kb, D, scale, dt, st)
+    call("vsa_coarse_fwd_pitched", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
+         out_c.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
     selected = torch.empty((B, H, Qb, topk), device=dev, dtype=torch.int32)
     call("vsa_topk", scores.data_ptr(), selected.data_ptr(), B * H * Qb, Kb, topk, dt, st)
     return qc, kc, vc, scores, probs, out_c, selected
@@ -357,9 +366,9 @@ class _VideoSparseAttention(torch.autograd.Function):
             ds_ws = torch.empty_like(probs)
             rowdot = torch.empty((B, H, Qb), device=q.device, dtype=torch.float32)
             dqc, dkc, dvc = torch.empty_like(qc), torch.empty_like(kc), torch.empty_like(vc)
-            call("vsa_coarse_bwd", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
+            call("vsa_coarse_bwd_pitched", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                  probs.data_ptr(), ds_ws.data_ptr(), rowdot.data_ptr(), dqc.data_ptr(), dkc.data_ptr(),
-                 dvc.data_ptr(), B * H, Qb, Kb, D, scale, dt, st)
+                 dvc.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
             del ds_ws
             # the block-mean backward of the pooled gradients rides on the stores of the fine backward
             dq, dk, dv = sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be, scale,
@@ -387,10 +396,10 @@ class _ShardedVideoSparseAttention(torch.autograd.Function):
         qc = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
         call("vsa_block_mean_fwd", q.data_ptr(), q_sizes.data_ptr(), qc.data_ptr(), B * H, Lq, D, be, dt, st)
         scores = torch.empty((B, H, Qb, Kb), device=dev, dtype=ty)
-        probs = torch.empty_like(scores)
+        probs = pooled_probs(scores.shape, scores)
         out_c = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
-        call("vsa_coarse_fwd", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
-             out_c.data_ptr(), B * H, Qb, Kb, D, scale, dt, st)
+        call("vsa_coarse_fwd_pitched", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
+             out_c.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
         selected = torch.empty((B, H, Qb, topk), device=dev, dtype=torch.int32)
         call("vsa_topk", scores.data_ptr(), selected.data_ptr(), B * H * Qb, Kb, topk, dt, st)
         del scores
@@ -429,9 +438,9 @@ class _ShardedVideoSparseAttention(torch.autograd.Function):
             ds_ws = torch.empty_like(probs)
             rowdot = torch.empty((B, H, Qb), device=q.device, dtype=torch.float32)
             dqc, dkc, dvc = torch.empty_like(qc), torch.empty_like(kc), torch.empty_like(vc)
-            call("vsa_coarse_bwd", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
+            call("vsa_coarse_bwd_pitched", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                  probs.data_ptr(), ds_ws.data_ptr(), rowdot.data_ptr(), dqc.data_ptr(), dkc.data_ptr(),
-                 dvc.data_ptr(), B * H, Qb, Kb, D, scale, dt, st)
+                 dvc.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
             del ds_ws
             inverse, offsets, counts = invert_routes(selected, Kb)
             delta = torch.empty_like(lse)

@@ -99,9 +99,9 @@ class _RasterVideoSparseAttention(torch.autograd.Function):
             ds_ws = torch.empty_like(probs)
             rowdot = torch.empty((B, H, nb), device=qt.device, dtype=torch.float32)
             dqc, dkc, dvc = torch.empty_like(qc), torch.empty_like(kc), torch.empty_like(vc)
-            call("vsa_coarse_bwd", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
+            call("vsa_coarse_bwd_pitched", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
                  probs.data_ptr(), ds_ws.data_ptr(), rowdot.data_ptr(), dqc.data_ptr(), dkc.data_ptr(),
-                 dvc.data_ptr(), B * H, nb, nb, D, scale, dt, st)
+                 dvc.data_ptr(), B * H, nb, nb, probs.shape[3], D, scale, dt, st)
             del ds_ws
             inverse, offsets, counts = ops.invert_routes(selected, nb)
             delta = torch.empty_like(lse)
