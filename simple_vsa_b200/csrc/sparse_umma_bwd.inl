@@ -139,9 +139,9 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
     for (int o = 1; o < kPer; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (part == 0) {
-      s_delta[row] = acc;
+      s_delta[row] = -acc;
       delta[qrow0 + row] = acc;
-      s_lse[row] = lse2[qrow0 + row] - log2f(scale);   // 2^(s c - lse) * scale in one exponential
+      s_lse[row] = log2f(scale) - lse2[qrow0 + row];   // 2^(s c - lse) * scale in one exponential
     }
   }
   __syncthreads();
@@ -242,6 +242,7 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
   } else {
     // elementwise warps: lane t = key token of the pair, kBwCols of the 64 query rows (columns c0..)
+    const float2 c2 = make_float2(c, c);     // two fp32 operations per instruction: dQ -1 %, dK/dV -2 % at 180 routes
     const int quarter = warp & 3;
     const int cg = (warp - 4) >> 2;
     const int c0 = cg * kBwCols;
@@ -270,14 +271,14 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           *reinterpret_cast<uint4*>(krow + kPairHalf + ch * 16) = make_uint4(0, 0, 0, 0);
         }
       }
-      float pf[kBwCols];      // 2^(S c - lse) * scale
+      float2 pf[kBwCols / 2]; // 2^(S c - lse) * scale
 #pragma unroll
       for (int j4 = 0; j4 < kBwCols / 4; ++j4) {
         const float4 l4 = *reinterpret_cast<const float4*>(s_lse + c0 + 4 * j4);
-        pf[4 * j4 + 0] = fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 0]), c, -l4.x));
-        pf[4 * j4 + 1] = fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 1]), c, -l4.y));
-        pf[4 * j4 + 2] = fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 2]), c, -l4.z));
-        pf[4 * j4 + 3] = fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 3]), c, -l4.w));
+        const float2 x = fma2(word_pair(sv + 4 * j4), c2, make_float2(l4.x, l4.y));
+        const float2 y = fma2(word_pair(sv + 4 * j4 + 2), c2, make_float2(l4.z, l4.w));
+        pf[2 * j4] = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+        pf[2 * j4 + 1] = make_float2(fast_exp2(y.x), fast_exp2(y.y));
       }
       bool ds_free;
       ok = VSA_WARP_WAIT_TEST(bar(DQ_DP_FULL + b), (p / kDqBufs) & 1, bar(DQ_DS_EMPTY), (p & 1) ^ 1, &ds_free);
@@ -293,10 +294,10 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
       for (int j4 = 0; j4 < kBwCols / 4; ++j4) {
         const float4 d4 = *reinterpret_cast<const float4*>(s_delta + c0 + 4 * j4);
-        packed[2 * j4] = Elem<elem_t>::pack(pf[4 * j4 + 0] * (__uint_as_float(dv[4 * j4 + 0]) - d4.x),
-                                   pf[4 * j4 + 1] * (__uint_as_float(dv[4 * j4 + 1]) - d4.y));
-        packed[2 * j4 + 1] = Elem<elem_t>::pack(pf[4 * j4 + 2] * (__uint_as_float(dv[4 * j4 + 2]) - d4.z),
-                                       pf[4 * j4 + 3] * (__uint_as_float(dv[4 * j4 + 3]) - d4.w));
+        const float2 x = mul2(pf[2 * j4], add2(word_pair(dv + 4 * j4), make_float2(d4.x, d4.y)));
+        const float2 y = mul2(pf[2 * j4 + 1], add2(word_pair(dv + 4 * j4 + 2), make_float2(d4.z, d4.w)));
+        packed[2 * j4] = Elem<elem_t>::pack(x.x, x.y);
+        packed[2 * j4 + 1] = Elem<elem_t>::pack(y.x, y.y);
       }
       if (!live) {   // a padding key row: its scores come from whatever sits in K and V there
 #pragma unroll
@@ -567,6 +568,7 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
   } else {
     // elementwise warps: lane t = query row of the pair, kBwCols of the 64 key tokens (columns c0..)
+    const float2 c2 = make_float2(c, c);
     const int quarter = warp & 3;
     const int cg = (warp - 4) >> 2;
     const int c0 = cg * kBwCols;
@@ -614,7 +616,11 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       float pf[kBwCols];
       if (!ragged) {
 #pragma unroll
-        for (int j = 0; j < kBwCols; ++j) pf[j] = fast_exp2(fmaf(__uint_as_float(sv[j]), c, -lse));
+        for (int j = 0; j < kBwCols / 2; ++j) {
+          const float2 x = fma2(word_pair(sv + 2 * j), c2, make_float2(-lse, -lse));
+          pf[2 * j] = fast_exp2(x.x);
+          pf[2 * j + 1] = fast_exp2(x.y);
+        }
       } else {   // scores of a padding column come from whatever sits in K there: select, do not multiply
 #pragma unroll
         for (int j = 0; j < kBwCols; ++j)
@@ -643,9 +649,10 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       uint32_t pg[kBwCols / 2];
       if (!ragged) {
 #pragma unroll
-        for (int j2 = 0; j2 < kBwCols / 2; ++j2)
-          pg[j2] = Elem<elem_t>::pack(pf[2 * j2] * (__uint_as_float(dvv[2 * j2]) - dl),
-                             pf[2 * j2 + 1] * (__uint_as_float(dvv[2 * j2 + 1]) - dl));
+        for (int j2 = 0; j2 < kBwCols / 2; ++j2) {
+          const float2 x = mul2(make_float2(pf[2 * j2], pf[2 * j2 + 1]), add2(word_pair(dvv + 2 * j2), make_float2(-dl, -dl)));
+          pg[j2] = Elem<elem_t>::pack(x.x, x.y);
+        }
       } else {   // dP of a padding column comes from whatever sits in V there
 #pragma unroll
         for (int j2 = 0; j2 < kBwCols / 2; ++j2) {

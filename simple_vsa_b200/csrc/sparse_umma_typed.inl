@@ -227,9 +227,10 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     float* m_warp = reinterpret_cast<float*>(sm + FwdSmem::m_warp);
     float* m_col = reinterpret_cast<float*>(sm + FwdSmem::m_col);
     float* l_col = reinterpret_cast<float*>(sm + FwdSmem::l_col);
-    float lsum[kEwCols];
+    float2 lsum[kEwCols / 2];
+    const float2 c2 = make_float2(c, c);
 #pragma unroll
-    for (int j = 0; j < kEwCols; ++j) lsum[j] = 0.f;
+    for (int j = 0; j < kEwCols / 2; ++j) lsum[j] = make_float2(0.f, 0.f);
 
     for (int p = 0; p < n_pairs && ok; ++p) {
       const int s = p & 1;
@@ -237,6 +238,7 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int idx = 2 * p + half;
       const int valid = idx < n_live ? (int)tile_valid[idx] : 0;
       const bool live = r < valid;
+      const bool full = valid >= (quarter & 1) * 32 + 32;    // every token of this warp is live
       const int sb = p % kSBufs;
       // the score accumulator and the free P buffer (released by the O^T MMA two pairs back) in one round trip
       ok = VSA_WARP_WAIT2(bar(S_FULL + sb), (p / kSBufs) & 1, bar(P_EMPTY + s), ph ^ 1);
@@ -256,34 +258,44 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           if (lane == 0) m_warp[quarter * 64 + c0 + j] = x;
         }
         named_barrier(1, kEwThreads);
-        if (st < 64) m_col[st] = fmaxf(fmaxf(m_warp[st], m_warp[64 + st]), fmaxf(m_warp[128 + st], m_warp[192 + st])) + kShiftBias;
+        if (st < 64) m_col[st] = -(fmaxf(fmaxf(m_warp[st], m_warp[64 + st]), fmaxf(m_warp[128 + st], m_warp[192 + st])) + kShiftBias);
         named_barrier(1, kEwThreads);
       }
-      // padding rows of a ragged tile (and the repeated tile of an odd tail): whatever sits in V there
-      // must not reach the tensor core, where 0 * NaN would poison the sum
-      if (!live && cg == 0) {
-        ok = VSA_WAIT(bar(V_FULL + s), ph);
-        uint8_t* vrow = sm + FwdSmem::v + s * kPairBytes + t * 128;
+      // This warp's 32 key tokens are all live: no mask (a select per score) and nothing of V to clear.  The softmax warps'
+      // dependent issue is one of the two bounds of this kernel: with the mask out of full tiles and two fp32 operations
+      // per instruction, [1, 8, 92160, 128], topk 180: 5.79 -> 5.62 ms.
+      if (!full) {
+        // padding rows of a ragged tile (and the repeated tile of an odd tail): whatever sits in V there
+        // must not reach the tensor core, where 0 * NaN would poison the sum
+        if (!live && cg == 0) {
+          ok = VSA_WAIT(bar(V_FULL + s), ph);
+          uint8_t* vrow = sm + FwdSmem::v + s * kPairBytes + t * 128;
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          *reinterpret_cast<uint4*>(vrow + ch * 16) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(vrow + kPairHalf + ch * 16) = make_uint4(0, 0, 0, 0);
+          for (int ch = 0; ch < 8; ++ch) {
+            *reinterpret_cast<uint4*>(vrow + ch * 16) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(vrow + kPairHalf + ch * 16) = make_uint4(0, 0, 0, 0);
+          }
         }
+        ok = __all_sync(0xffffffffu, ok);     // keep the warp's control flow uniform
+        if (!ok) break;
       }
-      ok = __all_sync(0xffffffffu, ok);     // keep the warp's control flow uniform
-      if (!ok) break;
       uint32_t packed[kEwCols / 2];
+      auto exponentiate = [&](auto masked) {
 #pragma unroll
-      for (int j4 = 0; j4 < kEwCols / 4; ++j4) {
-        const float4 m4 = *reinterpret_cast<const float4*>(m_col + c0 + 4 * j4);
-        const float p0 = live ? fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 0]), c, -m4.x)) : 0.f;
-        const float p1 = live ? fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 1]), c, -m4.y)) : 0.f;
-        const float p2 = live ? fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 2]), c, -m4.z)) : 0.f;
-        const float p3 = live ? fast_exp2(fmaf(__uint_as_float(sv[4 * j4 + 3]), c, -m4.w)) : 0.f;
-        lsum[4 * j4 + 0] += p0; lsum[4 * j4 + 1] += p1; lsum[4 * j4 + 2] += p2; lsum[4 * j4 + 3] += p3;
-        packed[2 * j4] = Elem<elem_t>::pack(p0, p1);
-        packed[2 * j4 + 1] = Elem<elem_t>::pack(p2, p3);
-      }
+        for (int j4 = 0; j4 < kEwCols / 4; ++j4) {
+          const float4 m4 = *reinterpret_cast<const float4*>(m_col + c0 + 4 * j4);
+          const float2 x = fma2(word_pair(sv + 4 * j4), c2, make_float2(m4.x, m4.y));
+          const float2 y = fma2(word_pair(sv + 4 * j4 + 2), c2, make_float2(m4.z, m4.w));
+          float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y)), f = make_float2(fast_exp2(y.x), fast_exp2(y.y));
+          if (decltype(masked)::value && !live) e = f = make_float2(0.f, 0.f);
+          lsum[2 * j4] = add2(lsum[2 * j4], e);
+          lsum[2 * j4 + 1] = add2(lsum[2 * j4 + 1], f);
+          packed[2 * j4] = Elem<elem_t>::pack(e.x, e.y);
+          packed[2 * j4 + 1] = Elem<elem_t>::pack(f.x, f.y);
+        }
+      };
+      if (full) exponentiate(std::false_type{});
+      else exponentiate(std::true_type{});
       uint8_t* prow = sm + FwdSmem::p + s * kPairHalf + t * 128;
 #pragma unroll
       for (int ch = 0; ch < kEwCols / 8; ++ch)     // this thread's query rows are 16-byte chunks of row t
@@ -298,7 +310,7 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // ---- epilogue: reduce the row sums across lanes (fixed order), normalise O^T, transpose via shared memory ----
 #pragma unroll
     for (int j = 0; j < kEwCols; ++j) {
-      const float x = warp_sum(lsum[j]);
+      const float x = warp_sum((j & 1) ? lsum[j / 2].y : lsum[j / 2].x);
       if (lane == 0) m_warp[quarter * 64 + c0 + j] = x;       // the maxima scratch is free by now
     }
     named_barrier(1, kEwThreads);
@@ -350,7 +362,7 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     if (st < 64) {
       const float l = l_col[st];
-      lse2[bh * Lq + (long long)qtile * kTile + st] = (redo || n_pairs == 0) ? NAN : m_col[st] + log2f(l);
+      lse2[bh * Lq + (long long)qtile * kTile + st] = (redo || n_pairs == 0) ? NAN : log2f(l) - m_col[st];
     }
   }
   tc_fence_before();
