@@ -13,8 +13,8 @@
 // (576); tensor work 1024 / 1536 / 2560 cycles; exponentials 1024 cycles (16 per clock and SM) in every pass.
 //
 // Measured before (four or two 64-token tiles per block row, mma.sync at D = 64) -> now, ms for forward / dQ / dK/dV:
-//   [1, 8, 92160, 128], blocks of 128, topk 90:   5.77 / 8.11 / 9.69  -> 3.82 / 5.78 / 7.12   (1140 / 1130 / 1220 TFLOP/s)
-//   [1, 10, 40960, 128], blocks of 256, topk 20:  1.71 / 2.10 / 2.51  -> 1.04 / 1.44 / 1.78
+//   [1, 8, 92160, 128], blocks of 128, topk 90:   5.77 / 8.11 / 9.69  -> 3.55 / 5.80 / 7.13   (1225 / 1125 / 1220 TFLOP/s)
+//   [1, 10, 40960, 128], blocks of 256, topk 20:  1.71 / 2.10 / 2.51  -> 0.99 / 1.44 / 1.79
 //   [1, 12, 16384, 64], blocks of 128, topk 16:   0.41 / 0.50 / 0.70  -> 0.26 / 0.32 / 0.37
 // What bounds them now: no single pipe (ncu on [1, 2, 46080, 128]: tensor 47 / 51 / 61 %, exponentials 50 / 34 / 31 %) but the
 // chain product -> elementwise -> product of a tile, of which three (forward) and two (backward) are in flight; at 92k
@@ -44,11 +44,11 @@ __device__ __forceinline__ void wide_issue_scores(uint32_t d_tmem, uint32_t a_ti
 }
 // D[128 x HD] (+)= A[128 x ROWS] (tensor memory, 16-bit) B[ROWS x HD] (dims contiguous).  The A columns were written by
 // column groups of GROUP scores each, every group packing its half-width result at the start of its own columns.
-template <int HD, int ROWS, int GROUP>
+template <int HD, int ROWS, int GROUP, int TILE = ROWS>
 __device__ __forceinline__ void wide_issue_product(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_tile, bool accumulate) {
   constexpr uint32_t idesc = instr_desc(128, HD, 0, 1, kInFmt);
   constexpr uint32_t hi = desc_hi(1024);
-  const uint32_t b0 = desc_lo(b_tile, ROWS * 128);
+  const uint32_t b0 = desc_lo(b_tile, TILE * 128);
   const uint32_t acc0 = accumulate ? 1u : 0u;
 #pragma unroll
   for (int ks = 0; ks < ROWS / 16; ++ks)
@@ -119,7 +119,7 @@ struct WfSmem {
 };
 static_assert(WfSmem<128>::total <= 232448, "shared memory of the wide forward");
 enum WfBar { WF_Q_FULL = 0, WF_K_FULL = 1, WF_K_EMPTY = 4, WF_V_FULL = 7, WF_V_EMPTY = 10, WF_S_FULL = 13, WF_S_EMPTY = 16,
-             WF_P_FULL = 19, WF_M_FULL = 22, WF_O_FULL = 23 };
+             WF_P_FULL = 19, WF_P2_FULL = 22, WF_M_FULL = 25, WF_O_FULL = 26 };
 
 template <int HD>
 __global__ void __launch_bounds__(kWfThreads, 1)
@@ -158,7 +158,8 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       mbar_init(bar(WF_V_EMPTY + i), 1);
       mbar_init(bar(WF_S_FULL + i), 1);
       mbar_init(bar(WF_S_EMPTY + i), 1);
-      mbar_init(bar(WF_P_FULL + i), 4);
+      mbar_init(bar(WF_P_FULL + i), 4);        // the first and the second 64 keys of a tile
+      mbar_init(bar(WF_P2_FULL + i), 4);
     }
     mbar_init(bar(WF_M_FULL), 4);
     mbar_init(bar(WF_O_FULL), 1);
@@ -220,7 +221,11 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         ok = VSA_WAIT(bar(WF_V_FULL + s), (p / Sm::stages) & 1) && VSA_WAIT(bar(WF_P_FULL + b), (p / kWfGroups) & 1);
         if (!ok) break;
         tc_fence_after();
-        wide_issue_product<HD, 128, 128>(tmem_o, tmem + b * 128, base + Sm::v + s * Sm::tile, p > 0);
+        wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128, base + Sm::v + s * Sm::tile, p > 0);
+        ok = VSA_WAIT(bar(WF_P2_FULL + b), (p / kWfGroups) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128 + 32, base + Sm::v + s * Sm::tile + 64 * 128, true);
         mma_commit(bar(WF_V_EMPTY + s));
         mma_commit(bar(WF_S_EMPTY + b));
       }
@@ -273,6 +278,8 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         fence_proxy_async_smem();
       }
       const float2 c2 = make_float2(c, c), m2 = make_float2(neg_m, neg_m);
+      // P is handed over in two halves, so that its product starts under the second: 3.82 -> 3.55 ms and 1.04 -> 0.99 ms on the
+      // first two shapes above.
       // P over scores that this thread has already read.  Full and ragged tiles are separate code: with one body the
       // compiler turned the mask into two more instructions per score for every tile.
       auto exponentiate = [&](auto ragged) {
@@ -295,14 +302,16 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             pk[i] = Elem<elem_t>::pack(e.x, e.y);
           }
           tmem_st(s_addr + 16 * j, pk);
+          if (j & 1) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar((j == 1 ? WF_P_FULL : WF_P2_FULL) + g));
+          }
         }
       };
       if (valid == kWRows) exponentiate(std::false_type{});
       else exponentiate(std::true_type{});
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(WF_P_FULL + g));
     }
     if (!ok && lane == 0) report_timeout(43);
 
