@@ -217,7 +217,10 @@ static int sparse_fwd_dispatch(const void* q, const void* k, const void* v, cons
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
     return sparse_fwd_tc(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, false, st, out_c,
                          gate, out_comb);
-  rc = sparse_fwd_scalar(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st);
+  if (!scalar_forced() && sparse_f32_eligible(D, be, dtype, BH, {q, k, v, out}))
+    rc = sparse_fwd_f32(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, st);
+  else
+    rc = sparse_fwd_scalar(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st);
   if (rc || !out_comb) return rc;
   return combine_fwd(out, out_c, gate, out_comb, BH, Lq, D, be, dtype, st);
 }
@@ -270,6 +273,9 @@ int vsa_sparse_bwd_dq(const void* dout, const void* q, const void* k, const void
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
     return sparse_dq_tc(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                         dtype, (cudaStream_t)stream);
+  if (!scalar_forced() && sparse_f32_eligible(D, be, dtype, BH, {dout, q, k, v, dq}))
+    return sparse_dq_f32(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
+                         (cudaStream_t)stream);
   return sparse_dq_scalar(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream);
 }
@@ -288,6 +294,9 @@ int vsa_sparse_bwd_dkdv(const void* dout, const void* q, const void* k, const vo
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
     return sparse_dkdv_tc(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                           topk, scale, dtype, (cudaStream_t)stream);
+  if (!scalar_forced() && sparse_f32_eligible(D, be, dtype, BH, {dout, q, k, v, dk, dv}))
+    return sparse_dkdv_f32(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be, topk,
+                           scale, (cudaStream_t)stream);
   return sparse_dkdv_scalar(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream);
 }

@@ -1,5 +1,7 @@
 // Internal launchers shared between the translation units of the library.
 #pragma once
+
+#include <initializer_list>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -50,6 +52,18 @@ int sparse_dkdv_scalar(const void* dout, const void* q, const void* k, const voi
                        const float* delta, const int32_t* counts, const int32_t* offsets, const int32_t* inverse,
                        const int32_t* kv_sizes, void* dk, void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be,
                        int topk, float scale, int dtype, cudaStream_t st);
+
+// ---- fp32 on 64 x 64 tiles, head dim 64 or 128, block volume 64, 128 or 256 (sparse_f32.cu) --------------------
+// operands: every tensor of the call that is read or written in 16-byte pieces
+bool sparse_f32_eligible(int D, int be, int dtype, int64_t BH, std::initializer_list<const void*> operands);
+int sparse_fwd_f32(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes, void* out,
+                   float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale, cudaStream_t st);
+int sparse_dq_f32(const void* dout, const void* q, const void* k, const void* v, const void* out_s, const float* lse2,
+                  const int32_t* selected, const int32_t* kv_sizes, float* delta, void* dq, int64_t BH, int64_t Lq, int64_t Lkv,
+                  int D, int be, int topk, float scale, cudaStream_t st);
+int sparse_dkdv_f32(const void* dout, const void* q, const void* k, const void* v, const float* lse2, const float* delta,
+                    const int32_t* counts, const int32_t* offsets, const int32_t* inverse, const int32_t* kv_sizes, void* dk,
+                    void* dv, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale, cudaStream_t st);
 
 // ---- tensor-core kernels, bf16 or fp16, head dim 64 or 128, block volume 64, 128 or 256 (sparse_mma.cu) ------
 bool sparse_tc_eligible(int D, int be, int dtype);
