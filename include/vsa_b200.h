@@ -349,6 +349,46 @@ int vsa_gather_rows(const void* src, const int32_t* map, void* dst,
  * kernels (everything else the reference accepts, and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
 int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
 
+/* ---- the whole operator in one call per direction ------------------------------------------------------------
+ * The same launches as the entry points above, in the order the operator needs them, so that a host pays for one call
+ * instead of four (forward) or five (backward): vsa_block_mean3_fwd, vsa_coarse_fwd_pitched, vsa_topk,
+ * vsa_sparse_fwd_combine; vsa_combine_bwd, vsa_coarse_bwd_pitched, vsa_route_invert, vsa_sparse_bwd_dq_fused,
+ * vsa_sparse_bwd_dkdv_fused.  Field names and layouts are theirs; gate and dgate may be NULL.
+ * Replaces the driver _vsa_with_sparse_executor: vsa/triton_impl.py:1655-1731. */
+typedef struct {
+  const void *q, *k, *v, *gate;
+  const int32_t *q_sizes, *kv_sizes;
+  void *q_mean, *k_mean, *v_mean, *scores, *probs, *out_c;
+  int32_t* selected;
+  void* out_s;
+  float* lse2;
+  void* out;
+  int64_t BH, Lq, Lkv;
+  int D, be, topk, pitch;
+  float scale;
+  int dtype;
+} VsaOperatorFwd;
+
+typedef struct {
+  const void *dout, *q, *k, *v, *gate, *out_s;
+  const float* lse2;
+  const int32_t *selected, *q_sizes, *kv_sizes;
+  const void *q_mean, *k_mean, *v_mean, *probs, *out_c;
+  void *d_out_c, *dscores_ws;
+  float* rowdot_ws;
+  void *dq_mean, *dk_mean, *dv_mean;
+  int32_t *counts, *offsets, *inverse, *cursor_ws;
+  float* delta;
+  void *dq, *dk, *dv, *dgate;
+  int64_t BH, Lq, Lkv;
+  int D, be, topk, pitch;
+  float scale;
+  int dtype;
+} VsaOperatorBwd;
+
+int vsa_operator_fwd(const VsaOperatorFwd* a, void* stream);
+int vsa_operator_bwd(const VsaOperatorBwd* a, void* stream);
+
 /* ---- raster-order activations: the tiling front end folded into the kernels --------------------------------
  * (No single reference counterpart: the reference tiles with index ops, vsa/fastvideo_tiling.py:128-145, and model
  * code transposes [B,S,H,D] to [B,H,L,D] around the operator.)  A model keeps q/k/v, the gate and the output as

@@ -18,6 +18,25 @@ ERR_BAD_ARGUMENT, ERR_UNSUPPORTED, ERR_LAUNCH, ERR_DEVICE_TIMEOUT = -1, -2, -3, 
 
 P, I, L, F = c_void_p, c_int, c_int64, c_float
 
+
+class OperatorFwd(ctypes.Structure):
+    """``VsaOperatorFwd`` of the header."""
+    _fields_ = [(n, P) for n in ("q", "k", "v", "gate", "q_sizes", "kv_sizes", "q_mean", "k_mean", "v_mean", "scores", "probs",
+                                 "out_c", "selected", "out_s", "lse2", "out")] + \
+               [(n, L) for n in ("BH", "Lq", "Lkv")] + [(n, I) for n in ("D", "be", "topk", "pitch")] + \
+               [("scale", F), ("dtype", I)]
+
+
+class OperatorBwd(ctypes.Structure):
+    """``VsaOperatorBwd`` of the header."""
+    _fields_ = [(n, P) for n in ("dout", "q", "k", "v", "gate", "out_s", "lse2", "selected", "q_sizes", "kv_sizes", "q_mean",
+                                 "k_mean", "v_mean", "probs", "out_c", "d_out_c", "dscores_ws", "rowdot_ws", "dq_mean",
+                                 "dk_mean", "dv_mean", "counts", "offsets", "inverse", "cursor_ws", "delta", "dq", "dk", "dv",
+                                 "dgate")] + \
+               [(n, L) for n in ("BH", "Lq", "Lkv")] + [(n, I) for n in ("D", "be", "topk", "pitch")] + \
+               [("scale", F), ("dtype", I)]
+
+
 # name -> argument types, in the order of include/vsa_b200.h
 SIGNATURES = {
     "vsa_block_mean3_fwd": [P, P, P, P, P, P, P, P, L, L, L, I, I, I, P],
@@ -55,6 +74,8 @@ SIGNATURES = {
     "vsa_device_status": [P],
     "vsa_selftest_wait_timeout": [L, P, P],
     "vsa_combine_bwd": [P, P, P, P, P, L, L, I, I, I, P],
+    "vsa_operator_fwd": [ctypes.POINTER(OperatorFwd), P],
+    "vsa_operator_bwd": [ctypes.POINTER(OperatorBwd), P],
 }
 PLAIN = {"vsa_last_error_string": ([], c_char_p), "vsa_version": ([], c_int),
          "vsa_launch_count": ([], c_int64),

@@ -620,4 +620,41 @@ int vsa_combine_bwd(const void* dout, const void* gate, const void* out_c, void*
   return combine_bwd(dout, gate, out_c, d_out_c, dgate, BH, Lq, D, be, dtype, (cudaStream_t)stream);
 }
 
+int vsa_operator_fwd(const VsaOperatorFwd* a, void* stream) {
+  VSA_REQUIRE(a, "operator forward: null pointer");
+  int rc = check_sparse(a->BH, a->Lq, a->Lkv, a->D, a->be, a->topk, a->dtype);
+  if (rc) return rc;
+  const int Qb = (int)(a->Lq / a->be), Kb = (int)(a->Lkv / a->be);
+  if ((rc = vsa_block_mean3_fwd(a->q, a->k, a->v, a->q_sizes, a->kv_sizes, a->q_mean, a->k_mean, a->v_mean, a->BH, a->Lq,
+                                a->Lkv, a->D, a->be, a->dtype, stream)))
+    return rc;
+  if ((rc = vsa_coarse_fwd_pitched(a->q_mean, a->k_mean, a->v_mean, a->scores, a->probs, a->out_c, a->BH, Qb, Kb, a->pitch, a->D,
+                                   a->scale, a->dtype, stream)))
+    return rc;
+  if ((rc = vsa_topk(a->scores, a->selected, a->BH * Qb, Kb, a->topk, a->dtype, stream))) return rc;
+  return vsa_sparse_fwd_combine(a->q, a->k, a->v, a->selected, a->kv_sizes, a->out_s, a->lse2, a->out_c, a->gate, a->out, a->BH,
+                                a->Lq, a->Lkv, a->D, a->be, a->topk, a->scale, a->dtype, stream);
+}
+
+int vsa_operator_bwd(const VsaOperatorBwd* a, void* stream) {
+  VSA_REQUIRE(a, "operator backward: null pointer");
+  int rc = check_sparse(a->BH, a->Lq, a->Lkv, a->D, a->be, a->topk, a->dtype);
+  if (rc) return rc;
+  const int Qb = (int)(a->Lq / a->be), Kb = (int)(a->Lkv / a->be);
+  if ((rc = vsa_combine_bwd(a->dout, a->gate, a->out_c, a->d_out_c, a->dgate, a->BH, a->Lq, a->D, a->be, a->dtype, stream)))
+    return rc;
+  if ((rc = vsa_coarse_bwd_pitched(a->d_out_c, a->out_c, a->q_mean, a->k_mean, a->v_mean, a->probs, a->dscores_ws, a->rowdot_ws,
+                                   a->dq_mean, a->dk_mean, a->dv_mean, a->BH, Qb, Kb, a->pitch, a->D, a->scale, a->dtype, stream)))
+    return rc;
+  if ((rc = vsa_route_invert(a->selected, a->counts, a->offsets, a->inverse, a->cursor_ws, a->BH, Qb, Kb, a->topk, stream)))
+    return rc;
+  if ((rc = vsa_sparse_bwd_dq_fused(a->dout, a->q, a->k, a->v, a->out_s, a->lse2, a->selected, a->kv_sizes, a->delta, a->dq,
+                                    a->dq_mean, a->q_sizes, a->BH, a->Lq, a->Lkv, a->D, a->be, a->topk, a->scale, a->dtype,
+                                    stream)))
+    return rc;
+  return vsa_sparse_bwd_dkdv_fused(a->dout, a->q, a->k, a->v, a->lse2, a->delta, a->counts, a->offsets, a->inverse, a->kv_sizes,
+                                   a->dk, a->dv, a->dk_mean, a->dv_mean, a->BH, a->Lq, a->Lkv, a->D, a->be, a->topk, a->scale,
+                                   a->dtype, stream);
+}
+
 }  // extern "C"

@@ -105,7 +105,17 @@ def _sizes(sizes: Tensor, device) -> Tensor:
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)     # the handle alone, without a Stream object around it
+
+
+def _spans(*nbytes: int):
+    """Offsets of consecutive pieces of one buffer, each on a 256-byte boundary, and the buffer's size (the last entry)."""
+    at, out = 0, []
+    for n in nbytes:
+        out.append(at)
+        at += -(-n // 256) * 256
+    out.append(at)
+    return out
 
 
 def _ptr(t: Optional[Tensor]):
@@ -204,6 +214,11 @@ def _sparse_backward_stored_ds(dout, q, k, v, out_s, lse, selected, kv_sizes, be
     return dq, dk, dv
 
 
+def _stored_ds(D: int, be: int, topk: int, dt: int) -> bool:
+    return os.environ.get("VSA_B200_BACKWARD", "") == "stored_ds" and \
+        bool(_lib.lib.vsa_sparse_bwd_ds_supported(D, be, topk, dt))
+
+
 def sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be: int, scale: float, pooled_grads=None):
     """dQ, dK, dV of the fine branch.  ``pooled_grads = (dq_mean, dk_mean, dv_mean, q_sizes)`` folds the
     block-mean backward of the pooled branch into the same kernels' stores.
@@ -218,8 +233,7 @@ def sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be: int, scal
     dt = _check_device_dtype(q, k, v)
     st = _stream(q.device)
     tk = selected.shape[-1]
-    if os.environ.get("VSA_B200_BACKWARD", "") == "stored_ds" and \
-            _lib.lib.vsa_sparse_bwd_ds_supported(D, be, tk, dt):
+    if _stored_ds(D, be, tk, dt):
         return _sparse_backward_stored_ds(dout, q, k, v, out_s, lse, selected, kv_sizes, be, scale, pooled_grads,
                                           dt, st)
     inverse, offsets, counts = invert_routes(selected, Lkv // be)
@@ -245,13 +259,11 @@ def sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be: int, scal
     return dq, dk, dv
 
 
-def pooled_probs(scores_shape, like: Tensor) -> Tensor:
-    """Buffer ``[B,H,Qb,pitch]`` for the pooled probabilities or dS of ``Kb <= pitch`` key blocks.  In 16-bit types a row
-    starts on a 16-byte boundary, which TMA asks of a matrix operand: with dense rows, block counts that are not
-    multiples of eight kept the pooled products on the CUDA cores.  The columns from ``Kb`` on are never read."""
-    B, H, Qb, Kb = scores_shape
-    pitch = Kb if like.dtype == torch.float32 else -(-Kb // 8) * 8
-    return torch.empty((B, H, Qb, pitch), device=like.device, dtype=like.dtype)
+def pooled_pitch(Kb: int, ty) -> int:
+    """Elements between rows of the pooled probabilities and dS.  In 16-bit types a row starts on a 16-byte boundary,
+    which TMA asks of a matrix operand: with dense rows, block counts that are not multiples of eight kept the pooled
+    products on the CUDA cores.  The columns from ``Kb`` on are never read."""
+    return Kb if ty == torch.float32 else -(-Kb // 8) * 8
 
 
 def pooled_forward(q, k, v, kv_sizes, q_sizes, be: int, scale: float, topk: int):
@@ -268,7 +280,7 @@ def pooled_forward(q, k, v, kv_sizes, q_sizes, be: int, scale: float, topk: int)
     call("vsa_block_mean3_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), q_sizes.data_ptr(), kv_sizes.data_ptr(),
          qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), B * H, Lq, Lkv, D, be, dt, st)
     scores = torch.empty((B, H, Qb, Kb), device=dev, dtype=ty)
-    probs = pooled_probs(scores.shape, scores)
+    probs = torch.empty((B, H, Qb, pooled_pitch(Kb, ty)), device=dev, dtype=ty)
     out_c = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
     call("vsa_coarse_fwd_pitched", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
          out_c.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
@@ -326,53 +338,97 @@ def sparse_attention(q, k, v, selected, variable_block_sizes, *, block_size: Blo
 
 
 class _VideoSparseAttention(torch.autograd.Function):
-    """Whole operator: pooled branch, Top-K, fine branch, gated combine -- and its backward."""
+    """Whole operator: pooled branch, Top-K, fine branch, gated combine -- and its backward.
+
+    One native call and one scratch buffer per direction: on small problems the host, not the GPU, sets the pace (host time at
+    1k tokens: forward 107 -> 74 us, training step 329 -> 210 us against separate calls and buffers).  With the timing hook
+    ``_lib.recorder`` set, the same launches go out through the separate entry points, so that each can be timed."""
 
     @staticmethod
     def forward(ctx, q, k, v, gate, kv_sizes, q_sizes, topk, be, scale, need_grad):
         B, H, Lq, D = q.shape
+        BH, Lkv = B * H, k.shape[2]
+        Qb, Kb = Lq // be, Lkv // be
         dt = _check_device_dtype(q, k, v)
         st = _stream(q.device)
-        qc, kc, vc, scores, probs, out_c, selected = pooled_forward(q, k, v, kv_sizes, q_sizes, be, scale, topk)
-        # the gated combine rides on the store of the fine output (no separate pass over out_s)
-        out_s, lse, out = sparse_forward(q, k, v, selected, kv_sizes, be, scale, need_grad, combine_with=(out_c, gate))
+        dev, ty, es = q.device, q.dtype, q.element_size()
+        pitch = pooled_pitch(Kb, ty)
+        # block means of q, k and v, pooled probabilities, row statistics: kept for the backward as one buffer
+        at = _spans(BH * Qb * D * es, BH * Kb * D * es, BH * Kb * D * es, BH * Qb * pitch * es, BH * Lq * 4)
+        state = torch.empty(at[5], device=dev, dtype=torch.uint8)
+        qc, kc, vc, probs, lse = (state.data_ptr() + o for o in at[:5])
+        scores = torch.empty((B, H, Qb, Kb), device=dev, dtype=ty)
+        out_c = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
+        selected = torch.empty((B, H, Qb, topk), device=dev, dtype=torch.int32)
+        out_s, out = torch.empty_like(q), torch.empty_like(q)
+        if _lib.recorder is None:
+            call("vsa_operator_fwd", _lib.OperatorFwd(
+                q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(gate), q_sizes.data_ptr(), kv_sizes.data_ptr(), qc, kc, vc,
+                scores.data_ptr(), probs, out_c.data_ptr(), selected.data_ptr(), out_s.data_ptr(), lse, out.data_ptr(), BH, Lq,
+                Lkv, D, be, topk, pitch, scale, dt), st)
+        else:
+            call("vsa_block_mean3_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), q_sizes.data_ptr(), kv_sizes.data_ptr(), qc,
+                 kc, vc, BH, Lq, Lkv, D, be, dt, st)
+            call("vsa_coarse_fwd_pitched", qc, kc, vc, scores.data_ptr(), probs, out_c.data_ptr(), BH, Qb, Kb, pitch, D, scale,
+                 dt, st)
+            call("vsa_topk", scores.data_ptr(), selected.data_ptr(), BH * Qb, Kb, topk, dt, st)
+            call("vsa_sparse_fwd_combine", q.data_ptr(), k.data_ptr(), v.data_ptr(), selected.data_ptr(), kv_sizes.data_ptr(),
+                 out_s.data_ptr(), lse, out_c.data_ptr(), _ptr(gate), out.data_ptr(), BH, Lq, Lkv, D, be, topk, scale, dt, st)
         if need_grad:
-            saved = [q, k, v, out_s, lse, selected, kv_sizes, q_sizes, qc, kc, vc, probs, out_c]
+            saved = [q, k, v, out_s, selected, kv_sizes, q_sizes, state, out_c]
             if gate is not None:
                 saved.append(gate)
             ctx.save_for_backward(*saved)
             ctx.has_gate = gate is not None
             ctx.be, ctx.scale = be, scale
         ctx.mark_non_differentiable(scores, selected, out_c, out_s)
+        ctx.set_materialize_grads(False)     # the four non-differentiable outputs would each get a tensor of zeros
         return out, scores, selected, out_c, out_s
 
     @staticmethod
     def backward(ctx, dout, _dscores, _dselected, _dout_c, _dout_s):
         saved = ctx.saved_tensors
-        q, k, v, out_s, lse, selected, kv_sizes, q_sizes, qc, kc, vc, probs, out_c = saved[:13]
-        gate = saved[13] if ctx.has_gate else None
+        q, k, v, out_s, selected, kv_sizes, q_sizes, state, out_c = saved[:9]
+        gate = saved[9] if ctx.has_gate else None
         be, scale = ctx.be, ctx.scale
         B, H, Lq, D = q.shape
-        Lkv = k.shape[2]
+        BH, Lkv, topk = B * H, k.shape[2], selected.shape[3]
         Qb, Kb = Lq // be, Lkv // be
         with torch.cuda.device(q.device):
             dt = _check_device_dtype(q, k, v)
             st = _stream(q.device)
-            dout = _dense(dout)
-            d_out_c = torch.empty_like(out_c)
+            dev, ty, es = q.device, q.dtype, q.element_size()
+            dout = torch.zeros_like(q) if dout is None else _dense(dout)
+            pitch = pooled_pitch(Kb, ty)
+            at = _spans(BH * Qb * D * es, BH * Kb * D * es, BH * Kb * D * es, BH * Qb * pitch * es, BH * Lq * 4)
+            state = _dense(state)
+            qc, kc, vc, probs, lse = (state.data_ptr() + o for o in at[:5])
             dgate = torch.empty_like(gate) if gate is not None else None
-            call("vsa_combine_bwd", dout.data_ptr(), _ptr(gate), out_c.data_ptr(), d_out_c.data_ptr(), _ptr(dgate),
-                 B * H, Lq, D, be, dt, st)
-            ds_ws = torch.empty_like(probs)
-            rowdot = torch.empty((B, H, Qb), device=q.device, dtype=torch.float32)
-            dqc, dkc, dvc = torch.empty_like(qc), torch.empty_like(kc), torch.empty_like(vc)
-            call("vsa_coarse_bwd_pitched", d_out_c.data_ptr(), out_c.data_ptr(), qc.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-                 probs.data_ptr(), ds_ws.data_ptr(), rowdot.data_ptr(), dqc.data_ptr(), dkc.data_ptr(),
-                 dvc.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
-            del ds_ws
-            # the block-mean backward of the pooled gradients rides on the stores of the fine backward
-            dq, dk, dv = sparse_backward(dout, q, k, v, out_s, lse, selected, kv_sizes, be, scale,
-                                         pooled_grads=(dqc, dkc, dvc, q_sizes))
+            if _lib.recorder is not None or _stored_ds(D, be, topk, dt):
+                d_out_c = torch.empty_like(out_c)
+                call("vsa_combine_bwd", dout.data_ptr(), _ptr(gate), out_c.data_ptr(), d_out_c.data_ptr(), _ptr(dgate), BH, Lq,
+                     D, be, dt, st)
+                ds_ws = torch.empty((B, H, Qb, pitch), device=dev, dtype=ty)
+                rowdot = torch.empty((B, H, Qb), device=dev, dtype=torch.float32)
+                dqc = torch.empty_like(out_c)
+                dkc, dvc = (torch.empty((B, H, Kb, D), device=dev, dtype=ty) for _ in range(2))
+                call("vsa_coarse_bwd_pitched", d_out_c.data_ptr(), out_c.data_ptr(), qc, kc, vc, probs, ds_ws.data_ptr(),
+                     rowdot.data_ptr(), dqc.data_ptr(), dkc.data_ptr(), dvc.data_ptr(), BH, Qb, Kb, pitch, D, scale, dt, st)
+                del ds_ws
+                lse_t = state[at[4]:at[4] + BH * Lq * 4].view(torch.float32).view(B, H, Lq)
+                # the block-mean backward of the pooled gradients rides on the stores of the fine backward
+                dq, dk, dv = sparse_backward(dout, q, k, v, out_s, lse_t, selected, kv_sizes, be, scale,
+                                             pooled_grads=(dqc, dkc, dvc, q_sizes))
+                return dq, dk, dv, dgate, None, None, None, None, None, None
+            to = _spans(BH * Qb * D * es, BH * Qb * pitch * es, BH * Qb * 4, BH * Qb * D * es, BH * Kb * D * es,
+                        BH * Kb * D * es, BH * Kb * 4, BH * Kb * 4, BH * Qb * topk * 4, BH * Kb * 4, BH * Lq * 4)
+            scratch = torch.empty(to[11], device=dev, dtype=torch.uint8)
+            pieces = [scratch.data_ptr() + o for o in to[:11]]
+            dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+            call("vsa_operator_bwd", _lib.OperatorBwd(
+                dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(gate), out_s.data_ptr(), lse,
+                selected.data_ptr(), q_sizes.data_ptr(), kv_sizes.data_ptr(), qc, kc, vc, probs, out_c.data_ptr(), *pieces,
+                dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _ptr(dgate), BH, Lq, Lkv, D, be, topk, pitch, scale, dt), st)
         return dq, dk, dv, dgate, None, None, None, None, None, None
 
 
@@ -396,7 +452,7 @@ class _ShardedVideoSparseAttention(torch.autograd.Function):
         qc = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
         call("vsa_block_mean_fwd", q.data_ptr(), q_sizes.data_ptr(), qc.data_ptr(), B * H, Lq, D, be, dt, st)
         scores = torch.empty((B, H, Qb, Kb), device=dev, dtype=ty)
-        probs = pooled_probs(scores.shape, scores)
+        probs = torch.empty((B, H, Qb, pooled_pitch(Kb, ty)), device=dev, dtype=ty)
         out_c = torch.empty((B, H, Qb, D), device=dev, dtype=ty)
         call("vsa_coarse_fwd_pitched", qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), scores.data_ptr(), probs.data_ptr(),
              out_c.data_ptr(), B * H, Qb, Kb, probs.shape[3], D, scale, dt, st)
