@@ -13,6 +13,8 @@
 // reference); P and dS are rounded to bf16 before their second GEMM
 // (vsa/triton_impl.py:175,960,1106-1107).
 #include "common.cuh"
+#include <type_traits>
+
 #include "kernels.h"
 
 namespace vsa {

@@ -256,34 +256,6 @@ __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16])
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Two fp32 operations per instruction (each half rounded as the scalar instruction rounds it).
-__device__ __forceinline__ uint64_t pair_bits(float2 x) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x.x), "f"(x.y));
-  return r;
-}
-__device__ __forceinline__ float2 bits_pair(uint64_t r) {
-  float2 x;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(r));
-  return x;
-}
-__device__ __forceinline__ float2 word_pair(const uint32_t* r) { return make_float2(__uint_as_float(r[0]), __uint_as_float(r[1])); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
-  return bits_pair(r);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
-  return bits_pair(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
-  return bits_pair(r);
-}
-
 __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
