@@ -16,7 +16,7 @@
 //   [1, 8, 92160, 128], blocks of 128, topk 90:   5.77 / 8.11 / 9.69  -> 3.55 / 5.80 / 7.13   (1225 / 1125 / 1220 TFLOP/s)
 //   [1, 10, 40960, 128], blocks of 256, topk 20:  1.71 / 2.10 / 2.51  -> 0.99 / 1.44 / 1.79
 //   [1, 12, 16384, 64], blocks of 128, topk 16:   0.41 / 0.50 / 0.70  -> 0.26 / 0.32 / 0.37
-// What bounds them now: no single pipe (ncu on [1, 2, 46080, 128]: tensor 47 / 51 / 61 %, exponentials 50 / 34 / 31 %) but the
+// What bounds them now: no single pipe (ncu on [1, 2, 46080, 128]: tensor 54 / 60 / 66 %, exponentials 57 / 41 / 34 %) but the
 // chain product -> elementwise -> product of a tile, of which three (forward) and two (backward) are in flight; at 92k
 // tokens the backward is within 20 % of what a long cuBLAS GEMM sustains under the board's power limit.
 //
