@@ -315,7 +315,9 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     if (!ok && lane == 0) report_timeout(43);
 
-    if (ok && n_tiles > 0) ok = VSA_WARP_WAIT(bar(WF_O_FULL), 0);      // every MMA is done: all of shared memory is free
+    // Every MMA is done and all of shared memory is free; with no live tile nobody else has waited for the load of Q, over
+    // which the rows are staged below.
+    if (ok) ok = VSA_WARP_WAIT(bar(n_tiles > 0 ? WF_O_FULL : WF_Q_FULL), 0);
     if (!ok && lane == 0) report_timeout(44);
     tc_fence_after();
     float* l_part = reinterpret_cast<float*>(sm + Sm::k);              // [groups][128]
@@ -607,7 +609,8 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (lane == 0) mbar_arrive(bar(WQ_DS_FULL + b));
     }
     if (!ok && lane == 0) report_timeout(54);
-    if (ok && n_tiles > 0) ok = VSA_WARP_WAIT(bar(WQ_ACC_FULL), 0);
+    // as in the forward: Q, over which dQ is staged, may still be landing when the route has no live tile
+    if (ok) ok = VSA_WARP_WAIT(bar(n_tiles > 0 ? WQ_ACC_FULL : WQ_QDO_FULL), 0);
     if (!ok && lane == 0) report_timeout(55);
     tc_fence_after();
     // block-mean backward folded in: query row r of the block also receives dmean[block] / max(size, 1) while r < size
@@ -616,7 +619,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const int size = q_sizes[qb];
       if (row < size - (qtile % sub) * kWRows) inv = (float)(size > 1 ? size : 1);
     }
-    uint8_t* stage = sm + Sm::q;          // every MMA is done
+    uint8_t* stage = sm + Sm::q;
     for (int j = cg; j < HD / 32; j += kWqGroups) {
       uint32_t av[32];
       if (ok && n_tiles > 0) {

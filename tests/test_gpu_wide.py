@@ -45,3 +45,49 @@ def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype):
     dead = torch.arange(be)[None, :] >= sizes[:, None]
     for x in leaves[1:]:
         assert (x.grad.view(B, H, kb, be, D)[:, :, dead.to(DEV)] == 0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("be,qb", [(128, 400), (256, 200)])
+def test_dq_of_query_blocks_without_a_live_key_is_the_pooled_gradient_alone(be, qb, D, dtype):
+    """Every other query block routes to empty blocks only, or outside the key table only: nothing of its own Q may reach its
+    dQ, which is the pooled gradient's share (or zero without one), and the blocks between them are what they are beside
+    ordinary neighbours."""
+    from simple_vsa_b200 import _lib
+    g = torch.Generator().manual_seed(be + D)
+    BH, Kb, tk, scale = 2, 8, 3, D ** -0.5
+    Lq, Lkv, code = qb * be, Kb * be, _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    new = lambda *shape: torch.randn(*shape, generator=g).to(dtype).to(DEV)
+    q, dout, k, v, dq_mean = new(BH, Lq, D), new(BH, Lq, D), new(BH, Lkv, D), new(BH, Lkv, D), new(BH, qb, D)
+    kv_sizes = torch.tensor([be, be // 2 + 3, 1, 0, 0, be, 0, 65], dtype=torch.int32, device=DEV)
+    q_sizes = torch.randint(0, be + 1, (qb,), generator=g, dtype=torch.int32)
+    ordinary = torch.rand(BH, qb, Kb, generator=g)
+    ordinary[..., 5] = 2.0                                # a full block in every row
+    ordinary = ordinary.topk(tk, dim=-1).indices.to(torch.int32)
+    dead = torch.arange(qb) % 2 == 1
+    routes = ordinary.clone()
+    routes[:, dead] = torch.tensor([3, 4, 6], dtype=torch.int32)
+    routes[:, torch.arange(qb) % 4 == 3] = torch.tensor([-1, Kb, 2 ** 30], dtype=torch.int32)
+    st = torch.cuda.current_stream().cuda_stream
+
+    def run(table, pooled):
+        sel, qs = table.to(DEV), q_sizes.to(DEV)
+        out, dq = torch.empty_like(q), torch.full_like(q, float("nan"))
+        lse, delta = torch.empty(BH, Lq, device=DEV), torch.empty(BH, Lq, device=DEV)
+        _lib.call("vsa_sparse_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), sel.data_ptr(), kv_sizes.data_ptr(), out.data_ptr(),
+                  lse.data_ptr(), BH, Lq, Lkv, D, be, tk, scale, code, st)
+        args = [dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), sel.data_ptr(),
+                kv_sizes.data_ptr(), delta.data_ptr(), dq.data_ptr()] + ([dq_mean.data_ptr(), qs.data_ptr()] if pooled else [])
+        _lib.call("vsa_sparse_bwd_dq" + ("_fused" if pooled else ""), *args, BH, Lq, Lkv, D, be, tk, scale, code, st)
+        torch.cuda.synchronize()
+        return out.cpu().view(BH, qb, be, D), dq.cpu().view(BH, qb, be, D)
+
+    rows = torch.arange(be)[None, :, None] < q_sizes[:, None, None]
+    share = torch.where(rows, dq_mean.cpu().float()[:, :, None] / q_sizes.clamp(min=1)[:, None, None], torch.zeros(())).to(dtype)
+    for pooled, want in ((False, torch.zeros_like(share)), (True, share)):
+        (out, dq), (out_ref, dq_ref) = run(routes, pooled), run(ordinary, pooled)
+        assert torch.equal(dq[:, dead], want[:, dead])
+        assert torch.isnan(out[:, dead].float()).all()
+        assert torch.equal(dq[:, ~dead], dq_ref[:, ~dead]) and torch.equal(out[:, ~dead], out_ref[:, ~dead])
+    assert _lib.device_status() == 0
