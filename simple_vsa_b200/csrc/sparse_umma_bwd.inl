@@ -141,7 +141,7 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (part == 0) {
       s_delta[row] = -acc;
       delta[qrow0 + row] = acc;
-      s_lse[row] = log2f(scale) - lse2[qrow0 + row];   // 2^(s c - lse) * scale in one exponential
+      s_lse[row] = log2f(fabsf(scale)) - lse2[qrow0 + row];   // 2^(s c - lse) * |scale| in one exponential
     }
   }
   __syncthreads();
@@ -271,7 +271,7 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           *reinterpret_cast<uint4*>(krow + kPairHalf + ch * 16) = make_uint4(0, 0, 0, 0);
         }
       }
-      float2 pf[kBwCols / 2]; // 2^(S c - lse) * scale
+      float2 pf[kBwCols / 2]; // 2^(S c - lse) * |scale|
 #pragma unroll
       for (int j4 = 0; j4 < kBwCols / 4; ++j4) {
         const float4 l4 = *reinterpret_cast<const float4*>(s_lse + c0 + 4 * j4);
@@ -332,9 +332,10 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       uint32_t av[kBwCols];
       tmem_ld(tmem_acc + lane_addr + c0, av);
       tmem_ld_wait();
+      const uint32_t sign = scale < 0.f ? 0x80000000u : 0u;
 #pragma unroll
       for (int j = 0; j < kBwCols; ++j)
-        stage[(c0 + j) * kD + t] = Elem<elem_t>::from(__uint_as_float(av[j]) + ((c0 + j) < rows_live ? gm : 0.f));
+        stage[(c0 + j) * kD + t] = Elem<elem_t>::from(__uint_as_float(av[j] ^ sign) + ((c0 + j) < rows_live ? gm : 0.f));
     } else {
       for (int j = 0; j < kBwCols; ++j) stage[(c0 + j) * kD + t] = Elem<elem_t>::from((c0 + j) < rows_live ? gm : 0.f);
     }

@@ -484,7 +484,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   tc_fence_before();
   __syncthreads();
   const float dl = elementwise ? s_delta[row] : 0.f;
-  const float neg_lse = elementwise ? log2f(scale) - lse2[row0 + row] : 0.f;     // 2^(s c - lse) * scale in one exponential
+  const float neg_lse = elementwise ? log2f(fabsf(scale)) - lse2[row0 + row] : 0.f;   // 2^(s c - lse) * |scale| in one exponential
   wide_tile_list(list, misc + 1, selected + (bh * Qb + qb) * (long long)topk, kv_sizes, topk, sub, (int)(Lkv / be), bh,
                  gridDim.y, kv_shard, tid, kWqThreads);
   tc_fence_after();
@@ -574,7 +574,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         fence_proxy_async_smem();
       }
-      float2 pf[kWqCols / 2];            // 2^(S c - lse) * scale
+      float2 pf[kWqCols / 2];            // 2^(S c - lse) * |scale|
 #pragma unroll
       for (int i = 0; i < kWqCols / 2; ++i) {
         const float2 x = fma2(word_pair(sv + 2 * i), c2, l2);
@@ -625,6 +625,10 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (ok && n_tiles > 0) {
         tmem_ld(tmem_acc + lane_addr + 32 * j, av);
         tmem_ld_wait();
+        if (scale < 0.f) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) av[i] ^= 0x80000000u;
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) av[i] = 0u;
