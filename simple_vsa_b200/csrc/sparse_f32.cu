@@ -100,14 +100,17 @@ __device__ __forceinline__ void product(float (&acc)[4][D / 16], const float* p,
   }
 }
 
+// Rows from `live` on are padding: they get zeros, not 0 * whatever stood in the rows summed over.
 template <int D>
-__device__ __forceinline__ void store_rows(float* __restrict__ g, const float (&acc)[4][D / 16], const float (&mul)[4], int tx, int ty) {
+__device__ __forceinline__ void store_rows(float* __restrict__ g, const float (&acc)[4][D / 16], const float (&mul)[4], int tx, int ty,
+                                           int live = kT) {
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int h = 0; h < D / 64; ++h)
       *reinterpret_cast<float4*>(g + (4 * ty + i) * D + 64 * h + 4 * tx) =
-          make_float4(acc[i][4 * h] * mul[i], acc[i][4 * h + 1] * mul[i], acc[i][4 * h + 2] * mul[i], acc[i][4 * h + 3] * mul[i]);
+          4 * ty + i < live ? make_float4(acc[i][4 * h] * mul[i], acc[i][4 * h + 1] * mul[i], acc[i][4 * h + 2] * mul[i], acc[i][4 * h + 3] * mul[i])
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 __device__ __forceinline__ float half_warp_max(float x) {
@@ -341,8 +344,8 @@ sparse_dkdv_f32_kernel(const float* __restrict__ dout, const float* __restrict__
     __syncthreads();
   }
   const float mk[4] = {scale, scale, scale, scale}, mv[4] = {1.f, 1.f, 1.f, 1.f};
-  store_rows<D>(dk + row0 * D, ak, mk, tx, ty);
-  store_rows<D>(dv + row0 * D, av, mv, tx, ty);
+  store_rows<D>(dk + row0 * D, ak, mk, tx, ty, valid);
+  store_rows<D>(dv + row0 * D, av, mv, tx, ty, valid);
 }
 
 template <typename Kern>

@@ -50,3 +50,21 @@ def test_fp32_tiles_match_float64(be, qb, kb, tk, D, monkeypatch):
         # error moves by a quarter with the order of the sums
         assert error[0] <= 2e-6
         assert error[0] <= 1.25 * error[1] + 1e-7
+
+
+@pytest.mark.parametrize("be,D", [(64, 64), (128, 128), (256, 64)])
+def test_padded_key_rows_get_exactly_zero_gradients_beside_a_nan(be, D):
+    """A query row whose gradient holds NaN or infinity poisons the live rows of the key blocks that it reads, as in every
+    kernel; their padding rows stay at zero."""
+    from simple_vsa_b200 import b200_sparse_attention
+    g = torch.Generator().manual_seed(be)
+    nb, sizes = 4, torch.tensor([be, 5, be - 1, be // 2])
+    q, k, v, dout = (torch.randn(1, 1, nb * be, D, generator=g).to(DEV) for _ in range(4))
+    dout[0, 0, 3, 1], dout[0, 0, be + 2, 0] = float("nan"), float("inf")
+    selected = torch.arange(nb, dtype=torch.int32).expand(1, 1, nb, nb).contiguous().to(DEV)
+    leaves = [x.requires_grad_() for x in (q, k, v)]
+    b200_sparse_attention(*leaves, selected, sizes, block_size=(1, 1, be)).backward(dout)
+    dead = (torch.arange(be)[None, :] >= sizes[:, None]).view(-1).to(DEV)
+    for x in leaves[1:]:
+        assert torch.isnan(x.grad[0, 0, ~dead]).any()
+        assert (x.grad[0, 0, dead] == 0).all()
