@@ -353,7 +353,8 @@ int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
  * The same launches as the entry points above, in the order the operator needs them, so that a host pays for one call
  * instead of four (forward) or five (backward): vsa_block_mean3_fwd, vsa_coarse_fwd_pitched, vsa_topk,
  * vsa_sparse_fwd_combine; vsa_combine_bwd, vsa_coarse_bwd_pitched, vsa_route_invert, vsa_sparse_bwd_dq_fused,
- * vsa_sparse_bwd_dkdv_fused.  Field names and layouts are theirs; gate and dgate may be NULL.
+ * vsa_sparse_bwd_dkdv_fused.  Field names and layouts are theirs; gate and dgate may be NULL.  dscores_ws is dead when dq is
+ * first written and may be its storage, where that is large enough (BH * Qb * pitch <= BH * Lq * D elements).
  * Replaces the driver _vsa_with_sparse_executor: vsa/triton_impl.py:1655-1731. */
 typedef struct {
   const void *q, *k, *v, *gate;
