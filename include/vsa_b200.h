@@ -349,6 +349,11 @@ int vsa_gather_rows(const void* src, const int32_t* map, void* dst,
  * kernels (everything else the reference accepts, and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
 int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
 
+/* The kernels that one fine pass of an ordinary call (vsa_sparse_fwd with lse2, vsa_sparse_bwd_dq, vsa_sparse_bwd_dkdv) takes:
+ * pass 0 = forward, 1 = dQ, 2 = dK/dV; L = Lq for the first two, Lkv for the third.  3 = tcgen05 on 128-row tiles, 2 = tcgen05
+ * on 64-token tiles, 1 = warp-level mma.sync, 0 = CUDA cores; negative for bad arguments. */
+int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype);
+
 /* ---- the whole operator in one call per direction ------------------------------------------------------------
  * The same launches as the entry points above, in the order the operator needs them, so that a host pays for one call
  * instead of four (forward) or five (backward): vsa_block_mean3_fwd, vsa_coarse_fwd_pitched, vsa_topk,

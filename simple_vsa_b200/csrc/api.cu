@@ -46,9 +46,11 @@ static bool mma_forced() {
   return e && std::strcmp(e, "mma") == 0;
 }
 
-// The fine kernels of an ordinary call on the tcgen05 path: head dim 128, or head dim 64 with blocks of 128 or 256 tokens.
-static bool on_umma(int D, int be, int dtype, int topk) {
-  return !scalar_forced() && !mma_forced() && (sparse_umma_eligible(D, be, dtype, topk) || sparse_wide64_eligible(D, be, dtype, topk));
+// The kernels that a pass of an ordinary call runs on: head dim 128 on tcgen05, head dim 64 with blocks of 128 or 256 tokens
+// on the 128-row tcgen05 kernels where they are the faster ones (sparse_wide64_pays).
+static bool on_umma(SparsePass pass, int64_t BH, int64_t L, int D, int be, int dtype, int topk) {
+  return !scalar_forced() && !mma_forced() &&
+         (sparse_umma_eligible(D, be, dtype, topk) || (sparse_wide64_eligible(D, be, dtype, topk) && sparse_wide64_pays(pass, BH, L, be, topk)));
 }
 
 static int check_dtype(int dtype) {
@@ -206,7 +208,7 @@ static int sparse_fwd_dispatch(const void* q, const void* k, const void* v, cons
                                void* out_comb, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk,
                                float scale, int dtype, cudaStream_t st) {
   int rc;
-  if (lse2 && on_umma(D, be, dtype, topk)) {
+  if (lse2 && on_umma(kPassForward, BH, Lq, D, be, dtype, topk)) {
     rc = sparse_fwd_umma(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, D, be, topk, scale, dtype, st, out_c, gate,
                          out_comb);
     if (rc) return rc;
@@ -267,7 +269,7 @@ int vsa_sparse_bwd_dq(const void* dout, const void* q, const void* k, const void
   int rc = check_sparse(BH, Lq, Lkv, D, be, topk, dtype);
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && out_s && lse2 && selected && kv_sizes && delta && dq, "sparse dQ: null pointer");
-  if (on_umma(D, be, dtype, topk))
+  if (on_umma(kPassDq, BH, Lq, D, be, dtype, topk))
     return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream);
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
@@ -288,7 +290,7 @@ int vsa_sparse_bwd_dkdv(const void* dout, const void* q, const void* k, const vo
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && lse2 && delta && counts && offsets && inverse && kv_sizes && dk && dv,
               "sparse dK/dV: null pointer");
-  if (on_umma(D, be, dtype, topk))
+  if (on_umma(kPassDkdv, BH, Lkv, D, be, dtype, topk))
     return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream);
   if (!scalar_forced() && sparse_tc_eligible(D, be, dtype))
@@ -313,7 +315,7 @@ int vsa_sparse_bwd_dq_fused(const void* dout, const void* q, const void* k, cons
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && out_s && lse2 && selected && kv_sizes && delta && dq && dq_mean && q_sizes,
               "sparse dQ (fused): null pointer");
-  if (on_umma(D, be, dtype, topk))
+  if (on_umma(kPassDq, BH, Lq, D, be, dtype, topk))
     return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream, dq_mean, q_sizes);
   rc = vsa_sparse_bwd_dq(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
@@ -331,7 +333,7 @@ int vsa_sparse_bwd_dkdv_fused(const void* dout, const void* q, const void* k, co
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && lse2 && delta && counts && offsets && inverse && kv_sizes && dk && dv &&
                   dk_mean && dv_mean, "sparse dK/dV (fused): null pointer");
-  if (on_umma(D, be, dtype, topk))
+  if (on_umma(kPassDkdv, BH, Lkv, D, be, dtype, topk))
     return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean);
   rc = vsa_sparse_bwd_dkdv(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
@@ -483,6 +485,13 @@ static int check_raster(const int32_t* map, int64_t rows, int heads, int64_t BH,
 int vsa_sparse_kernel_family(int D, int be, int topk, int dtype) {
   if (scalar_forced()) return 0;
   if (!mma_forced() && sparse_umma_eligible(D, be, dtype, topk)) return 2;
+  return sparse_tc_eligible(D, be, dtype) ? 1 : 0;
+}
+
+int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype) {
+  VSA_REQUIRE(pass >= 0 && pass <= 2 && BH >= 1 && be >= 1 && L >= be && L % be == 0, "sparse pass kernels: bad arguments");
+  if (scalar_forced()) return 0;
+  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return be % 128 == 0 ? 3 : 2;
   return sparse_tc_eligible(D, be, dtype) ? 1 : 0;
 }
 

@@ -286,6 +286,30 @@ bool sparse_wide64_eligible(int D, int be, int dtype, int topk) {
   return D == 64 && (be == 128 || be == 256) && (dtype == VSA_BF16 || dtype == VSA_F16) && topk * (be / kTile) <= kMaxTiles;
 }
 
+// The SM count decides between kernels only; without a device (a query on a build machine) a B200's is assumed.
+static int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+    return sms;
+  cudaGetLastError();
+  return 148;
+}
+
+// A CTA of the 128-row kernels has an SM to itself and spends several us on set-up and drain; four mma.sync CTAs (three in the
+// backward) share an SM and need little of either, so they are faster while a route holds few tiles.  us at [1, 12, 16384, 64],
+// blocks of 128, full blocks, 128-row kernels / mma.sync, by 64-token tiles per route:
+//   forward  2: 106 / 39   4: 117 / 60    8: 134 / 104   12: 149 / 149   16: 166 / 193
+//   dQ       2: 150 / 57   4: 161 / 85    8: 183 / 142   12: 204 / 199   16: 226 / 254
+//   dK/dV    2:  82 / 77   4: 108 / 120   8: 149 / 199   12: 185 / 278   16: 220 / 352
+// The forward and dQ cross between 8 and 12 tiles with blocks of 256 and on other grids too (32 to 25,600 row tiles), except
+// where the 128-row CTAs just fill the SMs once and the mma.sync CTAs have to share them: between 4 and 8 ([1, 4, 4096, 64],
+// 8 tiles: forward 15.1 / 14.1 us, dQ 22.5 / 17.2 us with the wide kernels second).
+bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
+  if (pass == kPassDkdv) return true;
+  const int64_t sms = sm_count(), rows128 = BH * (L / 128);
+  return topk * (be / kTile) > (rows128 <= sms && 2 * rows128 > sms ? 4 : 8);
+}
+
 int64_t sparse_ds_workspace_bytes(int64_t BH, int64_t Lq, int be, int topk) {
   const int64_t sub = be / kTile;
   return BH * (Lq / be) * topk * sub * sub * (int64_t)(kTile * kTile * 2);

@@ -161,6 +161,25 @@ def test_workspace_sizes_and_support_queries_need_no_gpu():
     assert lib.vsa_sparse_bwd_ds_supported(128, 64, 180, L.VSA_F32) == 0
 
 
+def test_kernels_of_a_pass():
+    import simple_vsa_b200._lib as L
+    kernels = lambda p, BH, n, D, be, tk, dt=L.VSA_BF16: L.lib.vsa_sparse_pass_kernels(p, BH, n, D, be, tk, dt)
+    for p in range(3):
+        assert kernels(p, 8, 65536, 128, 64, 16) == 2
+        assert kernels(p, 8, 65536, 128, 128, 16) == 3
+        assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F16) == 1
+        assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F32) == 0
+        assert kernels(p, 8, 65536, 64, 128, 513) == 1                     # 1026 tiles: beyond the tile list
+        # head dim 64: up to 8 tiles of 64 tokens a route the forward and dQ are faster on the warp-level kernels, up to 4 where
+        # the 128-row tiles fill the SMs (148 without a device) just once
+        assert [kernels(p, 4, 4096, 64, 128, tk) for tk in (2, 3)] == ([1, 3] if p < 2 else [3, 3])
+        assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([1, 3] if p < 2 else [3, 3])
+        assert [kernels(p, 8, 65536, 64, 128, tk) for tk in (1, 4, 5)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
+        assert [kernels(p, 8, 65536, 64, 256, tk) for tk in (1, 2, 3)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
+    assert kernels(3, 8, 65536, 128, 64, 16) == L.ERR_BAD_ARGUMENT
+    assert kernels(0, 8, 65, 128, 64, 1) == L.ERR_BAD_ARGUMENT
+
+
 def test_host_step_helpers():
     from simple_vsa_b200.host import _chunk_spans, _parse_cpulist
     for total, per in ((80, 4), (10, 4), (1, 8), (7, 3), (40, 40)):

@@ -13,7 +13,7 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("be,qb,kb,tk", [(128, 1, 1, 1), (128, 3, 7, 5), (256, 2, 5, 3), (256, 1, 9, 9)])
+@pytest.mark.parametrize("be,qb,kb,tk", [(128, 1, 1, 1), (128, 2, 5, 4), (128, 3, 7, 5), (256, 2, 5, 3), (256, 1, 9, 9)])
 def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype):
     from simple_vsa_b200 import _lib, b200_sparse_attention
     g = torch.Generator().manual_seed(be + 7 * kb + D)
@@ -56,7 +56,7 @@ def test_dq_of_query_blocks_without_a_live_key_is_the_pooled_gradient_alone(be, 
     ordinary neighbours."""
     from simple_vsa_b200 import _lib
     g = torch.Generator().manual_seed(be + D)
-    BH, Kb, tk, scale = 2, 8, 3, D ** -0.5
+    BH, Kb, tk, scale = 2, 8, 5, D ** -0.5
     Lq, Lkv, code = qb * be, Kb * be, _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
     new = lambda *shape: torch.randn(*shape, generator=g).to(dtype).to(DEV)
     q, dout, k, v, dq_mean = new(BH, Lq, D), new(BH, Lq, D), new(BH, Lkv, D), new(BH, Lkv, D), new(BH, qb, D)
@@ -67,8 +67,8 @@ def test_dq_of_query_blocks_without_a_live_key_is_the_pooled_gradient_alone(be, 
     ordinary = ordinary.topk(tk, dim=-1).indices.to(torch.int32)
     dead = torch.arange(qb) % 2 == 1
     routes = ordinary.clone()
-    routes[:, dead] = torch.tensor([3, 4, 6], dtype=torch.int32)
-    routes[:, torch.arange(qb) % 4 == 3] = torch.tensor([-1, Kb, 2 ** 30], dtype=torch.int32)
+    routes[:, dead] = torch.tensor([3, 4, 6, -2, 3], dtype=torch.int32)
+    routes[:, torch.arange(qb) % 4 == 3] = torch.tensor([-1, Kb, 2 ** 30, Kb + 1, -8], dtype=torch.int32)
     st = torch.cuda.current_stream().cuda_stream
 
     def run(table, pooled):
