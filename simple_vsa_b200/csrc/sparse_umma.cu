@@ -244,8 +244,7 @@ int check_kv_shard(int64_t Lkv, int be, int64_t* kv_shard, const char* what) {
 
 }  // namespace
 
-// The stored-dS backward walks a block of 64, 128 or 256 tokens as 1, 2 or 4 tiles of 64 tokens (its kernels' SUB parameter);
-// otherwise blocks that are multiples of 128 run on the 128-row kernels (sparse_wide.inl).
+// The 64-token kernels walk a block of 64, 128 or 256 tokens as 1, 2 or 4 tiles (their SUB parameter).
 #define VSA_BY_BLOCK_VOLUME(be_, launch_, kernel_) \
   return (be_) == 64 ? launch_(kernel_<1>) : (be_) == 128 ? launch_(kernel_<2>) : launch_(kernel_<4>)
 
@@ -276,6 +275,37 @@ constexpr float kShiftBias = 4.f;
 #define VSA_BY_DTYPE(dtype_, call_) ((dtype_) == VSA_F16 ? tc_f16::call_ : tc_bf16::call_)
 
 // ---- host entry points ---------------------------------------------------------------------------------------
+// The SM count decides between kernels only; without a device (a query on a build machine) a B200's is assumed.
+static int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+    return sms;
+  cudaGetLastError();
+  return 148;
+}
+
+// Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as tiles of 64 tokens.  Both
+// run one CTA per SM; a 128-row CTA does twice the rows in less than twice the time, so the 64-token kernels are the faster
+// ones where halving the CTAs saves no wave (times on one B200, head dim 128, full blocks, us, 64-token / 128-row):
+//   all 64-row tiles on the SMs at once ([1, 2, 4096], 2 / 8 / 32 tiles a route): forward 12.7 / 14.0, 15.2 / 16.3, 24.2 / 26.3;
+//     dQ 8.7 / 15.8, 11.7 / 19.8, 24.4 / 35.0; dK/dV 13.1 / 16.4, 18.0 / 22.4, 33.5 / 42.3;
+//   three waves against two ([1, 3, 8192]): forward 24.5 / 25.0, 31.3 / 30.1, 59.4 / 49.9; dQ 22.9 / 30.2, 31.7 / 38.0,
+//     68.3 / 67.8; dK/dV 20.9 / 17.6, 37.2 / 34.8, 86.2 / 77.5;
+//   many waves ([1, 12, 16384]): forward 139 / 140, 185 / 168, 383 / 276; dQ 175 / 181, 234 / 221, 484 / 385; dK/dV 142 / 103,
+//     244 / 175, 544 / 380.
+// A wave of dQ takes 7.3 + 0.49 n us on 64-token tiles and 15.2 + 0.61 n us on 128-row tiles, n the 64-token tiles of a route,
+// which is the comparison below; it names the faster kernel, or one within 2.5 %, at every point of 32 to 3072 row tiles x 2 to 64
+// tiles a route that was measured.  A wave of the forward costs 1.1 times as much on 128 rows and of dK/dV 1.25 times, at any n.
+bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk) {
+  if (be % 128 != 0) return false;
+  if (D == 64) return true;                       // there are no 64-token tcgen05 kernels at this head dim
+  const int64_t sms = sm_count();
+  const int64_t narrow = (BH * (L / 64) + sms - 1) / sms, wide = (BH * (L / 128) + sms - 1) / sms;
+  if (pass != kPassDq) return narrow > 1;
+  const int64_t n = (int64_t)topk * (be / 64);
+  return narrow * (60 + 4 * n) >= wide * (124 + 5 * n);
+}
+
 bool sparse_umma_eligible(int D, int be, int dtype, int topk) {
   if ((dtype != VSA_BF16 && dtype != VSA_F16) || D != 128) return false;
   if (be == 64 || be == 128 || be == 256) return topk * (be / kTile) <= kMaxTiles;
@@ -284,15 +314,6 @@ bool sparse_umma_eligible(int D, int be, int dtype, int topk) {
 
 bool sparse_wide64_eligible(int D, int be, int dtype, int topk) {
   return D == 64 && (be == 128 || be == 256) && (dtype == VSA_BF16 || dtype == VSA_F16) && topk * (be / kTile) <= kMaxTiles;
-}
-
-// The SM count decides between kernels only; without a device (a query on a build machine) a B200's is assumed.
-static int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
-    return sms;
-  cudaGetLastError();
-  return 148;
 }
 
 // A CTA of the 128-row kernels has an SM to itself and spends several us on set-up and drain; four mma.sync CTAs (three in the

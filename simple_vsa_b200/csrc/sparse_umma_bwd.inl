@@ -56,6 +56,7 @@ enum DqBar { DQ_QDO_FULL = 0, DQ_K_FULL = 1, DQ_K_EMPTY = 4, DQ_V_FULL = 7, DQ_V
              DQ_DS_EMPTY = 12, DQ_ACC_FULL = 13, DQ_S_FULL = 14, DQ_S_EMPTY = 14 + kDqBufs,
              DQ_DP_FULL = 14 + 2 * kDqBufs };
 
+template <int SUB>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                       const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -71,10 +72,10 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qtile = blockIdx.x;
   const long long bh = blockIdx.y;
-  const int Qb = (int)(Lq / kTile);
-  const int qb = qtile;
+  const int Qb = (int)(Lq / (kTile * SUB));
+  const int qb = qtile / SUB;
   const int32_t* sel = selected + (bh * Qb + qb) * (long long)topk;
-  const int n_iter = topk;
+  const int n_iter = topk * SUB;
   const float c = scale * kLog2e;
   const long long qrow0 = bh * Lq + (long long)qtile * kTile;
 
@@ -114,11 +115,11 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     tma_load_2d(base + DqSmem::d_o + kSlab, &map_do, 64, (int)qrow0, bar(DQ_QDO_FULL));
   }
   for (int it = tid; it < n_iter; it += kBwdThreads) {
-    const int kvb = sel[it];
+    const int kvb = sel[it / SUB];
     // an id outside the table is an empty tile, as route inversion treats it
-    const int left = (unsigned)kvb < (unsigned)(Lkv / kTile) ? kv_sizes[kvb] : 0;
+    const int left = (unsigned)kvb < (unsigned)(Lkv / (kTile * SUB)) ? kv_sizes[kvb] - (it % SUB) * kTile : 0;
     tile_valid[it] = (uint8_t)(left < 0 ? 0 : (left > kTile ? kTile : left));
-    tile_row[it] = left > 0 ? (int)kv_tensor_row(bh, gridDim.y, (long long)kvb * kTile, kv_shard) : 0;
+    tile_row[it] = left > 0 ? (int)kv_tensor_row(bh, gridDim.y, (long long)kvb * (kTile * SUB) + (it % SUB) * kTile, kv_shard) : 0;
   }
   if (warp >= 4 && warp < kDpWarp) {   // delta = rowsum(out_s * dout) and the saved statistic, eight threads per query row
     constexpr int kPer = kBwEwThreads / 64;            // threads per row
@@ -326,7 +327,7 @@ sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (mean_grad != nullptr) {
       const int size = q_sizes[qb];
       gm = Elem<elem_t>::to(mean_grad[(bh * Qb + qb) * (long long)kD + t]) / (float)(size > 1 ? size : 1);
-      rows_live = size;
+      rows_live = size - (qtile % SUB) * kTile;
     }
     if (ok && n_pairs > 0) {
       uint32_t av[kBwCols];

@@ -34,6 +34,7 @@ enum FwdPBar { PQ_FULL = 0, PQ_EMPTY = 2, PK_FULL = 4, PK_EMPTY = 6, PV_FULL = 8
                PP_EMPTY = 14, PO_FULL = 16, PO_EMPTY = 18, PL_FULL = 20, PL_EMPTY = 22, PS_FULL = 24,
                PS_EMPTY = 24 + kSBufs };
 
+template <int SUB>
 __global__ void __launch_bounds__(kFwdPThreads, 1)
 sparse_fwd_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                   const __grid_constant__ CUtensorMap map_v, const int32_t* __restrict__ selected,
@@ -48,8 +49,8 @@ sparse_fwd_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_q, con
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q_tiles = (int)(Lq / kTile);
   const long long n_items = (long long)q_tiles * BH;
-  const int Qb = (int)(Lq / kTile);
-  const int n_iter = topk;
+  const int Qb = (int)(Lq / (kTile * SUB));
+  const int n_iter = topk * SUB;
   const float c = scale * kLog2e;
 
   int32_t* tile_row = reinterpret_cast<int32_t*>(sm + FwdPSmem::tile_row);
@@ -102,7 +103,7 @@ sparse_fwd_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_q, con
       if (!ok) break;
       const int qtile = (int)(w % q_tiles);
       const long long bh = w / q_tiles;
-      const int32_t* sel = selected + (bh * Qb + qtile) * (long long)topk;
+      const int32_t* sel = selected + (bh * Qb + qtile / SUB) * (long long)topk;
       int32_t* rows = tile_row + b * kMaxTiles;
       uint8_t* valids = tile_valid + b * kMaxTiles;
       int n_live = 0;
@@ -110,11 +111,11 @@ sparse_fwd_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_q, con
         const int it = it0 + lane;
         int valid = 0, row = 0;
         if (it < n_iter) {
-          const int kvb = sel[it];
+          const int kvb = sel[it / SUB];
           // an id outside the table is an empty tile, as route inversion treats it
-          const int left = (unsigned)kvb < (unsigned)(Lkv / kTile) ? kv_sizes[kvb] : 0;
+          const int left = (unsigned)kvb < (unsigned)(Lkv / (kTile * SUB)) ? kv_sizes[kvb] - (it % SUB) * kTile : 0;
           valid = left < 0 ? 0 : (left > kTile ? kTile : left);
-          if (valid > 0) row = (int)kv_tensor_row(bh, BH, (long long)kvb * kTile, kv_shard);
+          if (valid > 0) row = (int)kv_tensor_row(bh, BH, (long long)kvb * (kTile * SUB) + (it % SUB) * kTile, kv_shard);
         }
         const unsigned live = __ballot_sync(0xffffffffu, valid > 0);
         if (valid > 0) {      // empty tiles are squeezed out, the routing order is kept
@@ -251,7 +252,7 @@ sparse_fwd_umma_persistent_kernel(const __grid_constant__ CUtensorMap map_q, con
       const uint8_t* valids = tile_valid + b * kMaxTiles;
       const int qtile = (int)(w % q_tiles);
       const long long bh = w / q_tiles;
-      const int qb = qtile;
+      const int qb = qtile / SUB;
       float2 lsum[kEwCols / 2];
       const float2 c2 = make_float2(c, c);
 #pragma unroll

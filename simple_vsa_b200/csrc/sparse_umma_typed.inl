@@ -61,6 +61,7 @@ constexpr int kFwdThreads = 128 + kEwThreads;   // K producer, V producer, two M
 enum FwdBar { Q_FULL = 0, K_FULL = 1, K_EMPTY = 4, V_FULL = 7, V_EMPTY = 9, P_FULL = 11, P_EMPTY = 13, O_FULL = 15,
               S_FULL = 16, S_EMPTY = 16 + kSBufs };
 
+template <int SUB>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const int32_t* __restrict__ selected,
@@ -74,10 +75,10 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qtile = blockIdx.x;
   const long long bh = blockIdx.y;
-  const int Qb = (int)(Lq / kTile);
-  const int qb = qtile;
+  const int Qb = (int)(Lq / (kTile * SUB));
+  const int qb = qtile / SUB;
   const int32_t* sel = selected + (bh * Qb + qb) * (long long)topk;
-  const int n_iter = topk;
+  const int n_iter = topk * SUB;
   const float c = scale * kLog2e;
 
   int32_t* tile_row = reinterpret_cast<int32_t*>(sm + FwdSmem::tile_row);
@@ -111,11 +112,11 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   }
   // every thread looks up some of the routed tiles (two dependent global loads, all in flight at once) ...
   for (int it = tid; it < n_iter; it += kFwdThreads) {
-    const int kvb = sel[it];
+    const int kvb = sel[it / SUB];
     // an id outside the table is an empty tile, as route inversion treats it
-    const int left = (unsigned)kvb < (unsigned)(Lkv / kTile) ? kv_sizes[kvb] : 0;
+    const int left = (unsigned)kvb < (unsigned)(Lkv / (kTile * SUB)) ? kv_sizes[kvb] - (it % SUB) * kTile : 0;
     tile_valid[it] = (uint8_t)(left < 0 ? 0 : (left > kTile ? kTile : left));
-    tile_row[it] = left > 0 ? (int)kv_tensor_row(bh, gridDim.y, (long long)kvb * kTile, kv_shard) : 0;
+    tile_row[it] = left > 0 ? (int)kv_tensor_row(bh, gridDim.y, (long long)kvb * (kTile * SUB) + (it % SUB) * kTile, kv_shard) : 0;
   }
   __syncthreads();
   if (warp == 2) {   // ... then one warp squeezes out the empty ones in place, keeping the routing order
@@ -385,7 +386,7 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
   if (BH > 65535) return fail(VSA_ERR_UNSUPPORTED, "sparse forward: batch*heads %lld exceeds 65535", (long long)BH);
   CUtensorMap mq, mk, mv;
   int rc;
-  if (be % kWRows == 0)
+  if (sparse_wide_rows(kPassForward, BH, Lq, D, be, topk))
     return D == 64 ? launch_fwd_wide<64>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map)
                    : launch_fwd_wide<128>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse forward (q)"))) return rc;
@@ -414,7 +415,7 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
                                               comb_map);
       return check_launch("sparse_fwd_umma_persistent_kernel");
     };
-    return launch(sparse_fwd_umma_persistent_kernel);
+    VSA_BY_BLOCK_VOLUME(be, launch, sparse_fwd_umma_persistent_kernel);
   }
   const int smem = FwdSmem::total + 1024;
   dim3 grid((unsigned)(Lq / kTile), (unsigned)BH);
@@ -424,7 +425,7 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
                                           (const elem_t*)gate, (elem_t*)out_comb, Lq, Lkv, kv_shard, topk, scale, comb_map);
     return check_launch("sparse_fwd_umma_kernel");
   };
-  return launch(sparse_fwd_umma_kernel);
+  VSA_BY_BLOCK_VOLUME(be, launch, sparse_fwd_umma_kernel);
 }
 
 int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v, const void* out_s,
@@ -436,7 +437,7 @@ int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v
   { const int rc0 = check_kv_shard(Lkv, be, &kv_shard, "sparse dQ"); if (rc0) return rc0; }
   CUtensorMap mq, mdo, mk, mv;
   int rc;
-  if (be % kWRows == 0)
+  if (sparse_wide_rows(kPassDq, BH, Lq, D, be, topk))
     return D == 64 ? launch_dq_wide<64>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map)
                    : launch_dq_wide<128>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse dQ (q)"))) return rc;
@@ -452,7 +453,7 @@ int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v
                                           out_map);
     return check_launch("sparse_dq_umma_kernel");
   };
-  return launch(sparse_dq_umma_kernel);
+  VSA_BY_BLOCK_VOLUME(be, launch, sparse_dq_umma_kernel);
 }
 
 int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void* v, const float* lse2,
@@ -467,7 +468,7 @@ int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void*
     return fail(VSA_ERR_UNSUPPORTED, "sparse dK/dV: packed edges hold at most %d routes per query block", 1 << kEdgeSlotBits);
   CUtensorMap mq, mdo, mk, mv;
   int rc;
-  if (be % kWRows == 0 && !ds_ws)
+  if (!ds_ws && sparse_wide_rows(kPassDkdv, BH, Lkv, D, be, topk))
     return D == 64 ? launch_dkdv_wide<64>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map)
                    : launch_dkdv_wide<128>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse dK/dV (q)"))) return rc;
@@ -485,10 +486,9 @@ int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void*
                                           kv_shard, topk, scale, out_map);
     return check_launch("sparse_dkdv_umma_kernel");
   };
-  if (!ds_ws) return launch(sparse_dkdv_umma_kernel<1, false>);
-  if (be == 64) return launch(sparse_dkdv_umma_kernel<1, true>);
-  if (be == 128) return launch(sparse_dkdv_umma_kernel<2, true>);
-  return launch(sparse_dkdv_umma_kernel<4, true>);
+  if (be == 64) return ds_ws ? launch(sparse_dkdv_umma_kernel<1, true>) : launch(sparse_dkdv_umma_kernel<1, false>);
+  if (be == 128) return ds_ws ? launch(sparse_dkdv_umma_kernel<2, true>) : launch(sparse_dkdv_umma_kernel<2, false>);
+  return ds_ws ? launch(sparse_dkdv_umma_kernel<4, true>) : launch(sparse_dkdv_umma_kernel<4, false>);
 }
 
 int sparse_dq_from_ds_umma(const void* k, const int32_t* selected, const int32_t* kv_sizes, const void* ds_ws, void* dq,

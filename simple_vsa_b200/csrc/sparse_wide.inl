@@ -950,8 +950,7 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 }
 
 // ---- host launchers of the 128-row kernels -----------------------------------------------------------------------
-// Taken whenever the block volume is a multiple of 128: 128 rows that share a route are what fills the M dimension, and at
-// no size measured (16 to 180 tiles per row, 64 to 720 row tiles) were the 64-token kernels faster on such blocks.
+// Taken for block volumes that are multiples of 128, where sparse_wide_rows (and, at head dim 64, sparse_wide64_pays) says so.
 template <int HD>
 int launch_fwd_wide(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes, void* out,
                     float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale, cudaStream_t st,

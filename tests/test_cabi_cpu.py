@@ -176,6 +176,12 @@ def test_kernels_of_a_pass():
         assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([1, 3] if p < 2 else [3, 3])
         assert [kernels(p, 8, 65536, 64, 128, tk) for tk in (1, 4, 5)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
         assert [kernels(p, 8, 65536, 64, 256, tk) for tk in (1, 2, 3)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
+        # head dim 128: 64-token tiles where all of them fit on the SMs at once ...
+        assert [kernels(p, BH, 64 * 128, 128, 128, 32) for BH in (1, 2)] == [2, 3]
+        assert [kernels(p, 1, 256 * nb, 128, 256, 16) for nb in (37, 38)] == [2, 3]
+    # ... and for short routes of dQ where 128-row tiles take more than half as many waves
+    assert [kernels(1, 3, 8192, 128, 128, tk) for tk in (1, 12, 32)] == [2, 2, 3]
+    assert [kernels(1, 80, 92160, 128, be, 1) for be in (128, 256)] == [3, 3]
     assert kernels(3, 8, 65536, 128, 64, 16) == L.ERR_BAD_ARGUMENT
     assert kernels(0, 8, 65, 128, 64, 1) == L.ERR_BAD_ARGUMENT
 

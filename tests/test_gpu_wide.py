@@ -1,6 +1,6 @@
-"""The 128-row tcgen05 kernels (blocks of 128 and 256 tokens, head dims 64 and 128) at the edges of their tiles, against
-the CPU oracle: live sizes around 0, 1, 64, 128 and the full block, a single tile, odd tile counts, more tiles than any ring
-is deep, query and key lengths that differ."""
+"""The tensor-core kernels on blocks of 128 and 256 tokens (128-row tcgen05 kernels, and those that take their place on small
+grids and short routes; head dims 64 and 128) at the edges of their tiles, against the CPU oracle: live sizes around 0, 1, 64,
+128 and the full block, a single tile, odd tile counts, more tiles than any ring is deep, query and key lengths that differ."""
 
 import pytest
 import torch
@@ -14,10 +14,18 @@ DEV = "cuda:0"
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("be,qb,kb,tk", [(128, 1, 1, 1), (128, 2, 5, 4), (128, 3, 7, 5), (256, 2, 5, 3), (256, 1, 9, 9)])
-def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype):
+@pytest.mark.parametrize("large", [False, True])
+def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype, large):
     from simple_vsa_b200 import _lib, b200_sparse_attention
     g = torch.Generator().manual_seed(be + 7 * kb + D)
-    B, H = 1, 2
+    # a few row tiles take the 64-token kernels at head dim 128; one full wave of 128-row tiles takes the others
+    B, H = 1, 296 // (qb * be // 64) if large else 2
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    for p, n in enumerate((qb, qb, kb)):
+        kernels = 3 if large or D == 64 else 2
+        if D == 64 and p < 2 and tk * be // 64 <= (4 if large else 8):
+            kernels = 1
+        assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == kernels
     q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
     k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
     sizes = torch.tensor(([be, 1, 0, 64, 127, 128, be - 1, 65, 129 % be] * 2)[:kb])
