@@ -268,6 +268,7 @@ constexpr int kDtypeCode = VSA_F16;
 // maximum before P overflows (and the tile goes to the exact kernel) and keeps scores down to 20 binades below it --
 // the middle of fp16's 2^-24 .. 2^16 instead of its top.  The row sum uses the same shift, so O/l and the saved
 // statistic are unchanged.  bf16 has 2^127 above the first pair's maximum and needs no bias.
+// (The 128-row forward at head dim 64 does without it; see there.)
 constexpr float kShiftBias = 4.f;
 #include "sparse_umma_typed.inl"
 }  // namespace tc_f16

@@ -255,7 +255,11 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
           for (int i = 0; i < 32; ++i) m = fmaxf(m, 32 * j + i < valid ? __uint_as_float(sv[i]) * c : -INFINITY);
         }
-        m += kShiftBias;
+        // Head dim 64 keeps fp16's precision at the bottom: the online softmax of the mma.sync kernels, which it shares its
+        // shapes with, has its largest P at 1, and P below 2^-14 lose bits.  With four binades less under the maximum the
+        // error against float64 rose 6 % where one key outweighs 8000 others by 10 nats (2.62e-4 -> 2.77e-4), and doubled at
+        // 12.  Scores 16 binades above the first tile's maximum go to the exact kernel (20 with the bias).
+        if (HD != 64) m += kShiftBias;
         m_row[row] = m;
         neg_m = -m;
         __syncwarp();

@@ -99,3 +99,28 @@ def test_dq_of_query_blocks_without_a_live_key_is_the_pooled_gradient_alone(be, 
         assert torch.isnan(out[:, dead].float()).all()
         assert torch.equal(dq[:, ~dead], dq_ref[:, ~dead]) and torch.equal(out[:, ~dead], out_ref[:, ~dead])
     assert _lib.device_status() == 0
+
+
+def test_small_fp16_probabilities_at_head_dim_64_are_as_precise_as_on_the_warp_level_kernels(monkeypatch):
+    """One key 12 nats above 5000 others: their probabilities sit near the bottom of fp16, and the output is made of them."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator().manual_seed(12)
+    be, qb, kb, D = 128, 2, 40, 64
+    q, k, v = (torch.randn(1, 1, n * be, D, generator=g) for n in (qb, kb, kb))
+    k *= 0.5
+    v += 1.0
+    q[..., 0], k[..., 0] = 4.0, 0.0
+    k[0, 0, 5], v[0, 0, 5] = 0.0, 0.0
+    k[0, 0, 5, 0] = 12.0 * D ** 0.5 / 4.0
+    q, k, v = (x.half() for x in (q, k, v))
+    assert _lib.lib.vsa_sparse_pass_kernels(0, 1, qb * be, D, be, kb, _lib.VSA_F16) == 3
+    want = (q[0, 0].double() @ k[0, 0].double().T * D ** -0.5).softmax(-1) @ v[0, 0].double()
+    selected = torch.arange(kb, dtype=torch.int32).expand(1, 1, qb, kb).contiguous().to(DEV)
+    sizes = torch.full((kb,), be, dtype=torch.int32, device=DEV)
+    error = {}
+    for mode in ("auto", "mma"):
+        monkeypatch.setenv("VSA_B200_KERNELS", mode)
+        out, lse = ops.sparse_forward(q.to(DEV), k.to(DEV), v.to(DEV), selected, sizes, be, D ** -0.5, True)
+        error[mode] = (out[0, 0].double().cpu() - want).norm() / want.norm()
+    # the same probabilities rounded at the same binades; what differs is the order of the fp32 sums around them
+    assert error["auto"] <= 1.05 * error["mma"]
