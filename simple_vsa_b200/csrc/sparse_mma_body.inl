@@ -187,7 +187,7 @@ sparse_fwd_mma_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
       }
     }
     // Two scores per instruction; the mask costs a select per score and is left out of full tiles: [1, 4, 92160, 64], topk 180,
-    // 4.01 -> 3.62 ms (dQ 4.95 -> 4.78, dK/dV 6.74 -> 6.51 with the same).
+    // 4.01 -> 3.62 ms (dQ 4.95 -> 4.78 with the same; dK/dV 6.74 -> 6.31 with packed arithmetic alone).
     const float2 c2 = make_float2(c, c);
     float tmax[2] = {-INFINITY, -INFINITY};
     auto scale_and_max = [&](auto masked) {
@@ -537,26 +537,24 @@ sparse_dkdv_mma_kernel(const T* __restrict__ dout, const T* __restrict__ q, cons
         }
       }
       // transposed tile: rows are key tokens, columns are query rows of this half
-      auto score_gradient = [&](auto masked) {
+      // One body with the mask in it: a second one for full tiles cost 8 % where the GPU is not full ([1, 2, 4096, 64], topk 8:
+      // 27.8 us with scalar arithmetic, 30.2 with two packed bodies, 27.0 with this one) and 3 % where it is.
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-          const int qi = h * 32 + nt * 8 + 2 * t;
-          const float2 l2 = *reinterpret_cast<const float2*>(st_lse + qi), d2 = *reinterpret_cast<const float2*>(st_dl + qi);
+      for (int nt = 0; nt < 4; ++nt) {
+        const int qi = h * 32 + nt * 8 + 2 * t;
+        const float2 l2 = *reinterpret_cast<const float2*>(st_lse + qi), d2 = *reinterpret_cast<const float2*>(st_dl + qi);
 #pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const float2 x = fma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), make_float2(c, c), make_float2(-l2.x, -l2.y));
-            float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-            float2 g = mul2(p, add2(make_float2(dp[nt][2 * r], dp[nt][2 * r + 1]), make_float2(-d2.x, -d2.y)));
-            if (decltype(masked)::value && !row_ok[r]) p = g = make_float2(0.f, 0.f);
-            s[nt][2 * r] = p.x;
-            s[nt][2 * r + 1] = p.y;
-            dp[nt][2 * r] = g.x;
-            dp[nt][2 * r + 1] = g.y;
-          }
+        for (int r = 0; r < 2; ++r) {
+          const float2 x = fma2(make_float2(s[nt][2 * r], s[nt][2 * r + 1]), make_float2(c, c), make_float2(-l2.x, -l2.y));
+          float2 p = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          float2 g = mul2(p, add2(make_float2(dp[nt][2 * r], dp[nt][2 * r + 1]), make_float2(-d2.x, -d2.y)));
+          if (!row_ok[r]) p = g = make_float2(0.f, 0.f);
+          s[nt][2 * r] = p.x;
+          s[nt][2 * r + 1] = p.y;
+          dp[nt][2 * r] = g.x;
+          dp[nt][2 * r + 1] = g.y;
         }
-      };
-      if (valid == kTile) score_gradient(std::false_type{});
-      else score_gradient(std::true_type{});
+      }
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
         uint32_t pa[4], da[4];
