@@ -375,11 +375,12 @@ def test_fine_attention_midsize_matches_oracle(be, nb, tk, ragged, monkeypatch):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("be,nb,tk", [(64, 20, 6), (128, 10, 4), (256, 6, 3)])
+@pytest.mark.parametrize("be,nb,tk", [(64, 20, 6), (128, 10, 4), (128, 10, 6), (256, 6, 3)])
 def test_head_dim_64_runs_on_the_warp_level_tensor_kernels(be, nb, tk, dtype, monkeypatch):
-    """Head dim 64 (bf16 / fp16, blocks of 64, 128, 256): the mma.sync kernels instantiated for 64-wide tiles, against
-    the oracle and against the CUDA-core kernels, ragged blocks included; the whole operator (pooled branch on the
-    CUDA-core GEMMs at this head dim) with a gate as well."""
+    """Head dim 64 (bf16 / fp16, blocks of 64, 128, 256): the mma.sync kernels instantiated for 64-wide tiles ("mma"), the
+    kernels that the library chooses (the same for blocks of 64; for larger ones the 128-row tcgen05 kernels from 9 tiles a
+    route up, and always for dK/dV) and the CUDA-core kernels against the oracle, ragged blocks included; the whole operator
+    with a gate as well."""
     from simple_vsa_b200 import _lib
     V = _V()
     torch.manual_seed(81)
@@ -389,6 +390,8 @@ def test_head_dim_64_runs_on_the_warp_level_tensor_kernels(be, nb, tk, dtype, mo
     assert _lib.lib.vsa_sparse_kernel_family(D, be, tk, dt_code) == 1
     assert _lib.lib.vsa_sparse_kernel_family(128, be, tk, dt_code) == 2
     assert _lib.lib.vsa_sparse_kernel_family(D, be, tk, _lib.VSA_F32) == 0
+    kernels = lambda p: _lib.lib.vsa_sparse_pass_kernels(p, B * H, L, D, be, tk, dt_code)
+    assert [kernels(p) for p in range(3)] == ([1, 1, 1] if be == 64 else [1, 1, 3] if tk * be <= 8 * 64 else [3, 3, 3])
     q, k, v, dout = (torch.randn(B, H, L, D).to(dtype) for _ in range(4))
     sizes = torch.full((nb,), be)
     sizes[1], sizes[nb // 2], sizes[-1] = 1, be // 2 + 3, be - 1
@@ -396,7 +399,7 @@ def test_head_dim_64_runs_on_the_warp_level_tensor_kernels(be, nb, tk, dtype, mo
     ol = [t.clone().requires_grad_() for t in (q, k, v)]
     want = O.sparse_attention(*ol, selected, sizes, be, q_blocks_per_chunk=8)
     want.backward(dout.float())
-    for mode in ("auto", "scalar"):
+    for mode in ("auto", "mma", "scalar"):
         monkeypatch.setenv("VSA_B200_KERNELS", mode)
         leaves = [t.to(DEV).requires_grad_() for t in (q, k, v)]
         out = V.b200_sparse_attention(*leaves, selected.to(DEV), sizes, block_size=(1, 1, be))
@@ -404,7 +407,7 @@ def test_head_dim_64_runs_on_the_warp_level_tensor_kernels(be, nb, tk, dtype, mo
         _assert_close(out, want, atol=2e-2, rtol=2e-2)
         for leaf, oleaf in zip(leaves, ol):
             _assert_close(leaf.grad, oleaf.grad, atol=3e-2, rtol=3e-2)
-        if mode == "auto":
+        if mode != "scalar":
             assert leaves[1].grad[0, :, be + 1:2 * be].abs().max() == 0      # padded key rows: exactly zero
     monkeypatch.delenv("VSA_B200_KERNELS")
     gate = torch.sigmoid(torch.randn(B, H, L, D)).to(dtype)
@@ -676,7 +679,7 @@ def test_compression_gate_trains_through_the_operator():
 
 
 def test_a_large_problem_off_the_tensor_path_warns_once():
-    """fp32 (the validation mode) is served by the CUDA-core kernels only; a problem of 1e11 useful FLOPs or more says so
+    """fp32 (the validation mode) is served by CUDA-core kernels only; a problem of 1e11 useful FLOPs or more says so
     once per process; tensor-core shapes (head dim 128 on tcgen05, head dim 64 on the warp-level kernels) and small
     validation-size problems never do."""
     import warnings
@@ -936,6 +939,8 @@ def test_the_two_schedules_of_the_forward_give_the_same_bits(be, nb, tk, monkeyp
     selected = torch.stack([torch.randperm(nb)[:tk] for _ in range(B * H * nb)]).view(B, H, nb, tk).to(torch.int32).to(DEV)
     selected[0, 2, 4, :] = 3                       # a query block whose whole route is the empty block
     scale = 1.0 / math.sqrt(D)
+    from simple_vsa_b200 import _lib
+    assert _lib.lib.vsa_sparse_pass_kernels(0, B * H, L, D, be, tk, _lib.VSA_BF16) == 2      # only the 64-token kernels have two
     results = {}
     for mode in ("classic", "persistent"):
         monkeypatch.setenv("VSA_B200_FWD", mode)
@@ -953,9 +958,9 @@ def test_the_two_schedules_of_the_forward_give_the_same_bits(be, nb, tk, monkeyp
 @pytest.mark.parametrize("seed", list(range(24)))
 def test_random_shapes_tensor_path_matches_cuda_core_path(seed, monkeypatch):
     """Seeded random problems (block 64, 128 or 256, 1..40 blocks, any topk, query length != key length, random ragged
-    and empty blocks, with and without a gate): the whole operator on the tcgen05 kernels against the same call on
+    and empty blocks, with and without a gate): the whole operator on the kernels that the library chooses against the same call on
     the CUDA-core kernels, forward and every gradient; seeds 10-13 and 21-23 run in fp16, the others in bf16; seeds 14-17 use blocks of 128 tokens; seeds from 18 up
-    have head dim 64 (the warp-level tensor-core kernels).  The routes are fixed by the first run's Top-K (pooled scores
+    have head dim 64 (the warp-level kernels; with blocks of 256 the 128-row tcgen05 kernels too).  The routes are fixed by the first run's Top-K (pooled scores
     are computed by the same kernels in both runs)."""
     V = _V()
     dt = torch.float16 if 10 <= seed < 14 or seed >= 21 else torch.bfloat16

@@ -189,6 +189,8 @@ def test_fp16_two_schedules_of_the_forward_give_the_same_bits(be, nb, tk, monkey
     sizes = torch.full((nb,), be, dtype=torch.int32, device=DEV)
     sizes[2], sizes[-1] = 9, be - 1
     selected = _zipf_routes(B, H, nb, nb, tk, 23).to(DEV)
+    from simple_vsa_b200 import _lib
+    assert _lib.lib.vsa_sparse_pass_kernels(0, B * H, L, D, be, tk, _lib.VSA_F16) == 2       # only the 64-token kernels have two
     res = {}
     for sched in ("classic", "persistent"):
         monkeypatch.setenv("VSA_B200_FWD", sched)

@@ -162,7 +162,7 @@ def test_explicit_zipf_routes_92k_tokens_block64_topk180():
 @pytest.mark.parametrize("be,tk,dtype", [(64, 180, torch.float16), (128, 90, torch.bfloat16)])
 def test_explicit_zipf_routes_92k_tokens_fp16_and_128_token_blocks(be, tk, dtype, monkeypatch):
     """The same size through the other instantiations of the tensor path: fp16 inputs (90 pairs per query CTA with P
-    kept inside fp16's range by the redo rule), and blocks of 128 tokens (two 64-token tiles per block, 720 blocks)."""
+    kept inside fp16's range by the redo rule), and blocks of 128 tokens (the 128-row kernels, 720 blocks)."""
     import sys
     monkeypatch.setattr(sys.modules[__name__], "_DT", dtype)
     B, H, L, D = 1, 2, 92160, 128

@@ -124,3 +124,39 @@ def test_small_fp16_probabilities_at_head_dim_64_are_as_precise_as_on_the_warp_l
         error[mode] = (out[0, 0].double().cpu() - want).norm() / want.norm()
     # the same probabilities rounded at the same binades; what differs is the order of the fp32 sums around them
     assert error["auto"] <= 1.05 * error["mma"]
+
+
+@pytest.mark.parametrize("dtype,k_factor,q_factor", [(torch.bfloat16, 8.0, 40.0), (torch.float16, 1.5, 20.0)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("be,qb", [(128, 2), (256, 1)])
+def test_one_half_of_a_tile_outside_the_shift_range_is_recomputed_exactly(be, qb, D, dtype, k_factor, q_factor):
+    """The softmax shift of a row comes from its first live key tile, here one of 5 keys.  A later block scores hundreds of binades
+    above it for the rows 64 to 127 of a tile (out of the element type's range: the exact kernel's work) and a few for the rows
+    before them.  Output, statistic and combined output match the oracle in both halves."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator().manual_seed(be + D)
+    H, kb, tk, scale = 296 // (qb * be // 64), 8, 6, D ** -0.5
+    q, gate = (torch.randn(1, H, qb * be, D, generator=g) for _ in range(2))
+    k, v = (torch.randn(1, H, kb * be, D, generator=g) for _ in range(2))
+    out_c = torch.randn(1, H, qb, D, generator=g).to(dtype)
+    q.view(1, H, -1, 128, D)[:, :, :, 64:] *= q_factor
+    k.view(1, H, kb, be, D)[:, :, 3] *= k_factor
+    q, k, v, gate = (x.to(dtype) for x in (q, k, v, gate))
+    sizes = torch.tensor([5, be, be, be - 3, be, 64, be, 1])
+    selected = torch.rand(1, H, qb, kb, generator=g)
+    selected[..., 0], selected[..., 3] = 3.0, 2.0           # the block of 5 keys comes first, the high-scoring one second
+    selected = selected.topk(tk, dim=-1).indices.to(torch.int32)
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    assert _lib.lib.vsa_sparse_pass_kernels(0, H, qb * be, D, be, tk, code) == 3
+    # the scores say which rows leave the range: 2^(score - shift) in fp32, fp16's 2^16 and bf16's 2^127 above it
+    s = torch.einsum("bhtd,bhsd->bhts", q.float(), k.float().view(1, H, kb, be, D)[:, :, [0, 3]].flatten(2, 3)) * scale * 1.4427
+    above = (s[..., be:2 * be - 3].amax(-1) - s[..., :5].amax(-1)).view(1, H, -1, 128)
+    limit = 127 if dtype == torch.bfloat16 else 16
+    assert (above[..., 64:].amax(-1) > limit + 10).all() and (above[..., :64] < limit - 2).all()
+    want, want_lse = O.sparse_attention(q, k, v, selected, sizes, be, return_lse2=True)
+    want_total = O.combine(want.to(dtype), out_c, gate, be, dtype)
+    out, lse, total = ops.sparse_forward(q.to(DEV), k.to(DEV), v.to(DEV), selected.to(DEV), sizes.to(DEV, torch.int32), be, scale,
+                                         True, combine_with=(out_c.to(DEV), gate.to(DEV)))
+    assert _lib.device_status() == 0
+    for got, ref, rtol in ((out, want, 2e-2), (total, want_total, 2e-2), (lse, want_lse, 1e-3)):
+        torch.testing.assert_close(got.float().cpu(), ref.float(), atol=2e-2 if rtol == 2e-2 else 5e-2, rtol=rtol)
