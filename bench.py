@@ -65,7 +65,7 @@ WORKLOADS = {
     "c4_92k_routes_local": dict(B=1, H=40, L=92160, D=128, block_size=(4, 4, 4), topk=180, gate=False, routes="local"),
     "c4_92k_routes_hotset": dict(B=1, H=40, L=92160, D=128, block_size=(4, 4, 4), topk=180, gate=False, routes="hotset"),
     # the reference's own CPU-runnable case: fp32, 16 full blocks of 64, head dim 64, topk 4 (fp32 runs on the CUDA-core kernels)
-    # the profiling case with blocks of 128 tokens (two 64-token tiles per block), same useful FLOPs as be 64 / topk 180
+    # the profiling case with blocks of 128 tokens (128-row kernels), same useful FLOPs as be 64 / topk 180
     "mid_92k_h8_be128_tk90_gate": dict(B=1, H=8, L=92160, D=128, block_size=(4, 4, 8), topk=90, gate=True),
     # c2 at head dim 64: the warp-level (mma.sync) tensor-core kernels; VSA_B200_KERNELS=scalar times the CUDA-core ones
     "c2_d64_16k_be64_tk32_gate": dict(B=1, H=12, L=16384, D=64, block_size=(4, 4, 4), topk=32, gate=True),

@@ -19,10 +19,9 @@
  *   counts, offsets                 [BH, Kb]         int32 (CSR of key block -> query blocks)
  *   inverse                         [BH, Qb*topk]    int32 query-block ids grouped by key block
  *
- * dtype: VSA_BF16 or VSA_F16 (tcgen05 kernels for D = 128 and be = 64, 128 or 256, warp-level
- * tensor-core kernels for D = 64 at those block volumes, scalar kernels otherwise; the reference
- * accepts both) or VSA_F32 (scalar kernels, the fp32
- * validation mode).
+ * dtype: VSA_BF16 or VSA_F16 (tensor-core kernels for D = 64 and 128 and be = 64, 128 or 256, see
+ * vsa_sparse_pass_kernels; CUDA-core kernels otherwise; the reference accepts both) or VSA_F32
+ * (CUDA-core kernels, the fp32 validation mode).
  *
  * Each comment names the function of the reference project (path inside that
  * project : lines) whose work the entry point replaces.

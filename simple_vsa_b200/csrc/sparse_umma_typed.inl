@@ -532,8 +532,9 @@ int launch_gemm(const void* A, int64_t a_rows, int64_t a_cols, int64_t a_pitch, 
   return check_launch(what);
 }
 
-// The scores keep the operator's dense layout.  With a row pitch that is not 16 bytes their product stays on the CUDA cores:
-// it is one of six, and a sum taken in another order can turn a rounding, and with it a tie at the edge of the Top-K.
+// The scores keep the operator's dense layout.  Unless both block counts are multiples of 8 their product runs on the CUDA cores:
+// the wide stores want rows of 16 bytes (Kb % 8 == 0), and a sum taken in another order can turn a rounding, and with it a tie
+// at the edge of the Top-K, so an odd Qb alone does not move a shape either.  It is one product of six.
 int coarse_fwd_umma(const void* qc, const void* kc, const void* vc, void* scores, void* probs, void* out_c, int64_t BH,
                     int Qb, int Kb, int pitch, int D, float scale, cudaStream_t st) {
   int rc = Qb % 8 == 0 && Kb % 8 == 0

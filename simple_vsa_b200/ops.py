@@ -80,7 +80,7 @@ _warned_slow_path = False
 
 def _warn_if_far_off_the_tensor_path(dt: int, B: int, H: int, Lq: int, D: int, be: int, topk: int) -> None:
     """One warning per process when a large problem lands on the CUDA-core kernels.  They exist as the validation
-    mode (fp32) and for shapes the reference accepts but its benchmarks never use; per FLOP they are two to three
+    mode (fp32) and for shapes the reference accepts but its benchmarks never use; per FLOP they are one to three
     orders of magnitude slower than the tcgen05 kernels, which a caller should learn from more than a slow step."""
     global _warned_slow_path
     if _warned_slow_path or 14.0 * B * H * Lq * topk * be * D < 1e11:
@@ -89,7 +89,8 @@ def _warn_if_far_off_the_tensor_path(dt: int, B: int, H: int, Lq: int, D: int, b
         return
     _warned_slow_path = True
     warnings.warn("simple_vsa_b200: this shape runs on the CUDA-core validation kernels (the tensor-core paths need "
-                  "bf16 or fp16, head dim 64 or 128, block volume 64, 128 or 256, and VSA_B200_KERNELS unset or =mma); expect a step hundreds of times slower per FLOP", RuntimeWarning, stacklevel=3)
+                  "bf16 or fp16, head dim 64 or 128, block volume 64, 128 or 256, and VSA_B200_KERNELS unset or =mma); expect a step tens of times slower per FLOP "
+                  "in fp32 at those sizes, hundreds of times elsewhere", RuntimeWarning, stacklevel=3)
 
 
 def _dense(x: Tensor) -> Tensor:
