@@ -880,8 +880,9 @@ def test_forward_with_the_combine_folded_in_equals_the_two_step_form(kernels, wi
                       atol=2e-2, rtol=2e-2)
 
 
-@pytest.mark.parametrize("be,nb,tk,W", [(64, 16, 5, 2), (64, 24, 6, 4), (256, 8, 3, 2), (128, 12, 4, 2)])
-def test_shard_major_kv_layout_equals_the_ordinary_layout(be, nb, tk, W):
+@pytest.mark.parametrize("be,nb,tk,W,H", [(64, 16, 5, 2, 3), (64, 24, 6, 4, 3), (256, 8, 3, 2, 3), (128, 12, 4, 2, 3),
+                                          (256, 8, 3, 2, 18), (128, 12, 4, 2, 24)])       # enough rows for the 128-row kernels
+def test_shard_major_kv_layout_equals_the_ordinary_layout(be, nb, tk, W, H):
     """The kernels of the sequence-parallel mode read K/V (and write dK/dV) in the rank-major layout an all-gather
     leaves, ``[W,B,H,L/W,D]``.  One GPU, no collective: the same operator on the same numbers in both layouts, a
     rank's share of the queries against all keys, ragged blocks, a gate, and a scaled key block so that the exact
@@ -889,9 +890,12 @@ def test_shard_major_kv_layout_equals_the_ordinary_layout(be, nb, tk, W):
     V = _V()
     from simple_vsa_b200 import ops
     torch.manual_seed(99)
-    B, H, D = 1, 3, 128
+    B, D = 1, 128
     L = be * nb
     l = L // W
+    from simple_vsa_b200 import _lib
+    for p, n in enumerate((l, l, L)):
+        assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n, D, be, tk, _lib.VSA_BF16) == (3 if H > 3 else 2)
     q_all, k, v = (torch.randn(B, H, L, D, device=DEV).to(torch.bfloat16) for _ in range(3))
     k[:, :, 5 * 64:6 * 64] *= 30.0
     sizes = torch.full((nb,), be)

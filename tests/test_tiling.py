@@ -145,10 +145,11 @@ def _two_step(V, meta, q, k, v, gate, topk, tile_size):
 @pytest.mark.parametrize("grid,tile_size,dtype", [((6, 10, 9), (4, 4, 4), torch.bfloat16),
                                                   ((8, 8, 8), (4, 4, 4), torch.float16),
                                                   ((5, 16, 12), (4, 8, 8), torch.bfloat16),
-                                                  ((4, 9, 16), (2, 8, 8), torch.bfloat16)])
+                                                  ((4, 9, 16), (2, 8, 8), torch.bfloat16),
+                                                  ((8, 9, 16), (2, 8, 8), torch.float16)])
 @pytest.mark.parametrize("with_gate", [False, True])
 def test_raster_order_operator_equals_the_two_step_form(grid, tile_size, dtype, with_gate):
-    """Clipped tiles on every axis, full tiles, blocks of 64 / 128 / 256 tokens: out, dq and dgate bit for bit (same
+    """Clipped tiles on every axis, full tiles, blocks of 64 / 128 / 256 tokens (128 on 64-token and on 128-row tiles): out, dq and dgate bit for bit (same
     kernels, same arithmetic, other store addresses); dk/dv up to the order of the fp32 sums over CSR rows."""
     import simple_vsa_b200 as V
     dev = "cuda:0"
