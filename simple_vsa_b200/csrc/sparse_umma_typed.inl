@@ -395,8 +395,9 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
   // Two schedules of the same arithmetic.  One CTA per query tile is faster when a tile walks many pairs (the
   // headline shape: 90); with short routes the per-CTA set-up and drain are a large share of a CTA's life and the
   // persistent form (one CTA per SM, next tile's list, loads and first S^T MMAs under the current tile's epilogue)
-  // wins: measured -7 % at 16 pairs per tile, -9 % at 8, +1 % at 40, +4 % at 90.  VSA_B200_FWD=classic|persistent
-  // overrides the choice.
+  // wins: measured -10 % at 4 pairs per tile, -11 % at 8, -10 % at 16, -7 % at 24, -4 % at 39 and within the spread of 2 % at
+  // 90.  The line lies where the two crossed before the softmax warps' arithmetic was packed (+1 % at 40 pairs, +4 % at 90).
+  // VSA_B200_FWD=classic|persistent overrides the choice.
   const char* fwd_env = std::getenv("VSA_B200_FWD");
   bool persistent = topk * (be / kTile) <= 48;
   if (fwd_env && std::strcmp(fwd_env, "persistent") == 0) persistent = true;
