@@ -43,6 +43,7 @@ template <> struct Elem<__nv_bfloat16> {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+  __device__ __forceinline__ static float2 unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 };
 
 template <> struct Elem<__half> {
@@ -55,6 +56,7 @@ template <> struct Elem<__half> {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+  __device__ __forceinline__ static float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<__half2*>(&w)); }
 };
 
 // ---- warp helpers -----------------------------------------------------------------------

@@ -95,9 +95,10 @@ int make_map_of(CUtensorMap* map, CUtensorMapDataType elem, const void* ptr, int
 __device__ __forceinline__ void report_timeout(int code) { atomicCAS(&g_device_status, 0, code); }
 // all waits of this file poll the status word so that a failure anywhere drains the grid quickly
 #define VSA_WAIT(bar_, parity_) mbar_wait((bar_), (parity_), &g_device_status)
-#define VSA_WARP_WAIT(bar_, parity_) warp_wait((bar_), (parity_), &g_device_status, lane)
-#define VSA_WARP_WAIT2(a_, pa_, b_, pb_) warp_wait2((a_), (pa_), (b_), (pb_), &g_device_status, lane)
-#define VSA_WARP_WAIT_TEST(a_, pa_, b_, pb_, done_) warp_wait_and_test((a_), (pa_), (b_), (pb_), &g_device_status, lane, (done_))
+#define VSA_WARP_WAIT(bar_, parity_) warp_wait((bar_), (parity_), &g_device_status)
+#define VSA_WARP_WAIT2(a_, pa_, b_, pb_) (VSA_WARP_WAIT(a_, pa_) && VSA_WARP_WAIT(b_, pb_))
+#define VSA_WARP_WAIT3(a_, pa_, b_, pb_, c_, pc_) (VSA_WARP_WAIT(a_, pa_) && VSA_WARP_WAIT(b_, pb_) && VSA_WARP_WAIT(c_, pc_))
+#define VSA_WARP_WAIT_TEST(a_, pa_, b_, pb_, done_) warp_wait_and_test((a_), (pa_), (b_), (pb_), &g_device_status, (done_))
 
 // One 64x128 tile = two boxes (head-dim halves); `dst` is the row offset inside a stacked pair.
 __device__ __forceinline__ void load_tile(uint32_t pair_base, int half_rows_off, const CUtensorMap* map, int row,
@@ -228,8 +229,9 @@ int make_map3d_of(CUtensorMap* map, CUtensorMapDataType elem, const void* ptr, i
 }
 
 template <typename Kern>
-int reserve_smem(Kern kern, int bytes, const char* what) {
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+int reserve_smem(Kern kern, int bytes, const char* what, bool two_per_sm = false) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && two_per_sm) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return fail(VSA_ERR_LAUNCH, "%s: shared memory: %s", what, cudaGetErrorString(e));
   return VSA_OK;
 }

@@ -374,6 +374,7 @@ sparse_fwd_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #include "sparse_umma_fwd_persistent.inl"
 #include "sparse_umma_bwd.inl"
 #include "sparse_wide.inl"
+#include "sparse_split.inl"
 #include "coarse_umma.inl"
 
 // ---- host launchers of this element type ----------------------------------------------------------------------
@@ -389,6 +390,8 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
   if (sparse_wide_rows(kPassForward, BH, Lq, D, be, topk))
     return D == 64 ? launch_fwd_wide<64>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map)
                    : launch_fwd_wide<128>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map);
+  return D == 64 ? launch_fwd_split<64>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map)
+                 : launch_fwd_split<128>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse forward (q)"))) return rc;
   if ((rc = make_map(&mk, k, BH * Lkv, "sparse forward (k)"))) return rc;
   if ((rc = make_map(&mv, v, BH * Lkv, "sparse forward (v)"))) return rc;
@@ -441,6 +444,8 @@ int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v
   if (sparse_wide_rows(kPassDq, BH, Lq, D, be, topk))
     return D == 64 ? launch_dq_wide<64>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map)
                    : launch_dq_wide<128>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map);
+  return D == 64 ? launch_dq_split<64>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map)
+                 : launch_dq_split<128>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse dQ (q)"))) return rc;
   if ((rc = make_map(&mdo, dout, BH * Lq, "sparse dQ (dout)"))) return rc;
   if ((rc = make_map(&mk, k, BH * Lkv, "sparse dQ (k)"))) return rc;
@@ -472,6 +477,9 @@ int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void*
   if (!ds_ws && sparse_wide_rows(kPassDkdv, BH, Lkv, D, be, topk))
     return D == 64 ? launch_dkdv_wide<64>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map)
                    : launch_dkdv_wide<128>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map);
+  if (!ds_ws)
+    return D == 64 ? launch_dkdv_split<64>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map)
+                   : launch_dkdv_split<128>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map);
   if ((rc = make_map(&mq, q, BH * Lq, "sparse dK/dV (q)"))) return rc;
   if ((rc = make_map(&mdo, dout, BH * Lq, "sparse dK/dV (dout)"))) return rc;
   if ((rc = make_map(&mk, k, BH * Lkv, "sparse dK/dV (k)"))) return rc;

@@ -60,6 +60,18 @@ __device__ __forceinline__ uint4 wide_pack8(const uint32_t* r) {
   return make_uint4(Elem<elem_t>::pack(__uint_as_float(r[0]), __uint_as_float(r[1])), Elem<elem_t>::pack(__uint_as_float(r[2]), __uint_as_float(r[3])),
                     Elem<elem_t>::pack(__uint_as_float(r[4]), __uint_as_float(r[5])), Elem<elem_t>::pack(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
+// N accumulator columns plus N values that every row receives.
+template <int N>
+__device__ __forceinline__ void wide_add_mean(uint32_t (&acc)[N], const float* mean) {
+#pragma unroll
+  for (int i = 0; i < N / 4; ++i) {
+    const float4 m = reinterpret_cast<const float4*>(mean)[i];
+    acc[4 * i] = __float_as_uint(__uint_as_float(acc[4 * i]) + m.x);
+    acc[4 * i + 1] = __float_as_uint(__uint_as_float(acc[4 * i + 1]) + m.y);
+    acc[4 * i + 2] = __float_as_uint(__uint_as_float(acc[4 * i + 2]) + m.z);
+    acc[4 * i + 3] = __float_as_uint(__uint_as_float(acc[4 * i + 3]) + m.w);
+  }
+}
 // HD/64 boxes of `rows` x 128 bytes, all on one barrier (the caller has announced the bytes).
 template <int HD>
 __device__ __forceinline__ void wide_load(uint32_t dst, const CUtensorMap* map, int row, uint32_t half_bytes, uint32_t bar) {

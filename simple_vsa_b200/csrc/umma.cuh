@@ -44,55 +44,39 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag,
                                           unsigned long long limit_ns = kWaitLimitNs) {
-  // Called by ONE lane per warp (see warp_wait): hundreds of threads polling the same barrier word
-  // measurably slowed the shared-memory pipe.  The clock and the abort flag live in global memory and
-  // are looked at once per 64 unsuccessful tries only.
+  // One thread.  No sleep between the tries: a try_wait suspends the thread by itself, and 20 ns of nanosleep made a hop from one
+  // warp to another cost 720 cycles instead of 207.  The clock and the abort flag live in global memory and are looked at once per
+  // 64 unsuccessful tries only.
   unsigned long long t0 = 0;
-#pragma unroll 1
-  for (int i = 0; i < 32; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
 #pragma unroll 1
   for (;;) {
 #pragma unroll 1
-    for (int i = 0; i < 64; ++i) {
+    for (int i = 0; i < 64; ++i)
       if (mbar_try_wait(bar, parity)) return true;
-      __nanosleep(20);   // measured with 0, 20, 100 and 400 ns: no difference in kernel time or board power
-    }
     if (*abort_flag != 0) return false;
     const unsigned long long now = global_ns();
     if (t0 == 0) t0 = now;
     else if (now - t0 > limit_ns) return false;
   }
 }
-// Whole-warp wait: lane 0 polls (one try first: the common case is a barrier that has already flipped);
-// the warp barrier orders the acquired data for the other lanes, the vote shares the result.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag, int lane) {
-  int ok = 1;
-  if (lane == 0) {
-    if (!mbar_try_wait(bar, parity)) ok = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
+// Whole-warp wait.  All lanes try together (one access, the same word) and vote: 111 cycles per hop between two warps beside
+// thirteen waiting ones, against 207 with one polling lane and a warp barrier behind it.  The vote keeps the branch uniform.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, const volatile int* abort_flag) {
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+    const unsigned long long now = global_ns();
+    if (t0 == 0) t0 = now;
+    if (__any_sync(0xffffffffu, now - t0 > kWaitLimitNs)) return false;
   }
-  __syncwarp();
-  return __all_sync(0xffffffffu, ok) != 0;
-}
-// Two barriers at once: lane 0 polls the first, lane 1 the second, in the same instruction stream, so the
-// pair costs one shared-memory round trip instead of two back to back (each is ~180 cycles even when the
-// barrier has long flipped, and the elementwise warps pay it once per pair of tiles).
-__device__ __forceinline__ bool warp_wait2(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b,
-                                           const volatile int* abort_flag, int lane) {
-  int ok = 1;
-  if (lane < 2) {
-    const uint32_t bar = lane == 0 ? bar_a : bar_b;
-    const uint32_t parity = lane == 0 ? parity_a : parity_b;
-    if (!mbar_try_wait(bar, parity)) ok = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-  }
-  __syncwarp();
-  return __all_sync(0xffffffffu, ok) != 0;
 }
 
-// Wait for barrier A and, in the same shared-memory round trip, LOOK at barrier B (mbarrier.test_wait: no
-// suspension).  Returns false on a time-out of A; *b_done tells whether B's phase had completed.  For a second
-// barrier that is needed a few hundred cycles later and has usually flipped by now: the later blocking wait (and
-// its ~180-cycle round trip) is then skipped.
+// Wait for barrier A, then LOOK at barrier B (mbarrier.test_wait: no suspension).  Returns false on a time-out of A; *b_done tells
+// whether B's phase had completed.  For a second barrier that is needed a few hundred cycles later and has usually flipped by now.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -103,16 +87,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 __device__ __forceinline__ bool warp_wait_and_test(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b,
-                                                   const volatile int* abort_flag, int lane, bool* b_done) {
-  int ok = 1, done = 1;
-  if (lane == 0) {
-    if (!mbar_try_wait(bar_a, parity_a)) ok = mbar_wait(bar_a, parity_a, abort_flag) ? 1 : 0;
-  } else if (lane == 1) {
-    done = mbar_test(bar_b, parity_b) ? 1 : 0;
-  }
-  __syncwarp();
-  *b_done = __all_sync(0xffffffffu, done) != 0;
-  return __all_sync(0xffffffffu, ok) != 0;
+                                                   const volatile int* abort_flag, bool* b_done) {
+  const bool ok = warp_wait(bar_a, parity_a, abort_flag);
+  *b_done = __all_sync(0xffffffffu, mbar_test(bar_b, parity_b)) != 0;
+  return ok;
 }
 
 // The executing thread's earlier cp.async copies arrive on the barrier when they have landed (the arrival is one
@@ -131,6 +109,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
 // One 2-D box shared -> global (bulk async-group completion: commit, then wait for the reads of shared memory).
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
@@ -216,6 +199,30 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// One lane of a converged warp, always the same one.  The compiler keeps what such a branch computes in uniform registers, where
+// tcgen05.mma wants its operands: eight MMAs of M64 x N128 x K16 issued and completed in 847 cycles beside eight busy warps, and
+// three such streams at 45 cycles per MMA, against 1086 and 57 from an `if (lane == 0)`.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// D[tmem] (+)= A B with M = 64 on all 128 lanes: lanes 0-63 hold the first half of the N columns, lanes 64-127 the second, and an A
+// operand in tensor memory is read by each lane half from its own lanes.
+__device__ __forceinline__ void mma_ws_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
 // mbarrier arrives once every tcgen05 operation issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -255,6 +262,11 @@ __device__ __forceinline__ void tmem_st(uint32_t taddr, const uint32_t (&r)[16])
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Registers of a thread from here on; executed by all four warps of a warp group.  The shares of all groups together may not
+// exceed what the block was launched with, and only code that the instruction dominates is compiled for its share.
+template <int N> __device__ __forceinline__ void registers_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void registers_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
