@@ -149,7 +149,7 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (threadIdx.x == 0) report_timeout(49);
     return;
   }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int qtile = blockIdx.x;
   const long long bh = blockIdx.y;
   const int sub = be / kWRows, Qb = (int)(Lq / be);
@@ -196,55 +196,8 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const uint32_t tmem_o = tmem + 128 * kWfGroups;
   bool ok = true;
 
-  if (warp == 0 || warp == 1) {
-    const bool is_k = warp == 0;
-    const CUtensorMap* map = is_k ? &map_k : &map_v;
-    const int full0 = is_k ? WF_K_FULL : WF_V_FULL, empty0 = is_k ? WF_K_EMPTY : WF_V_EMPTY;
-    const uint32_t ring = base + (is_k ? Sm::k : Sm::v);
-    if (lane == 0) {
-      for (int p = 0; p < n_tiles; ++p) {
-        const int s = p % Sm::stages;
-        const int row = (int)(list[p] >> 8) << 7;
-        ok = VSA_WAIT(bar(empty0 + s), ((p / Sm::stages) & 1) ^ 1);
-        if (!ok) break;
-        mbar_arrive_expect_tx(bar(full0 + s), Sm::tile);
-        wide_load<HD>(ring + s * Sm::tile, map, row, kWHalf, bar(full0 + s));
-      }
-      if (!ok) report_timeout(41);
-    }
-  } else if (warp == 2) {
-    if (lane == 0) {   // S = Q K^T
-      ok = VSA_WAIT(bar(WF_Q_FULL), 0);
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::stages, b = p % kWfGroups;
-        ok = VSA_WAIT(bar(WF_K_FULL + s), (p / Sm::stages) & 1) && VSA_WAIT(bar(WF_S_EMPTY + b), ((p / kWfGroups) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
-        wide_issue_scores<HD, 128, kWHalf>(tmem + b * 128, base + Sm::q, base + Sm::k + s * Sm::tile);
-        mma_commit(bar(WF_K_EMPTY + s));
-        mma_commit(bar(WF_S_FULL + b));
-      }
-      if (!ok) report_timeout(42);
-    }
-  } else if (warp == 3) {
-    if (lane == 0) {   // O += P V
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::stages, b = p % kWfGroups;
-        ok = VSA_WAIT(bar(WF_V_FULL + s), (p / Sm::stages) & 1) && VSA_WAIT(bar(WF_P_FULL + b), (p / kWfGroups) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128, base + Sm::v + s * Sm::tile, p > 0);
-        ok = VSA_WAIT(bar(WF_P2_FULL + b), (p / kWfGroups) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128 + 32, base + Sm::v + s * Sm::tile + 64 * 128, true);
-        mma_commit(bar(WF_V_EMPTY + s));
-        mma_commit(bar(WF_S_EMPTY + b));
-      }
-      if (ok) mma_commit(bar(WF_O_FULL));
-      if (!ok) report_timeout(45);
-    }
-  } else {
+  if (warp >= 4) {          // 3 x 152 + 56 registers are the four groups' 128 at launch
+    registers_inc<152>();
     // softmax: a thread owns query row `row`; group g takes every third key tile, in its own accumulator
     const int quarter = warp & 3, g = (warp - 4) >> 2;
     const int row = quarter * 32 + lane, st = tid - 128;
@@ -289,7 +242,7 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           uint8_t* vrow = sm + Sm::v + s * Sm::tile + row * 128;
 #pragma unroll
           for (int ch = 0; ch < HD / 8; ++ch)
-            *reinterpret_cast<uint4*>(vrow + (ch >> 3) * kWHalf + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(vrow + (ch >> 3) * kWHalf + ((ch ^ row) & 7) * 16) = make_uint4(0, 0, 0, 0);   // all banks
         }
         fence_proxy_async_smem();
       }
@@ -383,6 +336,66 @@ sparse_fwd_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const bool redo = (misc[2 + (row >> 6)] != 0u) && ok;
       lse2[row0 + row] = (redo || n_tiles == 0) ? NAN : m_row[row] + log2f(l);
     }
+  } else {
+    registers_dec<56>();
+    if (warp == 0 || warp == 1) {
+      const bool is_k = warp == 0;
+      const CUtensorMap* map = is_k ? &map_k : &map_v;
+      const int full0 = is_k ? WF_K_FULL : WF_V_FULL, empty0 = is_k ? WF_K_EMPTY : WF_V_EMPTY;
+      const uint32_t ring = base + (is_k ? Sm::k : Sm::v);
+      for (int p = 0; p < n_tiles; ++p) {
+        const int s = p % Sm::stages;
+        const int row = (int)(list[p] >> 8) << 7;
+        ok = VSA_WARP_WAIT(bar(empty0 + s), ((p / Sm::stages) & 1) ^ 1);
+        if (!ok) break;
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar(full0 + s), Sm::tile);
+          wide_load<HD>(ring + s * Sm::tile, map, row, kWHalf, bar(full0 + s));
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) report_timeout(41);
+    } else if (warp == 2) {
+      // S = Q K^T
+      ok = VSA_WARP_WAIT(bar(WF_Q_FULL), 0);
+      for (int p = 0; p < n_tiles && ok; ++p) {
+        const int s = p % Sm::stages, b = p % kWfGroups;
+        ok = VSA_WARP_WAIT(bar(WF_K_FULL + s), (p / Sm::stages) & 1) && VSA_WARP_WAIT(bar(WF_S_EMPTY + b), ((p / kWfGroups) & 1) ^ 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          wide_issue_scores<HD, 128, kWHalf>(tmem + b * 128, base + Sm::q, base + Sm::k + s * Sm::tile);
+          mma_commit(bar(WF_K_EMPTY + s));
+          mma_commit(bar(WF_S_FULL + b));
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) report_timeout(42);
+    } else if (warp == 3) {
+      // O += P V
+      for (int p = 0; p < n_tiles && ok; ++p) {
+        const int s = p % Sm::stages, b = p % kWfGroups;
+        ok = VSA_WARP_WAIT(bar(WF_V_FULL + s), (p / Sm::stages) & 1) && VSA_WARP_WAIT(bar(WF_P_FULL + b), (p / kWfGroups) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128, base + Sm::v + s * Sm::tile, p > 0);
+        }
+        __syncwarp();
+        ok = VSA_WARP_WAIT(bar(WF_P2_FULL + b), (p / kWfGroups) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          wide_issue_product<HD, 64, 128, 128>(tmem_o, tmem + b * 128 + 32, base + Sm::v + s * Sm::tile + 64 * 128, true);
+          mma_commit(bar(WF_V_EMPTY + s));
+          mma_commit(bar(WF_S_EMPTY + b));
+        }
+        __syncwarp();
+      }
+      if (ok && elect_one()) mma_commit(bar(WF_O_FULL));
+      __syncwarp();
+      if (!ok && lane == 0) report_timeout(45);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -434,7 +447,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (threadIdx.x == 0) report_timeout(59);
     return;
   }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int qtile = blockIdx.x;
   const long long bh = blockIdx.y;
   const int sub = be / kWRows, Qb = (int)(Lq / be);
@@ -511,62 +524,73 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   bool ok = true;
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int p = 0; p < n_tiles; ++p) {
-        const int sk = p % Sm::k_stages, sv = p % Sm::v_stages;
-        const int krow = (int)(list[p] >> 8) << 7;
-        ok = VSA_WAIT(bar(WQ_K_EMPTY + sk), ((p / Sm::k_stages) & 1) ^ 1);
-        if (!ok) break;
+    for (int p = 0; p < n_tiles; ++p) {
+      const int sk = p % Sm::k_stages, sv = p % Sm::v_stages;
+      const int krow = (int)(list[p] >> 8) << 7;
+      ok = VSA_WARP_WAIT(bar(WQ_K_EMPTY + sk), ((p / Sm::k_stages) & 1) ^ 1);
+      if (!ok) break;
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar(WQ_K_FULL + sk), Sm::tile);
         wide_load<HD>(base + Sm::k + sk * Sm::tile, &map_k, krow, kWHalf, bar(WQ_K_FULL + sk));
-        ok = VSA_WAIT(bar(WQ_V_EMPTY + sv), ((p / Sm::v_stages) & 1) ^ 1);
-        if (!ok) break;
+      }
+      __syncwarp();
+      ok = VSA_WARP_WAIT(bar(WQ_V_EMPTY + sv), ((p / Sm::v_stages) & 1) ^ 1);
+      if (!ok) break;
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar(WQ_V_FULL + sv), Sm::tile);
         wide_load<HD>(base + Sm::v + sv * Sm::tile, &map_v, krow, kWHalf, bar(WQ_V_FULL + sv));
       }
-      if (!ok) report_timeout(51);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(51);
   } else if (warp == 2) {
-    if (lane == 0) {   // S = Q K^T
-      ok = VSA_WAIT(bar(WQ_QDO_FULL), 0);
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::k_stages, b = p & 1;
-        ok = VSA_WAIT(bar(WQ_K_FULL + s), (p / Sm::k_stages) & 1) && VSA_WAIT(bar(WQ_S_EMPTY + b), ((p >> 1) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // S = Q K^T
+    ok = VSA_WARP_WAIT(bar(WQ_QDO_FULL), 0);
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int s = p % Sm::k_stages, b = p & 1;
+      ok = VSA_WARP_WAIT(bar(WQ_K_FULL + s), (p / Sm::k_stages) & 1) && VSA_WARP_WAIT(bar(WQ_S_EMPTY + b), ((p >> 1) & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_scores<HD, 128, kWHalf>(tmem + b * 128, base + Sm::q, base + Sm::k + s * Sm::tile);
         mma_commit(bar(WQ_S_FULL + b));
       }
-      if (!ok) report_timeout(52);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(52);
   } else if (warp == 1) {
-    if (lane == 0) {   // dP = dO V^T
-      ok = VSA_WAIT(bar(WQ_QDO_FULL), 0);
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::v_stages;
-        ok = VSA_WAIT(bar(WQ_V_FULL + s), (p / Sm::v_stages) & 1) && VSA_WAIT(bar(WQ_DP_EMPTY), (p & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // dP = dO V^T
+    ok = VSA_WARP_WAIT(bar(WQ_QDO_FULL), 0);
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int s = p % Sm::v_stages;
+      ok = VSA_WARP_WAIT(bar(WQ_V_FULL + s), (p / Sm::v_stages) & 1) && VSA_WARP_WAIT(bar(WQ_DP_EMPTY), (p & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_scores<HD, 128, kWHalf>(tmem_dp, base + Sm::d_o, base + Sm::v + s * Sm::tile);
         mma_commit(bar(WQ_V_EMPTY + s));
         mma_commit(bar(WQ_DP_FULL));
       }
-      if (!ok) report_timeout(56);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(56);
   } else if (warp == 3) {
-    if (lane == 0) {   // dQ += dS K
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::k_stages, b = p & 1;
-        ok = VSA_WAIT(bar(WQ_K_FULL + s), (p / Sm::k_stages) & 1) && VSA_WAIT(bar(WQ_DS_FULL + b), (p >> 1) & 1);
-        if (!ok) break;
-        tc_fence_after();
+    // dQ += dS K
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int s = p % Sm::k_stages, b = p & 1;
+      ok = VSA_WARP_WAIT(bar(WQ_K_FULL + s), (p / Sm::k_stages) & 1) && VSA_WARP_WAIT(bar(WQ_DS_FULL + b), (p >> 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_product<HD, 128, kWqCols>(tmem_acc, tmem + b * 128, base + Sm::k + s * Sm::tile, p > 0);
         mma_commit(bar(WQ_K_EMPTY + s));
         mma_commit(bar(WQ_S_EMPTY + b));
       }
-      if (ok) mma_commit(bar(WQ_ACC_FULL));
-      if (!ok) report_timeout(53);
+      __syncwarp();
     }
+    if (ok && elect_one()) mma_commit(bar(WQ_ACC_FULL));
+    __syncwarp();
+    if (!ok && lane == 0) report_timeout(53);
   } else {
     const int c0 = cg * kWqCols, st = tid - 128;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
@@ -586,7 +610,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           uint8_t* krow = sm + Sm::k + (p % Sm::k_stages) * Sm::tile + row * 128;
 #pragma unroll
           for (int ch = 0; ch < HD / 8; ++ch)
-            *reinterpret_cast<uint4*>(krow + (ch >> 3) * kWHalf + (ch & 7) * 16) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(krow + (ch >> 3) * kWHalf + ((ch ^ row) & 7) * 16) = make_uint4(0, 0, 0, 0);
         }
         fence_proxy_async_smem();
       }
@@ -624,17 +648,21 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(WQ_DS_FULL + b));
     }
+    // block-mean backward folded in: query row r of the block also receives dmean[block] / max(size, 1) while r < size
+    float mean = 0.f;
+    bool mean_row = false;
+    if (mean_grad != nullptr) {
+      const int size = q_sizes[qb];
+      mean_row = row < size - (qtile % sub) * kWRows;
+      if (st < HD) mean = Elem<elem_t>::to(mean_grad[(bh * Qb + qb) * (long long)HD + st]) / (float)(size > 1 ? size : 1);
+    }
     if (!ok && lane == 0) report_timeout(54);
     // as in the forward: Q, over which dQ is staged, may still be landing when the route has no live tile
     if (ok) ok = VSA_WARP_WAIT(bar(n_tiles > 0 ? WQ_ACC_FULL : WQ_QDO_FULL), 0);
     if (!ok && lane == 0) report_timeout(55);
     tc_fence_after();
-    // block-mean backward folded in: query row r of the block also receives dmean[block] / max(size, 1) while r < size
-    float inv = 0.f;
-    if (mean_grad != nullptr) {
-      const int size = q_sizes[qb];
-      if (row < size - (qtile % sub) * kWRows) inv = (float)(size > 1 ? size : 1);
-    }
+    if (st < HD) s_delta[st] = mean;       // every row's delta has long been read
+    named_barrier(1, kWqEwThreads);
     uint8_t* stage = sm + Sm::q;
     for (int j = cg; j < HD / 32; j += kWqGroups) {
       uint32_t av[32];
@@ -649,11 +677,7 @@ sparse_dq_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
         for (int i = 0; i < 32; ++i) av[i] = 0u;
       }
-      if (inv > 0.f) {
-        const elem_t* mg = mean_grad + (bh * Qb + qb) * (long long)HD + 32 * j;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) av[i] = __float_as_uint(__uint_as_float(av[i]) + Elem<elem_t>::to(mg[i]) / inv);
-      }
+      if (mean_row) wide_add_mean(av, s_delta + 32 * j);
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4)
         *reinterpret_cast<uint4*>(stage + row * (HD * 2) + (((4 * j + q4) ^ (row & 7)) << 4)) = wide_pack8(av + 8 * q4);
@@ -716,7 +740,7 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (threadIdx.x == 0) report_timeout(69);
     return;
   }
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int ktile = blockIdx.x;
   const long long bh = blockIdx.y;
   const int sub = be / kWRows, qsub = be / kTile;
@@ -817,58 +841,70 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
     if (!ok && lane == 0) report_timeout(61);
   } else if (warp == 2) {
-    if (lane == 0) {   // S^T = K Q^T
-      ok = VSA_WAIT(bar(WK_KV_FULL), 0);
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::q_stages, b = p & 1;
-        ok = VSA_WAIT(bar(WK_Q_FULL + s), (p / Sm::q_stages) & 1) && VSA_WAIT(bar(WK_S_EMPTY + b), ((p >> 1) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // S^T = K Q^T
+    ok = VSA_WARP_WAIT(bar(WK_KV_FULL), 0);
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int s = p % Sm::q_stages, b = p & 1;
+      ok = VSA_WARP_WAIT(bar(WK_Q_FULL + s), (p / Sm::q_stages) & 1) && VSA_WARP_WAIT(bar(WK_S_EMPTY + b), ((p >> 1) & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_scores<HD, 64, kSlab>(tmem + b * 128, base + Sm::k, base + Sm::q + s * Sm::part);
         mma_commit(bar(WK_S_FULL + b));
       }
-      if (!ok) report_timeout(62);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(62);
   } else if (warp == 1) {
-    if (lane == 0) {   // dP^T = V dO^T
-      ok = VSA_WAIT(bar(WK_KV_FULL), 0);
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int s = p % Sm::do_stages, b = p & 1;
-        ok = VSA_WAIT(bar(WK_DO_FULL + s), (p / Sm::do_stages) & 1) && VSA_WAIT(bar(WK_DP_EMPTY + b), ((p >> 1) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // dP^T = V dO^T
+    ok = VSA_WARP_WAIT(bar(WK_KV_FULL), 0);
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int s = p % Sm::do_stages, b = p & 1;
+      ok = VSA_WARP_WAIT(bar(WK_DO_FULL + s), (p / Sm::do_stages) & 1) && VSA_WARP_WAIT(bar(WK_DP_EMPTY + b), ((p >> 1) & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_scores<HD, 64, kSlab>(tmem + b * 128 + 64, base + Sm::v, base + Sm::d_o + s * Sm::part);
         mma_commit(bar(WK_DO_EMPTY + s));
         mma_commit(bar(WK_DP_FULL + b));
       }
-      if (!ok) report_timeout(66);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(66);
   } else if (warp == 3) {
-    if (lane == 0) {   // dV += P^T dO, dK += dS^T Q
-      for (int p = 0; p < n_tiles && ok; ++p) {
-        const int sq = p % Sm::q_stages, sd = p % Sm::do_stages, b = p & 1;
-        const uint32_t ph = (p >> 1) & 1;
-        ok = VSA_WAIT(bar(WK_DO_FULL + sd), (p / Sm::do_stages) & 1) && VSA_WAIT(bar(WK_P_FULL + b), ph);
-        if (!ok) break;
-        tc_fence_after();
+    // dV += P^T dO, dK += dS^T Q
+    for (int p = 0; p < n_tiles && ok; ++p) {
+      const int sq = p % Sm::q_stages, sd = p % Sm::do_stages, b = p & 1;
+      const uint32_t ph = (p >> 1) & 1;
+      ok = VSA_WARP_WAIT(bar(WK_DO_FULL + sd), (p / Sm::do_stages) & 1) && VSA_WARP_WAIT(bar(WK_P_FULL + b), ph);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_product<HD, 64, kWkCols>(tmem_dv, tmem + b * 128, base + Sm::d_o + sd * Sm::part, p > 0);
         mma_commit(bar(WK_DO_EMPTY + sd));
         mma_commit(bar(WK_S_EMPTY + b));
-        ok = VSA_WAIT(bar(WK_DS_FULL + b), ph);
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      ok = VSA_WARP_WAIT(bar(WK_DS_FULL + b), ph);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         wide_issue_product<HD, 64, kWkCols>(tmem_dk, tmem + b * 128 + 64, base + Sm::q + sq * Sm::part, p > 0);
         mma_commit(bar(WK_Q_EMPTY + sq));
         mma_commit(bar(WK_DP_EMPTY + b));
       }
-      if (ok) mma_commit(bar(WK_ACC_FULL));
-      if (!ok) report_timeout(63);
+      __syncwarp();
     }
+    if (ok && elect_one()) mma_commit(bar(WK_ACC_FULL));
+    __syncwarp();
+    if (!ok && lane == 0) report_timeout(63);
   } else {
     const int quarter = warp & 3, cg = (warp - 4) >> 2;
     const int row = quarter * 32 + lane, c0 = cg * kWkCols, st = tid - 128;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool live = row < valid;
+    float mean = 0.f;                       // one of the 2 x HD values that a live row receives from the pooled gradients
+    if (mean_grad_k != nullptr && st < 2 * HD) mean = Elem<elem_t>::to(st < HD ? mean_grad_k[mean_off + st] : mean_grad_v[mean_off + st - HD]) * mean_inv;
     const float2 c2 = make_float2(-c, -c), m1 = make_float2(-1.f, -1.f);
     for (int p = 0; p < n_tiles && ok; ++p) {
       const int b = p & 1, sq = p % Sm::q_stages;
@@ -926,6 +962,9 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     tc_fence_after();
     uint8_t* stage_k = sm + Sm::k;          // every MMA is done: dK over K, dV over V
     uint8_t* stage_v = sm + Sm::v;
+    float* s_mean = reinterpret_cast<float*>(sm + Sm::stats);
+    if (st < 2 * HD) s_mean[st] = mean;
+    named_barrier(1, kWkEwThreads);
     for (int j = cg; j < 2 * (HD / 32); j += kWkGroups) {
       const bool is_k = j < HD / 32;
       const int jj = is_k ? j : j - HD / 32;
@@ -941,11 +980,7 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
         for (int i = 0; i < 32; ++i) av[i] = 0u;
       }
-      if (mean_grad_k != nullptr && live) {
-        const elem_t* mg = (is_k ? mean_grad_k : mean_grad_v) + mean_off + 32 * jj;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) av[i] = __float_as_uint(fmaf(Elem<elem_t>::to(mg[i]), mean_inv, __uint_as_float(av[i])));
-      }
+      if (mean_grad_k != nullptr && live) wide_add_mean(av, s_mean + 32 * j);
 #pragma unroll
       for (int q4 = 0; q4 < 4; ++q4)
         *reinterpret_cast<uint4*>((is_k ? stage_k : stage_v) + row * (HD * 2) + (((4 * jj + q4) ^ (row & 7)) << 4)) = wide_pack8(av + 8 * q4);
@@ -966,7 +1001,7 @@ sparse_dkdv_wide_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 }
 
 // ---- host launchers of the 128-row kernels -----------------------------------------------------------------------
-// Taken for block volumes that are multiples of 128, where sparse_wide_rows (and, at head dim 64, sparse_wide64_pays) says so.
+// Taken for block volumes that are multiples of 128, where sparse_wide_rows says so.
 template <int HD>
 int launch_fwd_wide(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes, void* out,
                     float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int be, int topk, float scale, cudaStream_t st,
