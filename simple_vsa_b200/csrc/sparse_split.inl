@@ -363,13 +363,6 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         neg_m = -m_row[r];
         shifted = true;
       }
-      if (valid < kTile && idx < n_live) {  // padding rows of V meet P = 0 in the product: they must be finite (0 * NaN)
-        const int i = p * kParts + r / kVRows, s = i % kSfStages;
-        ok = VSA_WARP_WAIT(bar(SF_V_FULL + s), (i / kSfStages) & 1);
-        if (!ok) break;
-        if (r >= valid) split_zero_row<HD>(sm + Sm::v + s * Sm::part + half * (Sm::part / 2) + (r % kVRows) * 128, r, kVRows * 128);
-        fence_proxy_async_smem();
-      }
       const float2 c2 = make_float2(c, c), m2 = make_float2(neg_m, neg_m);
       uint32_t pk[2][16];
       // full and ragged tiles are separate code: a mask costs two more instructions per score
@@ -390,6 +383,15 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       };
       if (valid == kTile) exponentiate(std::false_type{});
       else exponentiate(std::true_type{});
+      if (valid < kTile && idx < n_live) {
+        // padding rows of V meet P = 0 in the product: they must be finite (0 * NaN).  V of this pair may be under way still, so
+        // its rows come after the exponentials
+        const int i = p * kParts + r / kVRows, s = i % kSfStages;
+        ok = VSA_WARP_WAIT(bar(SF_V_FULL + s), (i / kSfStages) & 1);
+        if (!ok) break;
+        if (r >= valid) split_zero_row<HD>(sm + Sm::v + s * Sm::part + half * (Sm::part / 2) + (r % kVRows) * 128, r, kVRows * 128);
+        fence_proxy_async_smem();
+      }
       ok = VSA_WARP_WAIT(bar(SF_P_EMPTY), (p & 1) ^ 1);
       if (!ok) break;
       tc_fence_after();
@@ -808,19 +810,19 @@ template <int HD>
 struct SkSmem {
   static constexpr uint32_t part = 16384;
   static constexpr uint32_t pair = (HD / 64) * part;
-  static constexpr int stages = 3;                                // of Q pairs and of dO pairs
+  static constexpr int q_stages = 3, do_stages = 3;               // pairs
   static constexpr uint32_t k = 0;                                // resident K tile, [HD/64][64 rows][128 bytes]
   static constexpr uint32_t q = k + HD * 128;
-  static constexpr uint32_t d_o = q + stages * pair;
-  static constexpr uint32_t stats = d_o + stages * pair;          // per Q stage and tile: lse [64], delta [64]
-  static constexpr uint32_t mean = stats + stages * 1024;         // float [2][HD]: what a live row receives from the pooled gradients
+  static constexpr uint32_t d_o = q + q_stages * pair;
+  static constexpr uint32_t stats = d_o + do_stages * pair;       // per Q stage and tile: lse [64], delta [64]
+  static constexpr uint32_t mean = stats + q_stages * 1024;        // float [2][HD]: what a live row receives from the pooled gradients
   static constexpr uint32_t bars = mean + 2 * HD * 4;
   static constexpr uint32_t misc = bars + 32 * 8;
   static constexpr uint32_t total = misc + 32;
 };
 static_assert(SkSmem<128>::total + 1024 <= 232448, "shared memory of the split dK/dV pass");
-enum SkBar { SK_K_FULL = 0, SK_V_FULL = 1, SK_VT_FULL = 2, SK_Q_FULL = 3, SK_Q_EMPTY = 6, SK_DO_FULL = 9, SK_DO_EMPTY = 12,
-             SK_S_FULL = 15, SK_S_EMPTY, SK_DP_FULL, SK_DP_EMPTY, SK_P_FULL, SK_P_EMPTY, SK_DS_FULL, SK_DS_EMPTY, SK_ACC_FULL };
+enum SkBar { SK_K_FULL = 0, SK_V_FULL = 1, SK_VT_FULL = 2, SK_Q_FULL = 3, SK_Q_EMPTY = 7, SK_DO_FULL = 11, SK_DO_EMPTY = 14,
+             SK_S_FULL = 17, SK_S_EMPTY, SK_DP_FULL, SK_DP_EMPTY, SK_P_FULL, SK_P_EMPTY, SK_DS_FULL, SK_DS_EMPTY, SK_ACC_FULL };
 
 template <int HD>
 __global__ void __launch_bounds__(kSkThreads, 1)
@@ -833,7 +835,7 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                          long long Lkv, long long kv_shard, int sub, int topk, float scale, RasterMap out_map) {
   using Sm = SkSmem<HD>;
   constexpr int kParts = HD / 64;
-  constexpr uint32_t kStage = Sm::d_o + (Sm::stages - 1) * Sm::pair;      // V on its way to tensor memory, in the last dO stage
+  constexpr uint32_t kStage = Sm::d_o + (Sm::do_stages - 1) * Sm::pair;      // V on its way to tensor memory, in the last dO stage
   extern __shared__ uint8_t smem_raw[];
   if (*(volatile int*)&g_device_status != 0) return;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -882,9 +884,11 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     mbar_init(bar(SK_K_FULL), 1);
     mbar_init(bar(SK_V_FULL), 1);
     mbar_init(bar(SK_VT_FULL), 4 * kParts);
-    for (int i = 0; i < Sm::stages; ++i) {
+    for (int i = 0; i < Sm::q_stages; ++i) {
       mbar_init(bar(SK_Q_FULL + i), 2 * kParts + 32);      // the boxes' lanes and 32 lanes' copies of the statistics
       mbar_init(bar(SK_Q_EMPTY + i), 1);
+    }
+    for (int i = 0; i < Sm::do_stages; ++i) {
       mbar_init(bar(SK_DO_FULL + i), 2 * kParts);
       mbar_init(bar(SK_DO_EMPTY + i), 2);                  // read by the dP products of one issuer and the dV products of another
     }
@@ -934,9 +938,9 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
     const float2 c2 = make_float2(-c, -c), m1 = make_float2(-1.f, -1.f);
     for (int p = 0; p < n_pairs && ok; ++p) {
-      const int s = p % Sm::stages;
+      const int s = p % Sm::q_stages;
       const uint32_t ph = p & 1;
-      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::stages) & 1, bar(SK_S_FULL), ph);
+      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::q_stages) & 1, bar(SK_S_FULL), ph);
       if (!ok) break;
       tc_fence_after();
       const float4* s_lse = reinterpret_cast<const float4*>(sm + Sm::stats + s * 1024 + half * 512 + c0 * 4);
@@ -1020,10 +1024,10 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
   } else if (warp == 0) {   // Q pairs with the statistics of their rows; a lane per tile and 64 head dims
     for (int p = 0; p < n_pairs; ++p) {
-      const int s = p % Sm::stages, h = lane >> 1;
+      const int s = p % Sm::q_stages, h = lane >> 1;
       const bool second = 2 * p + 1 < n_tiles;             // otherwise it lies outside the tensor: zeros, and P = 2^-inf = 0
       const long long row_a = tile_row(2 * p), row_b = second ? tile_row(2 * p + 1) : BH * Lq;
-      ok = VSA_WARP_WAIT(bar(SK_Q_EMPTY + s), ((p / Sm::stages) & 1) ^ 1);
+      ok = VSA_WARP_WAIT(bar(SK_Q_EMPTY + s), ((p / Sm::q_stages) & 1) ^ 1);
       if (!ok) break;
       const uint32_t st = base + Sm::stats + s * 1024 + lane * 4;
       cp_async4(st, lse2 + row_a + lane);
@@ -1051,9 +1055,9 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (!ok && lane == 0) report_timeout(91);
   } else if (warp == 1) {   // dO pairs
     for (int p = 0; p < n_pairs; ++p) {
-      const int s = p % Sm::stages, h = lane >> 1, i = 2 * p + (lane & 1);
+      const int s = p % Sm::do_stages, h = lane >> 1, i = 2 * p + (lane & 1);
       const int row = (int)(i < n_tiles ? tile_row(i) : BH * Lq);
-      ok = VSA_WARP_WAIT(bar(SK_DO_EMPTY + s), ((p / Sm::stages) & 1) ^ 1) && (p != Sm::stages - 1 || VSA_WARP_WAIT(bar(SK_VT_FULL), 0));
+      ok = VSA_WARP_WAIT(bar(SK_DO_EMPTY + s), ((p / Sm::do_stages) & 1) ^ 1) && (p != Sm::do_stages - 1 || VSA_WARP_WAIT(bar(SK_VT_FULL), 0));
       if (!ok) break;
       if (lane < 2 * kParts) {
         mbar_arrive_expect_tx(bar(SK_DO_FULL + s), kSlab);
@@ -1068,8 +1072,8 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const uint32_t a0 = desc_lo(base + Sm::k, 16);
     ok = VSA_WARP_WAIT(bar(SK_K_FULL), 0);
     for (int p = 0; p < n_pairs && ok; ++p) {
-      const int s = p % Sm::stages;
-      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::stages) & 1, bar(SK_S_EMPTY), (p & 1) ^ 1);
+      const int s = p % Sm::q_stages;
+      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::q_stages) & 1, bar(SK_S_EMPTY), (p & 1) ^ 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
@@ -1086,8 +1090,8 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   } else if (warp == 3) {   // dP^T = V dO^T
     ok = VSA_WARP_WAIT(bar(SK_VT_FULL), 0);
     for (int p = 0; p < n_pairs && ok; ++p) {
-      const int s = p % Sm::stages;
-      ok = VSA_WARP_WAIT2(bar(SK_DO_FULL + s), (p / Sm::stages) & 1, bar(SK_DP_EMPTY), (p & 1) ^ 1);
+      const int s = p % Sm::do_stages;
+      ok = VSA_WARP_WAIT2(bar(SK_DO_FULL + s), (p / Sm::do_stages) & 1, bar(SK_DP_EMPTY), (p & 1) ^ 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
@@ -1102,8 +1106,8 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (!ok && lane == 0) report_timeout(94);
   } else if (warp == 12) {  // dV += P^T dO
     for (int p = 0; p < n_pairs && ok; ++p) {
-      const int s = p % Sm::stages;
-      ok = VSA_WARP_WAIT2(bar(SK_DO_FULL + s), (p / Sm::stages) & 1, bar(SK_P_FULL), p & 1);
+      const int s = p % Sm::do_stages;
+      ok = VSA_WARP_WAIT2(bar(SK_DO_FULL + s), (p / Sm::do_stages) & 1, bar(SK_P_FULL), p & 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
@@ -1120,8 +1124,8 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (!ok && lane == 0) report_timeout(95);
   } else if (warp == 13) {  // dK += dS^T Q
     for (int p = 0; p < n_pairs && ok; ++p) {
-      const int s = p % Sm::stages;
-      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::stages) & 1, bar(SK_DS_FULL), p & 1);
+      const int s = p % Sm::q_stages;
+      ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::q_stages) & 1, bar(SK_DS_FULL), p & 1);
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
