@@ -46,11 +46,13 @@ static bool mma_forced() {
   return e && std::strcmp(e, "mma") == 0;
 }
 
-// The kernels that a pass of an ordinary call runs on: head dim 128 on tcgen05, head dim 64 with blocks of 128 or 256 tokens
-// on the 128-row tcgen05 kernels where they are the faster ones (sparse_wide64_pays).
+// The kernels that a pass of an ordinary call runs on: head dim 128 on tcgen05, head dim 64 too where it is the faster path.  Head
+// dim 64 has it in the ordinary layout only; the other entry points ask sparse_umma_eligible.
 static bool on_umma(SparsePass pass, int64_t BH, int64_t L, int D, int be, int dtype, int topk) {
-  return !scalar_forced() && !mma_forced() &&
-         (sparse_umma_eligible(D, be, dtype, topk) || (sparse_wide64_eligible(D, be, dtype, topk) && sparse_wide64_pays(pass, BH, L, be, topk)));
+  if (scalar_forced() || mma_forced()) return false;
+  if (sparse_umma_eligible(D, be, dtype, topk)) return true;
+  return sparse_umma64_eligible(D, be, dtype, topk) &&
+         (sparse_wide_rows(pass, BH, L, D, be, topk) || sparse_split64_pays(pass, BH, L, be, topk));
 }
 
 static int check_dtype(int dtype) {
@@ -491,7 +493,7 @@ int vsa_sparse_kernel_family(int D, int be, int topk, int dtype) {
 int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype) {
   VSA_REQUIRE(pass >= 0 && pass <= 2 && BH >= 1 && be >= 1 && L >= be && L % be == 0, "sparse pass kernels: bad arguments");
   if (scalar_forced()) return 0;
-  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk) ? 3 : 2;
+  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk) ? 3 : D == 128 ? 2 : 1;
   return sparse_tc_eligible(D, be, dtype) ? 1 : 0;
 }
 

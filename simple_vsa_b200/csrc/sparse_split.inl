@@ -173,8 +173,8 @@ struct SfSmem {
   static constexpr uint32_t q = v + kSfStages * part;             // head dims 64..127 of Q (0..63 are in tensor memory)
   static constexpr uint32_t list = q + (HD / 64 - 1) * kSlab;     // uint32 [kMaxTiles]
   static constexpr uint32_t m_row = list + 4 * kMaxTiles;         // float [64]
-  static constexpr uint32_t l_part = m_row + 256;                 // float [2 sums][128]
-  static constexpr uint32_t bars = l_part + 1024;
+  static constexpr uint32_t l_part = m_row + 256;                 // float [128]
+  static constexpr uint32_t bars = l_part + 512;
   static constexpr uint32_t misc = bars + 24 * 8;
   static constexpr uint32_t total = misc + 32;
 };
@@ -193,6 +193,10 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   using Sm = SfSmem<HD>;
   constexpr int kParts = HD / 64;
   constexpr int kVRows = 64 / kParts;               // keys of each tile in a part of V
+  // Head dim 64 takes the place of an online softmax, whose largest P is 1 exactly; with P rounded under a fixed shift the output was
+  // 2-3 % further from float64.  Its O leaves 64 columns free, so what the rounding of P loses is kept there, in the element type,
+  // and multiplied too.
+  constexpr bool kSplitP = HD == 64;
   constexpr uint32_t kQStage = Sm::v + (kSfStages - 1) * Sm::part;     // Q on its way to tensor memory, in the last part of V
   extern __shared__ uint8_t smem_raw[];
   if (*(volatile int*)&g_device_status != 0) return;
@@ -240,6 +244,7 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                   bh, BH, kv_shard, tid, kSfThreads);
   tc_fence_after();
   const uint32_t tmem_o = misc[0], tmem_s = tmem_o + 128, tmem_p = tmem_o + 192, tmem_q = tmem_o + 224;
+  const uint32_t tmem_plo = tmem_o + 64;            // head dim 64: what P lost in rounding
   const int n_live = (int)misc[1], n_pairs = (n_live + 1) >> 1;
   bool ok = true;
 
@@ -312,8 +317,10 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           const int s = (i0 + h) % kSfStages;
           const uint32_t b0 = desc_lo(base + Sm::v + s * Sm::part, kVRows * 128);
 #pragma unroll
-          for (int ks = 0; ks < kVRows / 16; ++ks)
+          for (int ks = 0; ks < kVRows / 16; ++ks) {
             mma_ws_ts(tmem_o, tmem_p + 8 * (h * (kVRows / 16) + ks), desc_pack(b0 + 128 * ks, hi), idesc, p > 0 || h > 0 || ks > 0 ? 1u : 0u);
+            if (kSplitP) mma_ws_ts(tmem_o, tmem_plo + 8 * ks, desc_pack(b0 + 128 * ks, hi), idesc, 1u);
+          }
           mma_commit(bar(SF_V_EMPTY + s));
         }
         mma_commit(bar(SF_P_EMPTY));
@@ -333,7 +340,7 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(SF_QT_FULL));
-    float2 lsum = make_float2(0.f, 0.f), lround = make_float2(0.f, 0.f);
+    float2 lsum = make_float2(0.f, 0.f);
     float neg_m = 0.f;
     bool shifted = n_pairs == 0;
     for (int p = 0; p < n_pairs && ok; ++p) {
@@ -364,7 +371,7 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         shifted = true;
       }
       const float2 c2 = make_float2(c, c), m2 = make_float2(neg_m, neg_m);
-      uint32_t pk[2][16];
+      uint32_t pk[2][16], lo[2][16];
       // full and ragged tiles are separate code: a mask costs two more instructions per score
       auto exponentiate = [&](auto ragged) {
 #pragma unroll
@@ -377,7 +384,10 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           }
           lsum = add2(lsum, e);
           const uint32_t w = Elem<elem_t>::pack(e.x, e.y);
-          if (HD == 64) lround = add2(lround, Elem<elem_t>::unpack(w));
+          if (kSplitP) {
+            const float2 rounded = Elem<elem_t>::unpack(w);
+            lo[i >> 4][i & 15] = Elem<elem_t>::pack(e.x - rounded.x, e.y - rounded.y);
+          }
           pk[i >> 4][i & 15] = w;
         }
       };
@@ -397,6 +407,10 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       tc_fence_after();
       tmem_st(tmem_p + lane_addr, pk[0]);
       tmem_st(tmem_p + lane_addr + 16, pk[1]);
+      if (kSplitP) {
+        tmem_st(tmem_plo + lane_addr, lo[0]);
+        tmem_st(tmem_plo + lane_addr + 16, lo[1]);
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -413,19 +427,15 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // add the two halves: each thread finishes half of the head dims of its row.  Every MMA is done, the rings are free.
     float* l_part = reinterpret_cast<float*>(sm + Sm::l_part);
     l_part[st] = lsum.x + lsum.y;
-    if (HD == 64) l_part[128 + st] = lround.x + lround.y;
     uint8_t* stage = sm + 64 * HD * 4;
-    float l = 0.f, norm = 0.f;
+    float l = 0.f;
     bool finite = true;
     split_add_halves<HD, HD>(tmem_o + lane_addr, ok && n_pairs > 0, sm, stage, 0, half, r, 1, [&](auto& ov, int) {
       l = l_part[r] + l_part[64 + r];
-      // Head dim 64 replaces an online softmax whose largest P is 1 exactly.  Normalising by the sum of the probabilities as they
-      // enter the product, i.e. rounded, takes their common rounding error out again; the statistic keeps the exact sum.
-      norm = HD == 64 ? l_part[128 + r] + l_part[192 + r] : l;
       finite = finite && l <= 3.0e38f;
 #pragma unroll
       for (auto& w : ov) {
-        const float o = __uint_as_float(w) / norm;
+        const float o = __uint_as_float(w) / l;
         finite = finite && fabsf(o) <= 3.0e38f;
         w = n_pairs == 0 ? 0x7fc00000u : __float_as_uint(o);
       }

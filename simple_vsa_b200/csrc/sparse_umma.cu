@@ -287,6 +287,27 @@ static int sm_count() {
   return 148;
 }
 
+// Head dim 64, blocks of 128 and 256 tokens: the 128-row kernels or 64-row ones.  us at [1, 12, 16384, 64], blocks of 128, 128-row
+// kernels / mma.sync, by 64-token tiles per route: forward 8: 134 / 104, 12: 149 / 149, 16: 166 / 193; dQ 8: 183 / 142, 12: 204 / 199,
+// 16: 226 / 254; dK/dV 2: 82 / 77, 4: 108 / 120.  Where the 128-row CTAs just fill the SMs once they win earlier: [1, 4, 4096, 64],
+// 8 tiles: forward 13.0 / 15.0, dQ 10.7 / 20.4.
+static bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
+  if (pass == kPassDkdv) return true;
+  const int64_t sms = sm_count(), rows128 = BH * (L / 128);
+  return topk * (be / kTile) > (rows128 <= sms && 2 * rows128 > sms ? 4 : 8);
+}
+// Head dim 64 on 64-row tiles: tcgen05 (sparse_split.inl) or mma.sync, of which three or four CTAs share an SM and need little set-up,
+// so that they are faster while a route holds few tiles.  us, tcgen05 / mma.sync, by tiles per route:
+//   [1, 12, 16384, 64]  forward 4: 97 / 60, 8: 113 / 103, 16: 144 / 190, 32: 206 / 364;  dQ 4: 141 / 86, 8: 162 / 142, 16: 206 / 255, 32: 291 / 482;
+//                       dK/dV 4: 151 / 118, 8: 187 / 195, 16: 257 / 349, 32: 394 / 652
+//   [1, 2, 2048, 64], all tiles on the SMs at once: forward 2: 8.4 / 4.8, 8: 10.6 / 11.5;  dQ 2: 6.7 / 7.1, 8: 8.5 / 14.7;  dK/dV 2: 8.0 / 13.5, 8: 11.5 / 23.6
+bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
+  const int64_t n = (int64_t)topk * (be / kTile);
+  const bool one_wave = BH * (L / kTile) <= sm_count();
+  if (pass == kPassForward) return n > (one_wave ? 4 : 8);
+  return one_wave || n > (pass == kPassDq ? 8 : 6);
+}
+
 // Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as tiles of 64 tokens.  Both
 // run one CTA per SM; a 128-row CTA does twice the rows in less than twice the time, so the 64-token kernels are the faster
 // ones where halving the CTAs saves no wave (times on one B200, head dim 128, full blocks, us, 64-token / 128-row):
@@ -301,7 +322,7 @@ static int sm_count() {
 // tiles a route that was measured.  A wave of the forward costs 1.1 times as much on 128 rows and of dK/dV 1.25 times, at any n.
 bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk) {
   if (be % 128 != 0) return false;
-  if (D == 64) return true;                       // there are no 64-token tcgen05 kernels at this head dim
+  if (D == 64) return sparse_wide64_pays(pass, BH, L, be, topk);
   const int64_t sms = sm_count();
   const int64_t narrow = (BH * (L / 64) + sms - 1) / sms, wide = (BH * (L / 128) + sms - 1) / sms;
   if (pass != kPassDq) return narrow > 1;
@@ -315,23 +336,8 @@ bool sparse_umma_eligible(int D, int be, int dtype, int topk) {
   return false;
 }
 
-bool sparse_wide64_eligible(int D, int be, int dtype, int topk) {
-  return D == 64 && (be == 128 || be == 256) && (dtype == VSA_BF16 || dtype == VSA_F16) && topk * (be / kTile) <= kMaxTiles;
-}
-
-// A CTA of the 128-row kernels has an SM to itself and spends several us on set-up and drain; four mma.sync CTAs (three in the
-// backward) share an SM and need little of either, so they are faster while a route holds few tiles.  us at [1, 12, 16384, 64],
-// blocks of 128, full blocks, 128-row kernels / mma.sync, by 64-token tiles per route:
-//   forward  2: 106 / 39   4: 117 / 60    8: 134 / 104   12: 149 / 149   16: 166 / 193
-//   dQ       2: 150 / 57   4: 161 / 85    8: 183 / 142   12: 204 / 199   16: 226 / 254
-//   dK/dV    2:  82 / 77   4: 108 / 120   8: 149 / 199   12: 185 / 278   16: 220 / 352
-// The forward and dQ cross between 8 and 12 tiles with blocks of 256 and on other grids too (32 to 25,600 row tiles), except
-// where the 128-row CTAs just fill the SMs once and the mma.sync CTAs have to share them: between 4 and 8 ([1, 4, 4096, 64],
-// 8 tiles: forward 15.1 / 14.1 us, dQ 22.5 / 17.2 us with the wide kernels second).
-bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
-  if (pass == kPassDkdv) return true;
-  const int64_t sms = sm_count(), rows128 = BH * (L / 128);
-  return topk * (be / kTile) > (rows128 <= sms && 2 * rows128 > sms ? 4 : 8);
+bool sparse_umma64_eligible(int D, int be, int dtype, int topk) {
+  return D == 64 && (be == 64 || be == 128 || be == 256) && (dtype == VSA_BF16 || dtype == VSA_F16) && topk * (be / kTile) <= kMaxTiles;
 }
 
 int64_t sparse_ds_workspace_bytes(int64_t BH, int64_t Lq, int be, int topk) {

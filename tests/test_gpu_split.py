@@ -1,0 +1,72 @@
+"""The 64-row tcgen05 kernels that put a tile of the other side on each lane half (blocks of 64 tokens at head dims 64 and 128, larger
+blocks on small grids) at the edges of their tiles, against the CPU oracle: odd and single tile counts (one half without a tile),
+more pairs than any ring is deep, live sizes around 0, 1, 32 (a part of V) and the full tile, query and key lengths that differ,
+whatever bits the padding rows hold, and score gaps beyond the range of the softmax shift."""
+
+import pytest
+import torch
+
+from oracle import vsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("be,qb,kb,tk", [(64, 1, 1, 1), (64, 3, 2, 2), (64, 5, 9, 3), (64, 4, 23, 17), (64, 26, 21, 8), (256, 1, 3, 1)])
+def test_64_row_tiles_match_the_oracle(be, qb, kb, tk, D, dtype):
+    from simple_vsa_b200 import _lib, b200_sparse_attention
+    g = torch.Generator().manual_seed(be + 7 * kb + D)
+    B, H = 1, 3
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    if be == 64 or D == 128:
+        for p, n in enumerate((qb, qb, kb)):
+            assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == (2 if D == 128 else 1)
+    q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
+    sizes = torch.tensor(([be, 1, 0, 32, be - 1, 33, be, 31, be] * 3)[:kb])
+    for x in (k, v):
+        x.view(B, H, kb, be, D)[:, :, torch.arange(be)[None, :] >= sizes[:, None]] = float("nan")
+    clean = [torch.nan_to_num(x.float(), nan=0.0).to(dtype) for x in (k, v)]
+    selected = torch.rand(B, H, qb, kb, generator=g)
+    selected[..., 0] = 2.0                                # block 0 is full: every row has a live key
+    selected = selected.topk(tk, dim=-1).indices.to(torch.int32)
+    want_in = [q.clone().requires_grad_()] + [x.clone().requires_grad_() for x in clean]
+    want = O.sparse_attention(*want_in, selected, sizes, be, q_blocks_per_chunk=8)
+    want.backward(dout.float())
+    leaves = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    out = b200_sparse_attention(*leaves, selected.to(DEV), sizes, block_size=(1, 1, be))
+    out.backward(dout.to(DEV))
+    assert _lib.device_status() == 0
+    # operands, P and dS carry 2^-9 (bf16) or 2^-12 (fp16) each, summed over many keys: relative 2-norm error near one rounding,
+    # far below four of them
+    bound = 4 * 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    for got, ref in zip([out] + [x.grad for x in leaves], [want] + [x.grad for x in want_in]):
+        got, ref = got.detach().float().cpu(), ref.detach().float()
+        assert torch.isfinite(got).all()
+        assert (got - ref).norm() <= bound * ref.norm()
+    dead = torch.arange(be)[None, :] >= sizes[:, None]
+    for x in leaves[1:]:
+        assert (x.grad.view(B, H, kb, be, D)[:, :, dead.to(DEV)] == 0).all()
+
+
+@pytest.mark.parametrize("dtype,k_factor", [(torch.bfloat16, 8.0), (torch.float16, 1.5)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_tile_outside_the_shift_range_is_recomputed_exactly(D, dtype, k_factor):
+    """A block later in the route scores hundreds of binades above the first pair for every other query block."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator().manual_seed(D)
+    be, H, qb, kb, tk, scale = 64, 2, 6, 9, 7, D ** -0.5
+    q = torch.randn(1, H, qb * be, D, generator=g)
+    k, v = (torch.randn(1, H, kb * be, D, generator=g) for _ in range(2))
+    q.view(1, H, qb, be, D)[:, :, 1::2] *= 40.0 if dtype == torch.bfloat16 else 20.0
+    k.view(1, H, kb, be, D)[:, :, 3] *= k_factor
+    q, k, v = (x.to(dtype) for x in (q, k, v))
+    sizes = torch.tensor([5, 9, be, be, be - 3, be, 64, be, 1])
+    selected = torch.tensor([0, 1, 2, 3, 4, 5, 8], dtype=torch.int32).expand(1, H, qb, tk).contiguous()
+    want, want_lse = O.sparse_attention(q, k, v, selected, sizes, be, return_lse2=True)
+    out, lse = ops.sparse_forward(q.to(DEV), k.to(DEV), v.to(DEV), selected.to(DEV), sizes.to(DEV, torch.int32), be, scale, True)[:2]
+    assert _lib.device_status() == 0
+    torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=2e-2)
+    torch.testing.assert_close(lse.float().cpu(), want_lse.float(), atol=5e-2, rtol=1e-3)
