@@ -1,34 +1,17 @@
-// Fine (block-sparse) attention forward on the Blackwell tensor path: TMA tile gathers by
-// block id, tcgen05.mma with accumulators in tensor memory, warp-specialised softmax.
-//
-// Formulation.  A 64-row query tile gives only M = 64 for the usual S = Q K^T product, which
-// runs tcgen05 at half rate.  The kernel therefore computes the TRANSPOSED products on PAIRS of
-// selected key tiles:
-//     S^T [128 key tokens x 64 query rows] = K2 [128 x 128] * Q^T          (M 128, N 64, K 128)
-//     O^T [128 dims       x 64 query rows] += V2^T [128 x 128] * P^T       (M 128, N 64, K 128)
-// K2/V2 are two 64-token tiles stacked in shared memory by four TMA boxes each.  In tensor
-// memory a lane is then a key token and a column a query row, so the softmax statistics run
-// ACROSS lanes.  They are handled without per-tile cross-lane traffic:
-//   * the shift m[q] is the exact column maximum of the FIRST live pair only (one cross-lane
-//     reduction per CTA); softmax is shift-invariant, so any later score simply gives
-//     P = 2^(s-m) > 1, which bf16 and fp32 hold up to 2^127;
-//   * every thread keeps its own partial row sums (64 registers) and they are reduced across
-//     lanes once at the end;
-//   * if a sum or an output leaves the finite range (scores more than ~2^7 apart in log2
-//     units from the first pair's maximum) the tile writes NaN into its log-sum-exp rows and
-//     the exact warp-level kernel recomputes just those tiles in a follow-up launch.
-// P^T is written by its owner thread as one swizzled 128-byte row of shared memory (N-major B
-// operand), so no transposition is ever needed.
-//
-// Roles: warp 0 = K producer, warp 1 = V producer (four lanes, one TMA box each; warp 1 also owns the
-// tensor memory), warp 2 = issuer of the S^T MMAs, warp 3 = issuer of the O^T MMAs, warps 4-19 = softmax (a TMEM lane quarter and half of the
-// query-row columns each).  Every mbarrier wait is bounded; on a time-out the CTA records an error code in a
-// device status word, stops issuing work, frees its tensor memory and returns.
+// Fine (block-sparse) attention on the Blackwell tensor path: TMA tile gathers by block id, tcgen05.mma with accumulators in tensor
+// memory, warp-specialised elementwise stages.  This file has the host side, the self-tests and the choice between the kernels:
+//   sparse_split.inl     64-row tiles, a tile of the other side per lane half (blocks of 64 tokens; larger ones on small grids)
+//   sparse_wide.inl      128-row tiles (blocks of 128 and 256 tokens)
+//   sparse_umma_bwd.inl  the opt-in backward that forms dS once
+//   coarse_umma.inl      the pooled branch
+// The softmax of every forward uses a fixed shift, the row maximum over the first live tiles: softmax is shift-invariant, so a later
+// score simply gives P = 2^(s-m) > 1, which bf16 and fp32 hold up to 2^127.  If a sum or an output leaves the finite range the tile
+// writes NaN into its log-sum-exp rows and the exact warp-level kernel recomputes just those tiles in a follow-up launch.
+// Every mbarrier wait is bounded; on a time-out the CTA records an error code in a device status word, stops issuing work, frees
+// its tensor memory and returns.
 #include <cuda.h>
 
 #include <algorithm>
-#include <cstdlib>
-#include <cstring>
 #include <mutex>
 #include <type_traits>
 
@@ -52,9 +35,6 @@ constexpr int kSlab = 64 * 128;        // one TMA box: 64 rows x 128 bytes
 constexpr int kPairHalf = 2 * kSlab;   // 128 rows x 128 bytes (one head-dim half of a stacked pair)
 constexpr int kPairBytes = 2 * kPairHalf;
 constexpr uint32_t kTmemCols = 512;
-// K pairs in flight: a reload from L2 takes ~2000 cycles, two stages left the S^T issuer waiting for it
-constexpr int kFwdKStages = 2;
-constexpr int kSBufs = 4;              // S^T accumulators in flight (64 columns each); O^T sits behind them
 
 // ---- host: tensor maps ---------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -246,7 +226,7 @@ int check_kv_shard(int64_t Lkv, int be, int64_t* kv_shard, const char* what) {
 
 }  // namespace
 
-// The 64-token kernels walk a block of 64, 128 or 256 tokens as 1, 2 or 4 tiles (their SUB parameter).
+// The kernels of the stored-dS backward walk a block of 64, 128 or 256 tokens as 1, 2 or 4 tiles (their SUB parameter).
 #define VSA_BY_BLOCK_VOLUME(be_, launch_, kernel_) \
   return (be_) == 64 ? launch_(kernel_<1>) : (be_) == 128 ? launch_(kernel_<2>) : launch_(kernel_<4>)
 

@@ -1,360 +1,22 @@
-// Backward of the fine attention on the Blackwell tensor path.  Included by sparse_umma.cu (same
-// translation unit: the kernels share its device status word, tensor-map helper and constants).
+// The backward that forms dS once (opt-in) on the Blackwell tensor path.  Included by sparse_umma_typed.inl.
 //
-// Both passes use the transposed, 128-row formulation of the forward so that every tcgen05.mma has
-// M = 128 although a block holds only 64 tokens, and so that P / dS are produced by the thread that
-// owns their row and are written once, as a swizzled 128-byte shared-memory row (N-major B operand):
-//
-//  query-owned dQ pass, per PAIR of selected key tiles (lanes = 128 key tokens, columns = 64 query rows)
-//      S^T  = K2 Q^T                 dP^T = V2 dO^T
-//      dS^T = 2^(S^T c - lse[q]) * (dP^T - delta[q]) * scale      (elementwise, statistics per COLUMN)
-//      dQ^T [128 dims x 64 rows] += K2^T dS^T
-//
-//  key-owned dK/dV pass, per PAIR of query tiles that selected this key tile (lanes = 128 query rows,
-//  columns = 64 key tokens)
+// The key-owned pass works on transposed, 128-row products, per PAIR of query tiles that selected this key tile (lanes = 128 query
+// rows, columns = 64 key tokens):
 //      S  = Q2 K^T                   dP = dO2 V^T
 //      P  = 2^(S c - lse[row]),      dS = P * (dP - delta[row])   (elementwise, statistics per LANE)
 //      dV^T [128 dims x 64 keys] += dO2^T P          dK^T += Q2^T dS          (dK^T * scale at the end)
-//
-// Nothing here needs a running maximum (the forward saved the log-sum-exp), so there is no
-// cross-lane traffic at all.  Roles per CTA: warp 0 and 1 = TMA producers (four lanes, one box each),
-// warp 2 = issuer of the S MMAs, warp 3 = issuer of the gradient MMAs, warps 4-11 = elementwise (a TMEM
-// lane quarter x 32 of the 64 columns each), warp 12 = issuer of the dP MMAs (the three issuers wait on
-// different operands and must not hold one another back).
+// P / dS are written by the thread that owns their row, once, as a swizzled 128-byte shared-memory row (N-major B operand), and dS
+// goes to memory from the same registers; a query-owned pass then multiplies it by K.  Roles of the first: warp 0 and 1 = TMA
+// producers (four lanes, one box each), warp 2 = issuer of the S MMAs, warp 3 = issuer of the gradient MMAs, warps 4-11 = elementwise
+// (a TMEM lane quarter x 32 of the 64 columns each), warp 12 = issuer of the dP MMAs.
 
-// The backward passes are closest to the shared-memory bandwidth limit (every operand byte is read by an
-// MMA once or twice per pair); eight wider elementwise warps disturb that pipe less than sixteen narrow ones.
+// Every operand byte is read by an MMA once or twice per pair, close to the shared-memory bandwidth limit; eight wider elementwise
+// warps disturb that pipe less than sixteen narrow ones.
 constexpr int kBwCols = 32;
 constexpr int kBwWarps = 4 * (64 / kBwCols);
 constexpr int kBwEwThreads = 32 * kBwWarps;
 constexpr int kBwdThreads = 128 + kBwEwThreads + 32;   // ... plus the dP issuer, the last warp
 constexpr int kDpWarp = 4 + kBwWarps;
-
-// ------------------------------------------------------------------------------------------------------
-// dQ
-// ------------------------------------------------------------------------------------------------------
-constexpr int kDqBufs = 3;     // (S^T, dP^T) accumulator pairs in flight: 3 x 128 columns, dQ^T behind them
-// A K pair stays in shared memory from its score MMA until its dQ MMA, i.e. across the whole elementwise
-// stage plus a ~2000-cycle reload; with two stages that chain was the throughput limit, so K gets three
-// (V is released right after dP^T and keeps two; dS^T makes do with one buffer to pay for it).
-constexpr int kDqKStages = 3;
-struct DqSmem {
-  static constexpr uint32_t q = 0;                                // 16 KB
-  static constexpr uint32_t d_o = q + 2 * kSlab;                  // 16 KB
-  static constexpr uint32_t k = d_o + 2 * kSlab;                  // 3 x 32 KB
-  static constexpr uint32_t v = k + kDqKStages * kPairBytes;      // 2 x 32 KB
-  static constexpr uint32_t ds = v + 2 * kPairBytes;              // 1 x 16 KB
-  static constexpr uint32_t tile_row = ds + kPairHalf;            // int32 [kMaxTiles]
-  static constexpr uint32_t tile_valid = tile_row + 4 * kMaxTiles;
-  static constexpr uint32_t lse = tile_valid + kMaxTiles;         // float [64]
-  static constexpr uint32_t delta = lse + 256;                    // float [64]
-  static constexpr uint32_t bars = delta + 256;
-  static constexpr uint32_t misc = bars + 32 * 8;
-  static constexpr uint32_t total = misc + 64;
-};
-enum DqBar { DQ_QDO_FULL = 0, DQ_K_FULL = 1, DQ_K_EMPTY = 4, DQ_V_FULL = 7, DQ_V_EMPTY = 9, DQ_DS_FULL = 11,
-             DQ_DS_EMPTY = 12, DQ_ACC_FULL = 13, DQ_S_FULL = 14, DQ_S_EMPTY = 14 + kDqBufs,
-             DQ_DP_FULL = 14 + 2 * kDqBufs };
-
-template <int SUB>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-sparse_dq_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
-                      const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                      const elem_t* __restrict__ dout, const elem_t* __restrict__ out_s, const float* __restrict__ lse2,
-                      const int32_t* __restrict__ selected, const int32_t* __restrict__ kv_sizes,
-                      float* __restrict__ delta, elem_t* __restrict__ dq, const elem_t* __restrict__ mean_grad,
-                      const int32_t* __restrict__ q_sizes, long long Lq, long long Lkv, long long kv_shard, int topk,
-                      float scale, RasterMap out_map) {
-  extern __shared__ uint8_t smem_raw[];
-  if (*(volatile int*)&g_device_status != 0) return;
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qtile = blockIdx.x;
-  const long long bh = blockIdx.y;
-  const int Qb = (int)(Lq / (kTile * SUB));
-  const int qb = qtile / SUB;
-  const int32_t* sel = selected + (bh * Qb + qb) * (long long)topk;
-  const int n_iter = topk * SUB;
-  const float c = scale * kLog2e;
-  const long long qrow0 = bh * Lq + (long long)qtile * kTile;
-
-  int32_t* tile_row = reinterpret_cast<int32_t*>(sm + DqSmem::tile_row);
-  uint8_t* tile_valid = sm + DqSmem::tile_valid;
-  float* s_lse = reinterpret_cast<float*>(sm + DqSmem::lse);
-  float* s_delta = reinterpret_cast<float*>(sm + DqSmem::delta);
-  volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(sm + DqSmem::misc);
-  auto bar = [&](int i) -> uint32_t { return base + DqSmem::bars + 8u * i; };
-
-  if (tid == 0) {
-    mbar_init(bar(DQ_QDO_FULL), 1);
-    for (int i = 0; i < kDqKStages; ++i) {
-      mbar_init(bar(DQ_K_FULL + i), 4);
-      mbar_init(bar(DQ_K_EMPTY + i), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(DQ_V_FULL + i), 4);
-      mbar_init(bar(DQ_V_EMPTY + i), 1);
-    }
-    mbar_init(bar(DQ_DS_FULL), kBwWarps);
-    mbar_init(bar(DQ_DS_EMPTY), 1);
-    for (int i = 0; i < kDqBufs; ++i) {
-      mbar_init(bar(DQ_S_FULL + i), 1);
-      mbar_init(bar(DQ_DP_FULL + i), 1);
-      mbar_init(bar(DQ_S_EMPTY + i), kBwWarps);
-    }
-    mbar_init(bar(DQ_ACC_FULL), 1);
-    fence_barrier_init();
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    // Q and dO of this tile depend on nothing the prologue computes: their loads fly under the tile-list build and delta
-    mbar_arrive_expect_tx(bar(DQ_QDO_FULL), 4 * kSlab);
-    tma_load_2d(base + DqSmem::q, &map_q, 0, (int)qrow0, bar(DQ_QDO_FULL));
-    tma_load_2d(base + DqSmem::q + kSlab, &map_q, 64, (int)qrow0, bar(DQ_QDO_FULL));
-    tma_load_2d(base + DqSmem::d_o, &map_do, 0, (int)qrow0, bar(DQ_QDO_FULL));
-    tma_load_2d(base + DqSmem::d_o + kSlab, &map_do, 64, (int)qrow0, bar(DQ_QDO_FULL));
-  }
-  for (int it = tid; it < n_iter; it += kBwdThreads) {
-    const int kvb = sel[it / SUB];
-    // an id outside the table is an empty tile, as route inversion treats it
-    const int left = (unsigned)kvb < (unsigned)(Lkv / (kTile * SUB)) ? kv_sizes[kvb] - (it % SUB) * kTile : 0;
-    tile_valid[it] = (uint8_t)(left < 0 ? 0 : (left > kTile ? kTile : left));
-    tile_row[it] = left > 0 ? (int)kv_tensor_row(bh, gridDim.y, (long long)kvb * (kTile * SUB) + (it % SUB) * kTile, kv_shard) : 0;
-  }
-  if (warp >= 4 && warp < kDpWarp) {   // delta = rowsum(out_s * dout) and the saved statistic, eight threads per query row
-    constexpr int kPer = kBwEwThreads / 64;            // threads per row
-    constexpr int kDims = kD / kPer;                 // dims per thread
-    const int st = tid - 128;
-    const int row = st / kPer, part = st % kPer;
-    const uint4* po = reinterpret_cast<const uint4*>(out_s + (qrow0 + row) * kD + part * kDims);
-    const uint4* pd = reinterpret_cast<const uint4*>(dout + (qrow0 + row) * kD + part * kDims);
-    float acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < kDims / 8; ++i) {
-      const uint4 a = po[i], b = pd[i];
-      const elem_t* ea = reinterpret_cast<const elem_t*>(&a);
-      const elem_t* eb = reinterpret_cast<const elem_t*>(&b);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc = fmaf(Elem<elem_t>::to(ea[j]), Elem<elem_t>::to(eb[j]), acc);
-    }
-#pragma unroll
-    for (int o = 1; o < kPer; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (part == 0) {
-      s_delta[row] = -acc;
-      delta[qrow0 + row] = acc;
-      s_lse[row] = log2f(fabsf(scale)) - lse2[qrow0 + row];   // 2^(s c - lse) * |scale| in one exponential
-    }
-  }
-  __syncthreads();
-  if (warp == 2) {
-    int n_live = 0;
-    for (int it0 = 0; it0 < n_iter; it0 += 32) {
-      const int it = it0 + lane;
-      const int valid = it < n_iter ? (int)tile_valid[it] : 0;
-      const int row = it < n_iter ? tile_row[it] : 0;
-      const unsigned live = __ballot_sync(0xffffffffu, valid > 0);
-      __syncwarp();
-      if (valid > 0) {
-        const int pos = n_live + __popc(live & ((1u << lane) - 1u));
-        tile_row[pos] = row;
-        tile_valid[pos] = (uint8_t)valid;
-      }
-      n_live += __popc(live);
-      __syncwarp();
-    }
-    if (lane == 0) misc[1] = (uint32_t)n_live;
-  }
-  if (warp == 1) {
-    tmem_alloc(base + DqSmem::misc, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = misc[0];
-  const int n_live = (int)misc[1];
-  const int n_pairs = (n_live + 1) >> 1;
-  const uint32_t tmem_acc = tmem + 128 * kDqBufs;
-  bool ok = true;
-
-  if (warp == 0 || warp == 1) {
-    const bool is_k = warp == 0;
-    const int which = lane & 1, dhalf = (lane >> 1) & 1;
-    const CUtensorMap* map = is_k ? &map_k : &map_v;
-    const int full0 = is_k ? DQ_K_FULL : DQ_V_FULL, empty0 = is_k ? DQ_K_EMPTY : DQ_V_EMPTY;
-    const uint32_t ring = base + (is_k ? DqSmem::k : DqSmem::v);
-    const int depth = is_k ? kDqKStages : 2;
-    for (int p = 0; p < n_pairs; ++p) {
-      const int s = p % depth;
-      const uint32_t ph = (p / depth) & 1;
-      int idx = 2 * p + which;
-      if (idx >= n_live) idx = 2 * p;
-      const int row = tile_row[idx];                          // row of the tile in the K/V tensors
-      ok = VSA_WARP_WAIT(bar(empty0 + s), ph ^ 1);
-      if (!ok) break;
-      if (lane < 4) {
-        mbar_arrive_expect_tx(bar(full0 + s), kSlab);
-        tma_load_2d(ring + s * kPairBytes + dhalf * kPairHalf + which * kSlab, map, dhalf * 64, row, bar(full0 + s));
-      }
-    }
-    if (!ok && lane == 0) report_timeout(11);
-  } else if (warp == 2) {
-    if (lane == 0) {   // scores: S^T = K2 Q^T
-      ok = VSA_WAIT(bar(DQ_QDO_FULL), 0);
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int ks = p % kDqKStages, b = p % kDqBufs;
-        ok = VSA_WAIT(bar(DQ_K_FULL + ks), (p / kDqKStages) & 1) &&
-             VSA_WAIT(bar(DQ_S_EMPTY + b), ((p / kDqBufs) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
-        // S^T is signalled on its own: the elementwise warps turn it into 2^(S c - lse) while dP^T still runs
-        issue_kmajor(tmem + b * 128, base + DqSmem::k + ks * kPairBytes, base + DqSmem::q);
-        mma_commit(bar(DQ_S_FULL + b));
-      }
-      if (!ok) report_timeout(12);
-    }
-  } else if (warp == kDpWarp) {
-    if (lane == 0) {   // dP^T = V2 dO^T from a thread of its own: a late V pair must not hold back the next S^T
-      ok = VSA_WAIT(bar(DQ_QDO_FULL), 0);
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int s = p & 1, b = p % kDqBufs;
-        ok = VSA_WAIT(bar(DQ_V_FULL + s), (p >> 1) & 1) && VSA_WAIT(bar(DQ_S_EMPTY + b), ((p / kDqBufs) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
-        issue_kmajor(tmem + b * 128 + 64, base + DqSmem::v + s * kPairBytes, base + DqSmem::d_o);
-        mma_commit(bar(DQ_V_EMPTY + s));
-        mma_commit(bar(DQ_DP_FULL + b));
-      }
-      if (!ok) report_timeout(16);
-    }
-  } else if (warp == 3) {
-    if (lane == 0) {   // dQ^T += K2^T dS^T
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int ks = p % kDqKStages;
-        ok = VSA_WAIT(bar(DQ_K_FULL + ks), (p / kDqKStages) & 1) && VSA_WAIT(bar(DQ_DS_FULL), p & 1);
-        if (!ok) break;
-        tc_fence_after();
-        issue_mnmajor(tmem_acc, base + DqSmem::k + ks * kPairBytes, base + DqSmem::ds, p > 0);
-        mma_commit(bar(DQ_K_EMPTY + ks));
-        mma_commit(bar(DQ_DS_EMPTY));
-      }
-      if (ok) mma_commit(bar(DQ_ACC_FULL));
-      if (!ok) report_timeout(13);
-    }
-  } else {
-    // elementwise warps: lane t = key token of the pair, kBwCols of the 64 query rows (columns c0..)
-    const float2 c2 = make_float2(c, c);     // two fp32 operations per instruction: dQ -1 %, dK/dV -2 % at 180 routes
-    const int quarter = warp & 3;
-    const int cg = (warp - 4) >> 2;
-    const int c0 = cg * kBwCols;
-    const int t = quarter * 32 + lane;
-    const int half = t >> 6, r = t & 63;
-    const int st = tid - 128;
-    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    for (int p = 0; p < n_pairs && ok; ++p) {
-      const int b = p % kDqBufs;
-      const int idx = 2 * p + half;
-      const int valid = idx < n_live ? (int)tile_valid[idx] : 0;
-      const bool live = r < valid;
-      ok = VSA_WARP_WAIT(bar(DQ_S_FULL + b), (p / kDqBufs) & 1);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t sv[kBwCols];
-      tmem_ld(tmem + b * 128 + lane_addr + c0, sv);
-      tmem_ld_wait();
-      // rows of K beyond a ragged tile's size (and the repeated tile of an odd tail) must be finite zeros:
-      // they meet dS = 0 in the dQ product, where 0 * NaN would poison the sum.  S(p) has completed.
-      if (!live && cg == 0) {
-        uint8_t* krow = sm + DqSmem::k + (p % kDqKStages) * kPairBytes + t * 128;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          *reinterpret_cast<uint4*>(krow + ch * 16) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(krow + kPairHalf + ch * 16) = make_uint4(0, 0, 0, 0);
-        }
-      }
-      float2 pf[kBwCols / 2]; // 2^(S c - lse) * |scale|
-#pragma unroll
-      for (int j4 = 0; j4 < kBwCols / 4; ++j4) {
-        const float4 l4 = *reinterpret_cast<const float4*>(s_lse + c0 + 4 * j4);
-        const float2 x = fma2(word_pair(sv + 4 * j4), c2, make_float2(l4.x, l4.y));
-        const float2 y = fma2(word_pair(sv + 4 * j4 + 2), c2, make_float2(l4.z, l4.w));
-        pf[2 * j4] = make_float2(fast_exp2(x.x), fast_exp2(x.y));
-        pf[2 * j4 + 1] = make_float2(fast_exp2(y.x), fast_exp2(y.y));
-      }
-      bool ds_free;
-      ok = VSA_WARP_WAIT_TEST(bar(DQ_DP_FULL + b), (p / kDqBufs) & 1, bar(DQ_DS_EMPTY), (p & 1) ^ 1, &ds_free);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t dv[kBwCols];
-      tmem_ld(tmem + b * 128 + 64 + lane_addr + c0, dv);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(DQ_S_EMPTY + b));      // both accumulators of this buffer have been read
-      uint32_t packed[kBwCols / 2];
-#pragma unroll
-      for (int j4 = 0; j4 < kBwCols / 4; ++j4) {
-        const float4 d4 = *reinterpret_cast<const float4*>(s_delta + c0 + 4 * j4);
-        const float2 x = mul2(pf[2 * j4], add2(word_pair(dv + 4 * j4), make_float2(d4.x, d4.y)));
-        const float2 y = mul2(pf[2 * j4 + 1], add2(word_pair(dv + 4 * j4 + 2), make_float2(d4.z, d4.w)));
-        packed[2 * j4] = Elem<elem_t>::pack(x.x, x.y);
-        packed[2 * j4 + 1] = Elem<elem_t>::pack(y.x, y.y);
-      }
-      if (!live) {   // a padding key row: its scores come from whatever sits in K and V there
-#pragma unroll
-        for (int j = 0; j < kBwCols / 2; ++j) packed[j] = 0u;
-      }
-      if (!ds_free) ok = VSA_WARP_WAIT(bar(DQ_DS_EMPTY), (p & 1) ^ 1);
-      if (!ok) break;
-      uint8_t* drow = sm + DqSmem::ds + t * 128;
-#pragma unroll
-      for (int ch = 0; ch < kBwCols / 8; ++ch)
-        *reinterpret_cast<uint4*>(drow + ((((kBwCols / 8) * cg + ch) ^ (t & 7)) << 4)) =
-            make_uint4(packed[4 * ch], packed[4 * ch + 1], packed[4 * ch + 2], packed[4 * ch + 3]);
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(DQ_DS_FULL));
-    }
-    if (!ok && lane == 0) report_timeout(14);
-    if (ok && n_pairs > 0) ok = VSA_WARP_WAIT(bar(DQ_ACC_FULL), 0);
-    if (!ok && lane == 0) report_timeout(15);
-    tc_fence_after();
-    elem_t* stage = reinterpret_cast<elem_t*>(sm + DqSmem::k);      // [64 query rows][128 dims]; every MMA is done
-    // block-mean backward folded in (optional): query row r of the block also receives dmean[block] / max(size, 1)
-    // while r < size (vsa/fused_common.py:62-103 of the reference); here lane t is the head dim, a column a row
-    float gm = 0.f;
-    int rows_live = 0;
-    if (mean_grad != nullptr) {
-      const int size = q_sizes[qb];
-      gm = Elem<elem_t>::to(mean_grad[(bh * Qb + qb) * (long long)kD + t]) / (float)(size > 1 ? size : 1);
-      rows_live = size - (qtile % SUB) * kTile;
-    }
-    if (ok && n_pairs > 0) {
-      uint32_t av[kBwCols];
-      tmem_ld(tmem_acc + lane_addr + c0, av);
-      tmem_ld_wait();
-      const uint32_t sign = scale < 0.f ? 0x80000000u : 0u;
-#pragma unroll
-      for (int j = 0; j < kBwCols; ++j)
-        stage[(c0 + j) * kD + t] = Elem<elem_t>::from(__uint_as_float(av[j] ^ sign) + ((c0 + j) < rows_live ? gm : 0.f));
-    } else {
-      for (int j = 0; j < kBwCols; ++j) stage[(c0 + j) * kD + t] = Elem<elem_t>::from((c0 + j) < rows_live ? gm : 0.f);
-    }
-    named_barrier(1, kBwEwThreads);
-#pragma unroll
-    for (int i = 0; i < 1024 / kBwEwThreads; ++i) {
-      const int cidx = st + kBwEwThreads * i;
-      const int row = cidx >> 4, ch = cidx & 15;
-      // with a raster map the gradient row goes straight to the token's raster row (padding rows have none)
-      const long long drow = out_map.map == nullptr ? qrow0 + row : raster_row(out_map, bh, (long long)qtile * kTile + row);
-      if (drow >= 0)
-        *reinterpret_cast<uint4*>(dq + drow * kD + ch * 8) = *reinterpret_cast<const uint4*>(stage + row * kD + ch * 8);
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem, kTmemCols);
-}
 
 // ------------------------------------------------------------------------------------------------------
 // dK / dV
@@ -382,8 +44,8 @@ enum DkBar { DK_KV_FULL = 0, DK_Q_FULL = 1, DK_DO_FULL = 4, DK_Q_EMPTY = 6, DK_D
              DK_P_EMPTY = 12, DK_DS_FULL = 13, DK_DS_EMPTY = 14, DK_ACC_FULL = 15, DK_S_FULL = 16,
              DK_DP_FULL = 16 + kDkBufs, DK_S_EMPTY = 16 + 2 * kDkBufs };
 
-// DS = true: the rows of `inverse` hold packed edges (query block << kEdgeSlotBits | slot in that block's route)
-// and every dS tile (64 query rows x 64 key tokens, 8 KB) is also written to `ds_ws` at tile index
+// The rows of `inverse` hold packed edges (query block << kEdgeSlotBits | slot in that block's route)
+// and every dS tile (64 query rows x 64 key tokens, 8 KB) is written to `ds_ws` at tile index
 // ((edge * SUB + query sub-tile) * SUB + key sub-tile), edge = (slice * Qb + query block) * topk + slot, for the
 // dQ pass that only multiplies it by K (sparse_dq_from_ds_kernel below) instead of recomputing S and dP.
 // Layout of a stored tile: [8 chunks of 8 key tokens][64 query rows][16 bytes] -- the order in which the rows'
@@ -391,9 +53,9 @@ enum DkBar { DK_KV_FULL = 0, DK_Q_FULL = 1, DK_DO_FULL = 4, DK_Q_EMPTY = 6, DK_D
 // from registers), and at the same time the un-swizzled K-major operand layout of tcgen05 (8 rows x 16 bytes per
 // core matrix), so the dQ pass copies the 8 KB verbatim into shared memory and multiplies.
 constexpr int kEdgeSlotBits = 11;
-template <int SUB, bool DS>
+template <int SUB>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
+sparse_dkdv_ds_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                         const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         const float* __restrict__ lse2, const float* __restrict__ delta,
                         const int32_t* __restrict__ counts, const int32_t* __restrict__ offsets,
@@ -405,7 +67,7 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   if (*(volatile int*)&g_device_status != 0) return;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int ktile = blockIdx.x;
   const long long bh = blockIdx.y;
   const int Kb = (int)(Lkv / (kTile * SUB)), Qb = (int)(Lq / (kTile * SUB));
@@ -448,9 +110,9 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   // row (inside this batch-head slice) of the i-th query tile that selected this key block
   auto tile_row = [&](int i) -> int {
     const int e = inv[i / SUB];
-    return (DS ? (e >> kEdgeSlotBits) : e) * (kTile * SUB) + (i % SUB) * kTile;
+    return (e >> kEdgeSlotBits) * (kTile * SUB) + (i % SUB) * kTile;
   };
-  // index of the dS tile of the i-th in-edge query tile (DS only)
+  // index of the dS tile of the i-th in-edge query tile
   auto ds_tile = [&](int i) -> long long {
     const int e = inv[i / SUB];
     const long long edge = (bh * Qb + (e >> kEdgeSlotBits)) * (long long)topk + (e & ((1 << kEdgeSlotBits) - 1));
@@ -520,54 +182,64 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     }
     if (!ok && lane == 0) report_timeout(21);
   } else if (warp == 2) {
-    if (lane == 0) {   // scores: S = Q2 K^T
-      ok = VSA_WAIT(bar(DK_KV_FULL), 0);
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int qs = p % kDkQStages, b = p % kDkBufs;
-        ok = VSA_WAIT(bar(DK_Q_FULL + qs), (p / kDkQStages) & 1) &&
-             VSA_WAIT(bar(DK_S_EMPTY + b), ((p / kDkBufs) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // scores: S = Q2 K^T
+    ok = VSA_WARP_WAIT(bar(DK_KV_FULL), 0);
+    for (int p = 0; p < n_pairs && ok; ++p) {
+      const int qs = p % kDkQStages, b = p % kDkBufs;
+      ok = VSA_WARP_WAIT(bar(DK_Q_FULL + qs), (p / kDkQStages) & 1) &&
+           VSA_WARP_WAIT(bar(DK_S_EMPTY + b), ((p / kDkBufs) & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         issue_kmajor(tmem + b * 128, base + DkSmem::q + qs * kPairBytes, base + DkSmem::k);
         mma_commit(bar(DK_S_FULL + b));
       }
-      if (!ok) report_timeout(22);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(22);
   } else if (warp == kDpWarp) {
-    if (lane == 0) {   // dP = dO2 V^T from a thread of its own: dO2 has two stages only and must not hold back the next S
-      ok = VSA_WAIT(bar(DK_KV_FULL), 0);
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int s = p & 1, b = p % kDkBufs;
-        ok = VSA_WAIT(bar(DK_DO_FULL + s), (p >> 1) & 1) && VSA_WAIT(bar(DK_S_EMPTY + b), ((p / kDkBufs) & 1) ^ 1);
-        if (!ok) break;
-        tc_fence_after();
+    // dP = dO2 V^T from a thread of its own: dO2 has two stages only and must not hold back the next S
+    ok = VSA_WARP_WAIT(bar(DK_KV_FULL), 0);
+    for (int p = 0; p < n_pairs && ok; ++p) {
+      const int s = p & 1, b = p % kDkBufs;
+      ok = VSA_WARP_WAIT(bar(DK_DO_FULL + s), (p >> 1) & 1) && VSA_WARP_WAIT(bar(DK_S_EMPTY + b), ((p / kDkBufs) & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         issue_kmajor(tmem + b * 128 + 64, base + DkSmem::d_o + s * kPairBytes, base + DkSmem::v);
         mma_commit(bar(DK_DP_FULL + b));
         mma_commit(bar(DK_DO_EMPTY + s));      // a commit covers the MMAs of the committing thread only: dP here, dV^T there
       }
-      if (!ok) report_timeout(26);
+      __syncwarp();
     }
+    if (!ok && lane == 0) report_timeout(26);
   } else if (warp == 3) {
-    if (lane == 0) {   // dV^T += dO2^T P and dK^T += Q2^T dS
-      for (int p = 0; p < n_pairs && ok; ++p) {
-        const int qs = p % kDkQStages, s = p & 1;
-        const uint32_t ph = (p >> 1) & 1;
-        ok = VSA_WAIT(bar(DK_DO_FULL + s), ph) && VSA_WAIT(bar(DK_P_FULL), p & 1);
-        if (!ok) break;
-        tc_fence_after();
+    // dV^T += dO2^T P and dK^T += Q2^T dS
+    for (int p = 0; p < n_pairs && ok; ++p) {
+      const int qs = p % kDkQStages, s = p & 1;
+      const uint32_t ph = (p >> 1) & 1;
+      ok = VSA_WARP_WAIT(bar(DK_DO_FULL + s), ph) && VSA_WARP_WAIT(bar(DK_P_FULL), p & 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         issue_mnmajor(tmem_dv, base + DkSmem::d_o + s * kPairBytes, base + DkSmem::p, p > 0);
         mma_commit(bar(DK_P_EMPTY));
         mma_commit(bar(DK_DO_EMPTY + s));      // second of two arrivals: the other issuer commits its dP reads of the stage
-        ok = VSA_WAIT(bar(DK_Q_FULL + qs), (p / kDkQStages) & 1) && VSA_WAIT(bar(DK_DS_FULL), p & 1);
-        if (!ok) break;
-        tc_fence_after();
+      }
+      __syncwarp();
+      ok = VSA_WARP_WAIT(bar(DK_Q_FULL + qs), (p / kDkQStages) & 1) && VSA_WARP_WAIT(bar(DK_DS_FULL), p & 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
         issue_mnmajor(tmem_dk, base + DkSmem::q + qs * kPairBytes, base + DkSmem::ds, p > 0);
         mma_commit(bar(DK_Q_EMPTY + qs));
         mma_commit(bar(DK_DS_EMPTY));
       }
-      if (ok) mma_commit(bar(DK_ACC_FULL));
-      if (!ok) report_timeout(23);
+      __syncwarp();
     }
+    if (ok && elect_one()) mma_commit(bar(DK_ACC_FULL));
+    __syncwarp();
+    if (!ok && lane == 0) report_timeout(23);
   } else {
     // elementwise warps: lane t = query row of the pair, kBwCols of the 64 key tokens (columns c0..)
     const float2 c2 = make_float2(c, c);
@@ -582,12 +254,12 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // statistics of this lane's query row, fetched one pair ahead of their use.  A row that does not exist (the
     // repeated tile of an odd tail) gets lse = +inf, i.e. P = 0 exactly, and delta = 0, so dS = 0 * finite = 0.
     float lse_n = INFINITY, dl_n = 0.f;
-    long long dst_n = -1;                    // DS: tile index of this lane's dS row in the coming pair
+    long long dst_n = -1;                    // tile index of this lane's dS row in the coming pair
     if (half < n_tiles) {
       const long long row = q_row_base + tile_row(half) + r;
       lse_n = lse2[row];
       dl_n = delta[row];
-      if (DS) dst_n = ds_tile(half);
+      dst_n = ds_tile(half);
     }
     uint8_t* prow = sm + DkSmem::p + t * 128;
     uint8_t* grow = sm + DkSmem::ds + t * 128;
@@ -604,7 +276,7 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           const long long row = q_row_base + tile_row(nidx) + r;
           lse_n = lse2[row];
           dl_n = delta[row];
-          if (DS) dst_n = ds_tile(nidx);
+          dst_n = ds_tile(nidx);
         }
       }
       // ---- P from S, published before dP is even looked at (the dP MMAs are still running)
@@ -663,7 +335,7 @@ sparse_dkdv_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           pg[j2] = Elem<elem_t>::pack(g0, g1);
         }
       }
-      if (DS && dst >= 0) {   // chunk-major tile: chunk c of row r at c * 1024 + r * 16 bytes
+      if (dst >= 0) {   // chunk-major tile: chunk c of row r at c * 1024 + r * 16 bytes
         uint4* g = reinterpret_cast<uint4*>(ds_ws + dst * (kTile * kTile)) + ((kBwCols / 8) * cg) * kTile + r;
 #pragma unroll
         for (int ch = 0; ch < kBwCols / 8; ++ch)

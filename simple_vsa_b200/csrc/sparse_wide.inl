@@ -1,26 +1,25 @@
 // Fine attention for block volumes that are multiples of 128 tokens (128 and 256), forward and backward, on the
 // Blackwell tensor path.  Included by sparse_umma_typed.inl, once per 16-bit element type.
 //
-// The 64-token kernels compute transposed products with N = 64, whose operands cost 48 cycles of shared-memory reads
-// per 32 cycles of tensor work.  128 consecutive tokens of a block share one route, so here the CTA owns 128 rows and
-// they are the M dimension themselves: the resident tile (Q; Q and dO; K and V) is the A operand, the streamed tile
-// the B operand, and P / dS never touch shared memory -- the thread that owns a row (a TMEM lane) packs them over the
-// fp32 scores it has just read, and the second product takes them from tensor memory as its A operand:
+// 128 consecutive tokens of a block share one route, so the CTA owns 128 rows and they are the M dimension themselves: half the
+// streamed bytes of 64-row tiles per score, 64 cycles of tensor work per M128 x N128 x K16, nothing to add in the epilogue.  The
+// resident tile (Q; Q and dO; K and V) is the A operand, the streamed tile the B operand, and P / dS never touch shared memory --
+// the thread that owns a row (a TMEM lane) packs them over the fp32 scores it has just read, and the second product takes them
+// from tensor memory as its A operand:
 //   forward  S[128 q x 128 k]  = Q K^T                             O[128 q x D]  += P V
 //   dQ       S = Q K^T,  dP = dO V^T  (128 q x 128 k)              dQ[128 q x D] += dS K
 //   dK/dV    S^T = K Q^T, dP^T = V dO^T  (128 k x 64 q)            dV[128 k x D] += P^T dO,  dK += dS^T Q
-// Shared-memory bytes per 128 x 128 scores at D = 128 (128 B/clk): forward 160 KB (was 352), dQ 224 (448), dK/dV 320
-// (576); tensor work 1024 / 1536 / 2560 cycles; exponentials 1024 cycles (16 per clock and SM) in every pass.
+// Shared-memory bytes per 128 x 128 scores at D = 128 (128 B/clk): forward 160 KB, dQ 224, dK/dV 320; tensor work 1024 / 1536 / 2560
+// cycles; exponentials 1024 cycles (16 per clock and SM) in every pass.
 //
-// Measured before (four or two 64-token tiles per block row, mma.sync at D = 64) -> now, ms for forward / dQ / dK/dV:
-//   [1, 8, 92160, 128], blocks of 128, topk 90:   5.77 / 8.11 / 9.69  -> 3.55 / 5.80 / 7.13   (1225 / 1125 / 1220 TFLOP/s)
-//   [1, 10, 40960, 128], blocks of 256, topk 20:  1.71 / 2.10 / 2.51  -> 0.99 / 1.44 / 1.79
-//   [1, 12, 16384, 64], blocks of 128, topk 16:   0.41 / 0.50 / 0.70  -> 0.26 / 0.32 / 0.37
-// What bounds them now: no single pipe (ncu on [1, 2, 46080, 128]: tensor 54 / 60 / 66 %, exponentials 57 / 41 / 34 %) but the
-// chain product -> elementwise -> product of a tile, of which three (forward) and two (backward) are in flight; at 92k
-// tokens the backward is within 20 % of what a long cuBLAS GEMM sustains under the board's power limit.
+// Measured, ms for forward / dQ / dK/dV: with transposed 64-token tiles (mma.sync at D = 64) -> these kernels -> whole-warp waits
+// and MMAs under elect.sync:
+//   [1, 8, 92160, 128], blocks of 128, topk 90:   5.77 / 8.11 / 9.69  -> 3.55 / 5.80 / 7.13 -> 3.37 / 5.20 / 6.92
+//   [1, 12, 16384, 128], blocks of 128, topk 16:                         0.277 / 0.387 / 0.381 -> 0.259 / 0.287 / 0.351
+// What bounds them: the chain product -> elementwise -> product of a tile, of which three (forward) and two (backward) are in
+// flight; at 92k tokens the backward is within 10 % of what a long cuBLAS GEMM sustains under the board's power limit.
 //
-// The softmax shift of the forward is the row maximum over the first live key tile, as in the 64-token kernels (a row
+// The softmax shift of the forward is the row maximum over the first live key tile, as in the 64-row kernels (a row
 // is one thread here, so it needs no exchange between lanes); rows that leave the finite range are marked the same
 // way, 64 rows at a time, for the exact kernel.
 constexpr int kWRows = 128;                       // rows of a wide tile
