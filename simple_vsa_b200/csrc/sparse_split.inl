@@ -393,18 +393,18 @@ sparse_fwd_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       };
       if (valid == kTile) exponentiate(std::false_type{});
       else exponentiate(std::true_type{});
+      ok = VSA_WARP_WAIT(bar(SF_P_EMPTY), (p & 1) ^ 1);
+      if (!ok) break;
+      tc_fence_after();
       if (valid < kTile && idx < n_live) {
-        // padding rows of V meet P = 0 in the product: they must be finite (0 * NaN).  V of this pair may be under way still, so
-        // its rows come after the exponentials
+        // Padding rows of V meet P = 0 in the product: they must be finite (0 * NaN).  Not before P V of the last pair has completed:
+        // only then has the part's slot been filled for every earlier pair, so that this parity can mean nothing but this pair.
         const int i = p * kParts + r / kVRows, s = i % kSfStages;
         ok = VSA_WARP_WAIT(bar(SF_V_FULL + s), (i / kSfStages) & 1);
         if (!ok) break;
         if (r >= valid) split_zero_row<HD>(sm + Sm::v + s * Sm::part + half * (Sm::part / 2) + (r % kVRows) * 128, r, kVRows * 128);
         fence_proxy_async_smem();
       }
-      ok = VSA_WARP_WAIT(bar(SF_P_EMPTY), (p & 1) ^ 1);
-      if (!ok) break;
-      tc_fence_after();
       tmem_st(tmem_p + lane_addr, pk[0]);
       tmem_st(tmem_p + lane_addr + 16, pk[1]);
       if (kSplitP) {

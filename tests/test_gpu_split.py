@@ -70,3 +70,25 @@ def test_a_tile_outside_the_shift_range_is_recomputed_exactly(D, dtype, k_factor
     assert _lib.device_status() == 0
     torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=2e-2)
     torch.testing.assert_close(lse.float().cpu(), want_lse.float(), atol=5e-2, rtol=1e-3)
+
+
+@pytest.mark.parametrize("D,tk", [(128, 40), (64, 40)])
+def test_many_ragged_tiles_leave_their_neighbours_alone(D, tk, monkeypatch):
+    """Half the blocks ragged, two CTAs on every SM, twenty pairs each: clearing the padding rows of one pair must not reach the rows
+    of the pair before it, whatever the timing.  Against the warp-level kernels: two roundings of values around 1 in bf16 apart."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator(device=DEV).manual_seed(D)
+    be, H, nb = 64, 8, 200
+    q, k, v = (torch.randn(1, H, nb * be, D, device=DEV, generator=g).to(torch.bfloat16) for _ in range(3))
+    sizes = torch.randint(1, 2 * be, (nb,), device=DEV, generator=g, dtype=torch.int32).clamp(max=be)
+    selected = torch.rand(1, H, nb, nb, device=DEV, generator=g).topk(tk, dim=-1).indices.to(torch.int32)
+    outs = {}
+    for mode in ("auto", "mma"):
+        monkeypatch.setenv("VSA_B200_KERNELS", mode)
+        outs[mode] = [ops.sparse_forward(q, k, v, selected, sizes, be, D ** -0.5, True)[0] for _ in range(5)]
+    assert _lib.device_status() == 0
+    want = outs["mma"][0].float()
+    for out in outs["auto"]:
+        assert torch.equal(out, outs["auto"][0])
+        # P carries 2^-9 and the output 2^-9 of values below 1/2: a cleared row of V would show as one of ~1500 weights, times |v|
+        assert (out.float() - want).abs().max() < 4e-3
