@@ -278,28 +278,30 @@ static bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, i
 }
 // Head dim 64 on 64-row tiles: tcgen05 (sparse_split.inl) or mma.sync, of which three or four CTAs share an SM and need little set-up,
 // so that they are faster while a route holds few tiles.  us, tcgen05 / mma.sync, by tiles per route:
-//   [1, 12, 16384, 64]  forward 4: 97 / 60, 8: 113 / 103, 16: 144 / 190, 32: 206 / 364;  dQ 4: 141 / 86, 8: 162 / 142, 16: 206 / 255, 32: 291 / 482;
+//   [1, 12, 16384, 64]  forward 4: 97 / 60, 8: 113 / 103, 12: 133 / 146, 16: 150 / 190, 32: 215 / 364;
+//                       dQ 4: 141 / 86, 8: 162 / 142, 12: 185 / 199, 16: 206 / 256, 32: 292 / 483;
 //                       dK/dV 4: 151 / 118, 8: 187 / 195, 16: 257 / 349, 32: 394 / 652
-//   [1, 2, 2048, 64], all tiles on the SMs at once: forward 2: 8.4 / 4.8, 8: 10.6 / 11.5;  dQ 2: 6.7 / 7.1, 8: 8.5 / 14.7;  dK/dV 2: 8.0 / 13.5, 8: 11.5 / 23.6
+//   [1, 2, 2048, 64], all tiles on the SMs at once: forward 2: 8.4 / 4.8, 6: 10.5 / 9.6, 8: 10.6 / 11.5, 12: 11.8 / 15.8;
+//                       dQ 2: 6.7 / 7.1, 6: 7.9 / 12.6, 12: 9.3 / 19.6;  dK/dV 2: 8.0 / 13.5, 6: 11.1 / 22.4, 12: 13.3 / 27.3
 bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
   const int64_t n = (int64_t)topk * (be / kTile);
   const bool one_wave = BH * (L / kTile) <= sm_count();
-  if (pass == kPassForward) return n > (one_wave ? 4 : 8);
+  if (pass == kPassForward) return n > (one_wave ? 6 : 8);
   return one_wave || n > (pass == kPassDq ? 8 : 6);
 }
 
-// Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as tiles of 64 tokens.  Both
-// run one CTA per SM; a 128-row CTA does twice the rows in less than twice the time, so the 64-token kernels are the faster
-// ones where halving the CTAs saves no wave (times on one B200, head dim 128, full blocks, us, 64-token / 128-row):
-//   all 64-row tiles on the SMs at once ([1, 2, 4096], 2 / 8 / 32 tiles a route): forward 12.7 / 14.0, 15.2 / 16.3, 24.2 / 26.3;
-//     dQ 8.7 / 15.8, 11.7 / 19.8, 24.4 / 35.0; dK/dV 13.1 / 16.4, 18.0 / 22.4, 33.5 / 42.3;
-//   three waves against two ([1, 3, 8192]): forward 24.5 / 25.0, 31.3 / 30.1, 59.4 / 49.9; dQ 22.9 / 30.2, 31.7 / 38.0,
-//     68.3 / 67.8; dK/dV 20.9 / 17.6, 37.2 / 34.8, 86.2 / 77.5;
-//   many waves ([1, 12, 16384]): forward 139 / 140, 185 / 168, 383 / 276; dQ 175 / 181, 234 / 221, 484 / 385; dK/dV 142 / 103,
-//     244 / 175, 544 / 380.
-// A wave of dQ takes 7.3 + 0.49 n us on 64-token tiles and 15.2 + 0.61 n us on 128-row tiles, n the 64-token tiles of a route,
-// which is the comparison below; it names the faster kernel, or one within 2.5 %, at every point of 32 to 3072 row tiles x 2 to 64
-// tiles a route that was measured.  A wave of the forward costs 1.1 times as much on 128 rows and of dK/dV 1.25 times, at any n.
+// Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as 64-row tiles (sparse_split.inl).
+// A 128-row CTA does twice the rows in less than twice the time, so 64-row tiles are the faster ones where halving the CTAs saves no
+// wave (times on one B200, head dim 128, full blocks, us, 64-row / 128-row, 2 / 8 / 32 tiles of 64 a route):
+//   all 64-row tiles on the SMs at once ([1, 2, 4096]): forward 11.2 / 12.5, 13.6 / 15.9, 21.4 / 24.7; dQ 8.2 / 9.1, 10.7 / 12.5,
+//     19.8 / 24.9; dK/dV 10.9 / 14.1, 15.0 / 19.9, 26.3 / 38.6;
+//   three waves against two ([1, 3, 8192]): forward 21.5 / 23.1, 25.8 / 29.1, 46.2 / 46.5; dQ 21.6 / 17.4, 27.4 / 23.7, 50.8 / 48.8;
+//     dK/dV 19.1 / 15.5, 31.5 / 30.2, 66.6 / 70.2;
+//   many waves ([1, 12, 16384]): forward 120 / 131, 148 / 160, 260 / 258; dQ 162 / 110, 197 / 144, 361 / 283; dK/dV 131 / 84,
+//     207 / 144, 424 / 347.
+// The comparison of dQ is that of the kernels before whole-warp waits (a wave took 7.3 + 0.49 n us on 64-row and 15.2 + 0.61 n us on
+// 128-row tiles, n the tiles of a route).  It was kept when both sides became faster, the 128-row one more so: at three waves
+// against two it names the slower side by up to a fifth for short routes, and so does the forward's rule by a tenth.
 bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk) {
   if (be % 128 != 0) return false;
   if (D == 64) return sparse_wide64_pays(pass, BH, L, be, topk);
