@@ -92,3 +92,33 @@ def test_many_ragged_tiles_leave_their_neighbours_alone(D, tk, monkeypatch):
         assert torch.equal(out, outs["auto"][0])
         # P carries 2^-9 and the output 2^-9 of values below 1/2: a cleared row of V would show as one of ~1500 weights, times |v|
         assert (out.float() - want).abs().max() < 4e-3
+
+
+@pytest.mark.parametrize("qb", [1, 2, 3])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_key_that_nobody_attends_to_keeps_finite_gradients(D, qb):
+    """A key whose score is -inf for every query has probability zero: its dK and dV are exactly zero, as they are in the formula,
+    also where an odd number of query tiles leaves half of the last pair without a tile (zero rows times an infinite key are NaN)."""
+    from simple_vsa_b200 import _lib, b200_sparse_attention
+    g = torch.Generator().manual_seed(qb + D)
+    be, B, H, kb, tk = 64, 1, 2, 3, 2
+    q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, H, kb * be, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    q[..., 0] = q[..., 0].abs() + 0.5
+    k[:, :, [3, 40], 0] = float("-inf")
+    sizes = torch.tensor([be, 50, be])
+    selected = torch.tensor([0, 1], dtype=torch.int32).expand(B, H, qb, tk).contiguous()
+    want_in = [x.clone().requires_grad_() for x in (q, k, v)]
+    want = O.sparse_attention(*want_in, selected, sizes, be)
+    want.backward(dout.float())
+    leaves = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    out = b200_sparse_attention(*leaves, selected.to(DEV), sizes, block_size=(1, 1, be))
+    out.backward(dout.to(DEV))
+    assert _lib.device_status() == 0
+    bound = 4 * 2.0 ** -9                                  # as above
+    for got, ref in ((out, want), (leaves[1].grad, want_in[1].grad), (leaves[2].grad, want_in[2].grad)):
+        got, ref = got.detach().float().cpu(), ref.detach().float()
+        assert torch.isfinite(ref).all() and torch.isfinite(got).all()
+        assert (got - ref).norm() <= bound * ref.norm()
+    for x in leaves[1:]:
+        assert (x.grad[:, :, [3, 40]] == 0).all()
