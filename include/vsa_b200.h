@@ -344,14 +344,13 @@ int vsa_gather_rows(const void* src, const int32_t* map, void* dst,
 /* What the fine-attention entry points run on for a shape in this process (environment switches included):
  * 2 = tcgen05/TMA with every option of this header (bf16 or fp16, D = 128, be = 64, 128 or 256, topk*ceil(be/64) <= 1024),
  * 1 = tensor cores for the ordinary layout only, without shard-major K/V, raster-order stores and stored dS (bf16 or fp16,
- * D = 64 or 128, be = 64, 128 or 256: tcgen05 for D = 64 while topk*ceil(be/64) <= 1024, else warp-level mma.sync), 0 = CUDA-core
- * kernels (everything else the reference accepts, and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
+ * D = 64 or 128, be = 64, 128 or 256: warp-level mma.sync, or tcgen05 for D = 64 where it is faster and topk*ceil(be/64) <=
+ * 1024; vsa_sparse_pass_kernels tells), 0 = CUDA-core kernels (everything else the reference accepts, and the fp32 validation mode).  No reference counterpart: its Triton launcher has one kernel family. */
 int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
 
 /* The kernels that one fine pass of an ordinary call (vsa_sparse_fwd with lse2, vsa_sparse_bwd_dq, vsa_sparse_bwd_dkdv) takes:
  * pass 0 = forward, 1 = dQ, 2 = dK/dV; L = Lq for the first two, Lkv for the third.  3 = tcgen05 on 128-row tiles, 2 = tcgen05
- * on 64-row tiles with every option, 1 = 64-row tiles for the ordinary layout only (tcgen05 at D = 64, else warp-level mma.sync),
- * 0 = CUDA cores; negative for bad arguments. */
+ * on 64-row tiles, 1 = warp-level mma.sync, 0 = CUDA cores; negative for bad arguments. */
 int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype);
 
 /* ---- the whole operator in one call per direction ------------------------------------------------------------

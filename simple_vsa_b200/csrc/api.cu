@@ -493,7 +493,7 @@ int vsa_sparse_kernel_family(int D, int be, int topk, int dtype) {
 int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype) {
   VSA_REQUIRE(pass >= 0 && pass <= 2 && BH >= 1 && be >= 1 && L >= be && L % be == 0, "sparse pass kernels: bad arguments");
   if (scalar_forced()) return 0;
-  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk) ? 3 : D == 128 ? 2 : 1;
+  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk) ? 3 : 2;
   return sparse_tc_eligible(D, be, dtype) ? 1 : 0;
 }
 

@@ -167,13 +167,14 @@ def test_kernels_of_a_pass():
     for p in range(3):
         assert kernels(p, 8, 65536, 128, 64, 16) == 2
         assert kernels(p, 8, 65536, 128, 128, 16) == 3
-        assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F16) == 1
+        assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F16) == 2
+        assert kernels(p, 8, 65536, 64, 64, 4) == 1                        # short routes: mma.sync
         assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F32) == 0
         assert kernels(p, 8, 65536, 64, 128, 513) == 1                     # 1026 tiles: beyond the tile list
         # head dim 64: up to 8 tiles of 64 tokens a route the forward and dQ are faster on the warp-level kernels, up to 4 where
         # the 128-row tiles fill the SMs (148 without a device) just once
         assert [kernels(p, 4, 4096, 64, 128, tk) for tk in (2, 3)] == ([1, 3] if p < 2 else [3, 3])
-        assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([1, 3] if p < 2 else [3, 3])
+        assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([2, 3] if p < 2 else [3, 3])
         assert [kernels(p, 8, 65536, 64, 128, tk) for tk in (1, 4, 5)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
         assert [kernels(p, 8, 65536, 64, 256, tk) for tk in (1, 2, 3)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
         # head dim 128: 64-token tiles where all of them fit on the SMs at once ...
