@@ -48,11 +48,11 @@ static bool mma_forced() {
 
 // The kernels that a pass of an ordinary call runs on: head dim 128 on tcgen05, head dim 64 too where it is the faster path.  Head
 // dim 64 has it in the ordinary layout only; the other entry points ask sparse_umma_eligible.
-static bool on_umma(SparsePass pass, int64_t BH, int64_t L, int D, int be, int dtype, int topk) {
+static bool on_umma(SparsePass pass, int64_t BH, int64_t L, int D, int be, int dtype, int topk, bool fused = false) {
   if (scalar_forced() || mma_forced()) return false;
   if (sparse_umma_eligible(D, be, dtype, topk)) return true;
   return sparse_umma64_eligible(D, be, dtype, topk) &&
-         (sparse_wide_rows(pass, BH, L, D, be, topk) || sparse_split64_pays(pass, BH, L, be, topk));
+         (sparse_wide_rows(pass, BH, L, D, be, topk) || sparse_split64_pays(pass, BH, L, be, topk, fused));
 }
 
 static int check_dtype(int dtype) {
@@ -317,7 +317,7 @@ int vsa_sparse_bwd_dq_fused(const void* dout, const void* q, const void* k, cons
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && out_s && lse2 && selected && kv_sizes && delta && dq && dq_mean && q_sizes,
               "sparse dQ (fused): null pointer");
-  if (on_umma(kPassDq, BH, Lq, D, be, dtype, topk))
+  if (on_umma(kPassDq, BH, Lq, D, be, dtype, topk, true))
     return sparse_dq_umma(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
                           dtype, (cudaStream_t)stream, dq_mean, q_sizes);
   rc = vsa_sparse_bwd_dq(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, D, be, topk, scale,
@@ -335,7 +335,7 @@ int vsa_sparse_bwd_dkdv_fused(const void* dout, const void* q, const void* k, co
   if (rc) return rc;
   VSA_REQUIRE(dout && q && k && v && lse2 && delta && counts && offsets && inverse && kv_sizes && dk && dv &&
                   dk_mean && dv_mean, "sparse dK/dV (fused): null pointer");
-  if (on_umma(kPassDkdv, BH, Lkv, D, be, dtype, topk))
+  if (on_umma(kPassDkdv, BH, Lkv, D, be, dtype, topk, true))
     return sparse_dkdv_umma(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,
                             topk, scale, dtype, (cudaStream_t)stream, dk_mean, dv_mean);
   rc = vsa_sparse_bwd_dkdv(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, D, be,

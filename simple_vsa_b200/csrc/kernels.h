@@ -89,7 +89,8 @@ bool sparse_umma_eligible(int D, int be, int dtype, int topk);
 // head dim 64 on tcgen05: ordinary layout only (no shard-major K/V, raster stores or stored dS)
 bool sparse_umma64_eligible(int D, int be, int dtype, int topk);
 enum SparsePass { kPassForward = 0, kPassDq = 1, kPassDkdv = 2 };
-bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk);    // L as below
+// L as below; fused: a gradient pass that adds the pooled gradients
+bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk, bool fused);
 // 128-row kernels (true) or tiles of 64 rows; L = Lq for the forward and dQ, Lkv for dK/dV
 bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk);
 int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes,

@@ -276,18 +276,24 @@ static bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, i
   const int64_t sms = sm_count(), rows128 = BH * (L / 128);
   return topk * (be / kTile) > (rows128 <= sms && 2 * rows128 > sms ? 4 : 8);
 }
-// Head dim 64 on 64-row tiles: tcgen05 (sparse_split.inl) or mma.sync, of which three or four CTAs share an SM and need little set-up,
-// so that they are faster while a route holds few tiles.  us, tcgen05 / mma.sync, by tiles per route:
-//   [1, 12, 16384, 64]  forward 4: 97 / 60, 8: 113 / 103, 12: 133 / 146, 16: 150 / 190, 32: 215 / 364;
-//                       dQ 4: 141 / 86, 8: 162 / 142, 12: 185 / 199, 16: 206 / 256, 32: 292 / 483;
-//                       dK/dV 4: 151 / 118, 8: 187 / 195, 16: 257 / 349, 32: 394 / 652
-//   [1, 2, 2048, 64], all tiles on the SMs at once: forward 2: 8.4 / 4.8, 6: 10.5 / 9.6, 8: 10.6 / 11.5, 12: 11.8 / 15.8;
-//                       dQ 2: 6.7 / 7.1, 6: 7.9 / 12.6, 12: 9.3 / 19.6;  dK/dV 2: 8.0 / 13.5, 6: 11.1 / 22.4, 12: 13.3 / 27.3
-bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
-  const int64_t n = (int64_t)topk * (be / kTile);
-  const bool one_wave = BH * (L / kTile) <= sm_count();
-  if (pass == kPassForward) return n > (one_wave ? 6 : 8);
-  return one_wave || n > (pass == kPassDq ? 8 : 6);
+// Head dim 64 on 64-row tiles: tcgen05 (sparse_split.inl; the forward has two CTAs on an SM, the backward one) or mma.sync, of which
+// three or four CTAs share an SM and need little set-up, so that they are faster while a route holds few tiles: the longer, the less
+// the 64-row tcgen05 tiles fill their last wave.  us, tcgen05 / mma.sync, blocks of 64, by tiles per route:
+//   [1, 2, 4096, 64], 128 row tiles    forward 2: 9.4 / 5.0, 7: 11.7 / 10.9, 8: 11.2 / 11.9;  dQ 1: 6.9 / 3.7, 3: 7.2 / 6.5, 4: 7.1 / 7.6;
+//                                      dK/dV 1: 7.4 / 7.0, 2: 8.2 / 8.2, 3: 8.8 / 10.6
+//   [1, 4, 4096, 64], 256              forward 7: 13.5 / 13.1, 8: 13.5 / 14.3;  dQ 7: 15.3 / 14.8, 8: 15.0 / 16.3;  dK/dV 2: 13.4 / 11.9, 3: 15.6 / 15.4
+//   [1, 3, 8192, 64], 384              forward 10: 22.1 / 21.0, 12: 23.6 / 24.4;  dQ 8: 21.4 / 20.7, 10: 23.0 / 24.9;  dK/dV 4: 22.1 / 21.3, 5: 23.4 / 25.1
+//   [1, 5, 8192, 64], 640              forward 8: 29.9 / 28.8, 10: 32.2 / 34.9;  dQ 8: 34.1 / 34.0, 10: 36.9 / 41.4;  dK/dV 5: 34.5 / 33.9, 6: 37.5 / 39.1
+//   [1, 12, 8192, 64], 1536            forward 9: 64.7 / 59.9, 10: 63.5 / 65.8;  dQ 9: 80.9 / 78.7, 10: 79.8 / 85.7;  dK/dV 7: 84.6 / 83.2, 8: 89.8 / 93.8
+//   [1, 12, 16384, 64], 3072           forward 9: 126 / 114, 10: 124 / 125, 12: 133 / 146;  dQ 9: 162 / 149, 10: 159 / 163;  dK/dV 8: 178 / 172, 9: 187 / 191
+// With the pooled gradients (`fused`) mma.sync needs one more launch per gradient, which moves the line on small grids: 128 row tiles,
+// dQ 1: 7.4 / 6.3, 2: 7.2 / 7.6, dK/dV 1: 7.4 / 12.0; 256, dQ 5: 15.2 / 14.2, 6: 14.9 / 15.9; 3072, dQ 9: 177 / 156, 12: 184 / 199,
+// dK/dV 7: 176 / 168, 8: 185 / 188.  At no point measured is the slower side taken by more than 5 %.
+bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk, bool fused) {
+  const int64_t n = (int64_t)topk * (be / kTile), sms = sm_count(), tiles = BH * (L / kTile), waves = (tiles + sms - 1) / sms;
+  if (pass == kPassForward) return n >= (waves <= 2 ? 8 : waves == 3 ? 12 : 10);
+  if (pass == kPassDq) return n >= (waves == 1 ? 4 : waves <= 5 ? 8 : 10) - (fused && waves <= 2 ? 2 : 0);
+  return n >= std::min<int64_t>({waves + 1, 5 + waves / 4, 9}) - (fused ? (waves < 8 ? 2 : 1) : 0);
 }
 
 // Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as 64-row tiles (sparse_split.inl).

@@ -24,7 +24,7 @@ def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype, large):
     for p, n in enumerate((qb, qb, kb)):
         kernels = 3 if large or D == 64 else 2
         if D == 64 and p < 2 and tk * be // 64 <= (4 if large else 8):
-            kernels = 1 if large or (p == 0 and tk * be // 64 <= 6) else 2
+            kernels = 1 if large or tk * be // 64 < (8, 4)[p] else 2
         assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == kernels
     q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
     k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
