@@ -297,25 +297,21 @@ bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int top
 }
 
 // Whether blocks of 128 and 256 tokens take the 128-row kernels (sparse_wide.inl) or are walked as 64-row tiles (sparse_split.inl).
-// A 128-row CTA does twice the rows in less than twice the time, so 64-row tiles are the faster ones where halving the CTAs saves no
-// wave (times on one B200, head dim 128, full blocks, us, 64-row / 128-row, 2 / 8 / 32 tiles of 64 a route):
-//   all 64-row tiles on the SMs at once ([1, 2, 4096]): forward 11.2 / 12.5, 13.6 / 15.9, 21.4 / 24.7; dQ 8.2 / 9.1, 10.7 / 12.5,
-//     19.8 / 24.9; dK/dV 10.9 / 14.1, 15.0 / 19.9, 26.3 / 38.6;
-//   three waves against two ([1, 3, 8192]): forward 21.5 / 23.1, 25.8 / 29.1, 46.2 / 46.5; dQ 21.6 / 17.4, 27.4 / 23.7, 50.8 / 48.8;
-//     dK/dV 19.1 / 15.5, 31.5 / 30.2, 66.6 / 70.2;
-//   many waves ([1, 12, 16384]): forward 120 / 131, 148 / 160, 260 / 258; dQ 162 / 110, 197 / 144, 361 / 283; dK/dV 131 / 84,
-//     207 / 144, 424 / 347.
-// The comparison of dQ is that of the kernels before whole-warp waits (a wave took 7.3 + 0.49 n us on 64-row and 15.2 + 0.61 n us on
-// 128-row tiles, n the tiles of a route).  It was kept when both sides became faster, the 128-row one more so: at three waves
-// against two it names the slower side by up to a fifth for short routes, and so does the forward's rule by a tenth.
+// A 128-row CTA does twice the rows in less than twice the time, so 64-row tiles are the faster ones where they all are on the SMs at
+// once.  us, 64-row / 128-row, head dim 128, full blocks of 128, by tiles of 64 a route (one B200):
+//   [1, 2, 4096], 128 row tiles    forward 2: 11.4 / 12.5, 8: 13.3 / 15.6, 32: 20.9 / 24.2;  dQ 7.7 / 8.7, 10.0 / 11.8, 19.0 / 24.4;
+//                                  dK/dV 10.2 / 12.3, 15.1 / 20.7, 25.7 / 37.8
+// Beyond that the 128-row dQ is faster at every point measured (192 to 11,520 row tiles, 2 to 64 tiles a route), dK/dV at all but a
+// few of one or two waves (blocks of 256, [1, 3, 4096], 4: 12.3 / 15.2):
+//   [1, 3, 4096], 192              dQ 4: 14.2 / 9.7, 8: 16.9 / 12.1, 32: 33.0 / 24.5;  dK/dV 16.7 / 15.1, 21.7 / 19.8, 40.6 / 42.6
+//   [1, 3, 8192], 384              dQ 4: 21.1 / 18.2, 8: 24.9 / 22.7, 32: 48.5 / 47.9;  dK/dV 24.3 / 21.9, 29.7 / 25.7, 62.8 / 62.8
+//   [1, 12, 16384], 3072           dQ 4: 156 / 118, 8: 178 / 137, 32: 358 / 296;  dK/dV 155 / 104, 199 / 137, 457 / 350
+// The forward takes 128 rows there too, although 64-row tiles are up to a tenth faster for short routes ([1, 12, 16384], 4 tiles:
+// 130 / 141).
 bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk) {
   if (be % 128 != 0) return false;
   if (D == 64) return sparse_wide64_pays(pass, BH, L, be, topk);
-  const int64_t sms = sm_count();
-  const int64_t narrow = (BH * (L / 64) + sms - 1) / sms, wide = (BH * (L / 128) + sms - 1) / sms;
-  if (pass != kPassDq) return narrow > 1;
-  const int64_t n = (int64_t)topk * (be / 64);
-  return narrow * (60 + 4 * n) >= wide * (124 + 5 * n);
+  return BH * (L / kTile) > sm_count();
 }
 
 bool sparse_umma_eligible(int D, int be, int dtype, int topk) {

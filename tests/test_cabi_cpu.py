@@ -176,7 +176,7 @@ def test_kernels_of_a_pass():
         assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([2, 3] if p < 2 else [3, 3])
         assert [kernels(p, 8, 65536, 64, 128, tk) for tk in (1, 4, 5)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
         assert [kernels(p, 8, 65536, 64, 256, tk) for tk in (1, 2, 3)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
-        # head dim 128: 64-token tiles where all of them fit on the SMs at once ...
+        # head dim 128: 64-row tiles where all of them fit on the SMs at once ...
         assert [kernels(p, BH, 64 * 128, 128, 128, 32) for BH in (1, 2)] == [2, 3]
         assert [kernels(p, 1, 256 * nb, 128, 256, 16) for nb in (37, 38)] == [2, 3]
     # head dim 64, blocks of 64: the first route length that tcgen05 takes, and the last of mma.sync, by pass, for 1, 2, 3, 11 and 21
@@ -184,8 +184,9 @@ def test_kernels_of_a_pass():
     for BH, n, lines in ((1, 4096, (8, 4, 2)), (4, 4096, (8, 8, 3)), (3, 8192, (12, 8, 4)), (12, 8192, (10, 10, 7)), (12, 16384, (10, 10, 9))):
         for p, line in enumerate(lines):
             assert [kernels(p, BH, n, 64, 64, tk) for tk in (line - 1, line)] == [1, 2]
-    # head dim 128: 64-row tiles for short routes of dQ where 128-row tiles take more than half as many waves
-    assert [kernels(1, 3, 8192, 128, 128, tk) for tk in (1, 12, 32)] == [2, 2, 3]
+    # and 128-row tiles for any route of dQ otherwise
+    assert [kernels(1, 3, 8192, 128, 128, tk) for tk in (1, 12, 32)] == [3, 3, 3]
+    assert [kernels(1, 12, 16384, 128, 128, tk) for tk in (1, 4)] == [3, 3]
     assert [kernels(1, 80, 92160, 128, be, 1) for be in (128, 256)] == [3, 3]
     assert kernels(3, 8, 65536, 128, 64, 16) == L.ERR_BAD_ARGUMENT
     assert kernels(0, 8, 65, 128, 64, 1) == L.ERR_BAD_ARGUMENT
