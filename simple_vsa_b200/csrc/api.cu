@@ -52,7 +52,7 @@ static bool on_umma(SparsePass pass, int64_t BH, int64_t L, int D, int be, int d
   if (scalar_forced() || mma_forced()) return false;
   if (sparse_umma_eligible(D, be, dtype, topk)) return true;
   return sparse_umma64_eligible(D, be, dtype, topk) &&
-         (sparse_wide_rows(pass, BH, L, D, be, topk) || sparse_split64_pays(pass, BH, L, be, topk, fused));
+         (sparse_wide_rows(pass, BH, L, D, be, topk, fused) || sparse_split64_pays(pass, BH, L, be, topk, fused));
 }
 
 static int check_dtype(int dtype) {
@@ -493,7 +493,7 @@ int vsa_sparse_kernel_family(int D, int be, int topk, int dtype) {
 int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype) {
   VSA_REQUIRE(pass >= 0 && pass <= 2 && BH >= 1 && be >= 1 && L >= be && L % be == 0, "sparse pass kernels: bad arguments");
   if (scalar_forced()) return 0;
-  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk) ? 3 : 2;
+  if (on_umma((SparsePass)pass, BH, L, D, be, dtype, topk)) return sparse_wide_rows((SparsePass)pass, BH, L, D, be, topk, false) ? 3 : 2;
   return sparse_tc_eligible(D, be, dtype) ? 1 : 0;
 }
 

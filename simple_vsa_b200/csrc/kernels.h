@@ -92,7 +92,7 @@ enum SparsePass { kPassForward = 0, kPassDq = 1, kPassDkdv = 2 };
 // L as below; fused: a gradient pass that adds the pooled gradients
 bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk, bool fused);
 // 128-row kernels (true) or tiles of 64 rows; L = Lq for the forward and dQ, Lkv for dK/dV
-bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk);
+bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk, bool fused);
 int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* selected, const int32_t* kv_sizes,
                     void* out, float* lse2, int64_t BH, int64_t Lq, int64_t Lkv, int D, int be, int topk, float scale,
                     int dtype, cudaStream_t st, const void* out_c = nullptr, const void* gate = nullptr,

@@ -267,14 +267,25 @@ static int sm_count() {
   return 148;
 }
 
-// Head dim 64, blocks of 128 and 256 tokens: the 128-row kernels or 64-row ones.  us at [1, 12, 16384, 64], blocks of 128, 128-row
-// kernels / mma.sync, by 64-token tiles per route: forward 8: 134 / 104, 12: 149 / 149, 16: 166 / 193; dQ 8: 183 / 142, 12: 204 / 199,
-// 16: 226 / 254; dK/dV 2: 82 / 77, 4: 108 / 120.  Where the 128-row CTAs just fill the SMs once they win earlier: [1, 4, 4096, 64],
-// 8 tiles: forward 13.0 / 15.0, dQ 10.7 / 20.4.
-static bool sparse_wide64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int topk) {
-  if (pass == kPassDkdv) return true;
-  const int64_t sms = sm_count(), rows128 = BH * (L / 128);
-  return topk * (be / kTile) > (rows128 <= sms && 2 * rows128 > sms ? 4 : 8);
+// Head dim 64, blocks of 128 and 256 tokens: whether the 128-row kernels are faster than both the 64-row tcgen05 kernels and
+// mma.sync.  us, 64-row / 128-row / mma.sync, blocks of 128, by tiles of 64 a route:
+//   [1, 2, 4096, 64], 128 row tiles    forward 8: 11.1 / 12.5 / 11.6, 16: 13.7 / 15.0 / 20.0;  dQ 4: 7.1 / 7.9 / 7.4, 16: 10.3 / 13.0 / 21.4;
+//                                      dK/dV 2: 8.9 / 11.4 / 11.8, 16: 17.0 / 26.4 / 35.8: never
+//   [1, 4, 4096, 64], 256              forward 6: 12.4 / 12.3 / 11.8, 8: 13.5 / 13.0 / 14.7;  dQ 2: 11.9 / 7.2 / 6.3, 4: 12.7 / 8.3 / 9.7;
+//                                      dK/dV 4: 15.7 / 14.6 / 20.3, 6: 17.5 / 19.0 / 26.5 (blocks of 256, 16: 29.7 / 36.8 / 68.7)
+//   [1, 3, 8192, 64], 384              forward 12: 23.5 / 25.2 / 24.7, 24: 32.1 / 32.9 / 45.5;  dQ 4: 18.1 / 14.7 / 12.3, 6: 19.9 / 16.5 / 16.5;
+//                                      dK/dV 4: 20.5 / 18.2 / 26.9, 16: 36.6 / 37.4 / 62.9
+//   [1, 4, 8192, 64], 512              forward 8: 22.9 / 22.8 / 21.4, 10: 24.7 / 24.2 / 25.9, 16: 29.7 / 28.0 / 38.9
+//   [1, 12, 16384, 64], 3072           forward 12: 131 / 136 / 149, 24: 179 / 179 / 283;  dQ 4: 125 / 85 / 77, 6: 136 / 94 / 106;
+//                                      dK/dV 2: 103 / 66 / 61, 4: 132 / 89 / 100, 16: 241 / 190 / 329
+// With the pooled gradients (`fused`) dQ crosses earlier while the grid is small: 256 row tiles, 2: 12.9 / 7.7 / 10.4; 640, 4: 31.2 / 22.4 /
+// 24.1; 3072, 4: 138 / 92 / 85.
+static bool sparse_wide64_pays(SparsePass pass, int64_t tiles, int64_t n, bool fused) {
+  const int64_t sms = sm_count(), waves = (tiles + sms - 1) / sms;
+  if (waves == 1) return false;
+  if (pass == kPassForward) return n >= (waves == 2 ? 8 : waves == 4 ? 10 : 24);
+  if (pass == kPassDkdv) return waves > 2 || n < 6;
+  return n >= (waves == 2 ? 4 : 6) - (fused && waves <= 8 ? 2 : 0);
 }
 // Head dim 64 on 64-row tiles: tcgen05 (sparse_split.inl; the forward has two CTAs on an SM, the backward one) or mma.sync, of which
 // three or four CTAs share an SM and need little set-up, so that they are faster while a route holds few tiles: the longer, the less
@@ -293,6 +304,7 @@ bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int top
   const int64_t n = (int64_t)topk * (be / kTile), sms = sm_count(), tiles = BH * (L / kTile), waves = (tiles + sms - 1) / sms;
   if (pass == kPassForward) return n >= (waves <= 2 ? 8 : waves == 3 ? 12 : 10);
   if (pass == kPassDq) return n >= (waves == 1 ? 4 : waves <= 5 ? 8 : 10) - (fused && waves <= 2 ? 2 : 0);
+  if (be > kTile) return true;      // [1, 2, 4096, 64], 2: 8.9 / 11.8; longer routes and larger grids: the 128-row kernels are asked first
   return n >= std::min<int64_t>({waves + 1, 5 + waves / 4, 9}) - (fused ? (waves < 8 ? 2 : 1) : 0);
 }
 
@@ -308,10 +320,11 @@ bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int top
 //   [1, 12, 16384], 3072           dQ 4: 156 / 118, 8: 178 / 137, 32: 358 / 296;  dK/dV 155 / 104, 199 / 137, 457 / 350
 // The forward takes 128 rows there too, although 64-row tiles are up to a tenth faster for short routes ([1, 12, 16384], 4 tiles:
 // 130 / 141).
-bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk) {
+bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk, bool fused) {
   if (be % 128 != 0) return false;
-  if (D == 64) return sparse_wide64_pays(pass, BH, L, be, topk);
-  return BH * (L / kTile) > sm_count();
+  const int64_t tiles = BH * (L / kTile), n = (int64_t)topk * (be / kTile);
+  if (D == 64) return sparse_wide64_pays(pass, tiles, n, fused);
+  return tiles > sm_count();
 }
 
 bool sparse_umma_eligible(int D, int be, int dtype, int topk) {

@@ -52,7 +52,7 @@ int sparse_fwd_umma(const void* q, const void* k, const void* v, const int32_t* 
   if (BH == 0 || Lq == 0) return VSA_OK;
   { const int rc0 = check_kv_shard(Lkv, be, &kv_shard, "sparse forward"); if (rc0) return rc0; }
   if (BH > 65535) return fail(VSA_ERR_UNSUPPORTED, "sparse forward: batch*heads %lld exceeds 65535", (long long)BH);
-  if (sparse_wide_rows(kPassForward, BH, Lq, D, be, topk))
+  if (sparse_wide_rows(kPassForward, BH, Lq, D, be, topk, false))
     return D == 64 ? launch_fwd_wide<64>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map)
                    : launch_fwd_wide<128>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map);
   return D == 64 ? launch_fwd_split<64>(q, k, v, selected, kv_sizes, out, lse2, BH, Lq, Lkv, be, topk, scale, st, out_c, gate, out_comb, kv_shard, comb_map)
@@ -66,7 +66,7 @@ int sparse_dq_umma(const void* dout, const void* q, const void* k, const void* v
   if (BH == 0 || Lq == 0) return VSA_OK;
   if (BH > 65535) return fail(VSA_ERR_UNSUPPORTED, "sparse dQ: batch*heads %lld exceeds 65535", (long long)BH);
   { const int rc0 = check_kv_shard(Lkv, be, &kv_shard, "sparse dQ"); if (rc0) return rc0; }
-  if (sparse_wide_rows(kPassDq, BH, Lq, D, be, topk))
+  if (sparse_wide_rows(kPassDq, BH, Lq, D, be, topk, dq_mean != nullptr))
     return D == 64 ? launch_dq_wide<64>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map)
                    : launch_dq_wide<128>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map);
   return D == 64 ? launch_dq_split<64>(dout, q, k, v, out_s, lse2, selected, kv_sizes, delta, dq, BH, Lq, Lkv, be, topk, scale, st, dq_mean, q_sizes, kv_shard, out_map)
@@ -85,7 +85,7 @@ int sparse_dkdv_umma(const void* dout, const void* q, const void* k, const void*
     return fail(VSA_ERR_UNSUPPORTED, "sparse dK/dV: packed edges hold at most %d routes per query block", 1 << kEdgeSlotBits);
   CUtensorMap mq, mdo, mk, mv;
   int rc;
-  if (!ds_ws && sparse_wide_rows(kPassDkdv, BH, Lkv, D, be, topk))
+  if (!ds_ws && sparse_wide_rows(kPassDkdv, BH, Lkv, D, be, topk, dk_mean != nullptr))
     return D == 64 ? launch_dkdv_wide<64>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map)
                    : launch_dkdv_wide<128>(dout, q, k, v, lse2, delta, counts, offsets, inverse, kv_sizes, dk, dv, BH, Lq, Lkv, be, topk, scale, st, dk_mean, dv_mean, kv_shard, out_map);
   if (ds_ws == nullptr)

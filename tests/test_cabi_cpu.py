@@ -170,12 +170,6 @@ def test_kernels_of_a_pass():
         assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F16) == 2
         assert kernels(p, 8, 65536, 64, 64, 16, L.VSA_F32) == 0
         assert kernels(p, 8, 65536, 64, 128, 513) == 1                     # 1026 tiles: beyond the tile list
-        # head dim 64: up to 8 tiles of 64 tokens a route the forward and dQ are faster on the warp-level kernels, up to 4 where
-        # the 128-row tiles fill the SMs (148 without a device) just once
-        assert [kernels(p, 4, 4096, 64, 128, tk) for tk in (2, 3)] == ([1, 3] if p < 2 else [3, 3])
-        assert [kernels(p, 2, 4096, 64, 128, tk) for tk in (4, 5)] == ([2, 3] if p < 2 else [3, 3])
-        assert [kernels(p, 8, 65536, 64, 128, tk) for tk in (1, 4, 5)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
-        assert [kernels(p, 8, 65536, 64, 256, tk) for tk in (1, 2, 3)] == ([1, 1, 3] if p < 2 else [3, 3, 3])
         # head dim 128: 64-row tiles where all of them fit on the SMs at once ...
         assert [kernels(p, BH, 64 * 128, 128, 128, 32) for BH in (1, 2)] == [2, 3]
         assert [kernels(p, 1, 256 * nb, 128, 256, 16) for nb in (37, 38)] == [2, 3]
@@ -184,6 +178,16 @@ def test_kernels_of_a_pass():
     for BH, n, lines in ((1, 4096, (8, 4, 2)), (4, 4096, (8, 8, 3)), (3, 8192, (12, 8, 4)), (12, 8192, (10, 10, 7)), (12, 16384, (10, 10, 9))):
         for p, line in enumerate(lines):
             assert [kernels(p, BH, n, 64, 64, tk) for tk in (line - 1, line)] == [1, 2]
+    # head dim 64, blocks of 128: by pass, for 1, 2, 3, 4 and 21 waves of 148 row tiles; two of them a block
+    for BH, n, want in ((2, 4096, {1: (1, 1, 2), 2: (1, 2, 2), 4: (2, 2, 2), 24: (2, 2, 2)}),
+                        (4, 4096, {1: (1, 1, 3), 2: (1, 3, 3), 3: (1, 3, 2), 4: (3, 3, 2), 24: (3, 3, 2)}),
+                        (3, 8192, {2: (1, 1, 3), 3: (1, 3, 3), 5: (1, 3, 3), 6: (2, 3, 3), 11: (2, 3, 3), 12: (3, 3, 3)}),
+                        (4, 8192, {2: (1, 1, 3), 3: (1, 3, 3), 4: (1, 3, 3), 5: (3, 3, 3)}),
+                        (12, 16384, {1: (1, 1, 3), 2: (1, 1, 3), 3: (1, 3, 3), 4: (1, 3, 3), 5: (2, 3, 3), 11: (2, 3, 3), 12: (3, 3, 3)})):
+        for tk, passes in want.items():
+            assert tuple(kernels(p, BH, n, 64, 128, tk) for p in range(3)) == passes, (BH, n, tk)
+            if tk % 2 == 0:
+                assert tuple(kernels(p, BH, n, 64, 256, tk // 2) for p in range(3)) == passes, (BH, n, tk)
     # and 128-row tiles for any route of dQ otherwise
     assert [kernels(1, 3, 8192, 128, 128, tk) for tk in (1, 12, 32)] == [3, 3, 3]
     assert [kernels(1, 12, 16384, 128, 128, tk) for tk in (1, 4)] == [3, 3]

@@ -390,7 +390,7 @@ def test_head_dim_64_runs_on_the_warp_level_tensor_kernels(be, nb, tk, dtype, mo
     assert _lib.lib.vsa_sparse_kernel_family(128, be, tk, dt_code) == 2
     assert _lib.lib.vsa_sparse_kernel_family(D, be, tk, _lib.VSA_F32) == 0
     kernels = lambda p: _lib.lib.vsa_sparse_pass_kernels(p, B * H, L, D, be, tk, dt_code)
-    assert [kernels(p) for p in range(3)] == ([1, 2, 2] if be == 64 else [2, 2, 3] if tk * be <= 8 * 64 else [3, 3, 3])
+    assert [kernels(p) for p in range(3)] == ([1, 2, 2] if be == 64 else [2, 2, 2])
     q, k, v, dout = (torch.randn(B, H, L, D).to(dtype) for _ in range(4))
     sizes = torch.full((nb,), be)
     sizes[1], sizes[nb // 2], sizes[-1] = 1, be // 2 + 3, be - 1

@@ -18,13 +18,13 @@ DEV = "cuda:0"
 def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype, large):
     from simple_vsa_b200 import _lib, b200_sparse_attention
     g = torch.Generator().manual_seed(be + 7 * kb + D)
-    # a few row tiles take the 64-token kernels at head dim 128; one full wave of 128-row tiles takes the others
+    # a few row tiles take the 64-row kernels; one full wave of 128-row tiles takes the others (head dim 64, short routes: mma.sync)
     B, H = 1, 296 // (qb * be // 64) if large else 2
     code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
     for p, n in enumerate((qb, qb, kb)):
-        kernels = 3 if large or D == 64 else 2
-        if D == 64 and p < 2 and tk * be // 64 <= (4 if large else 8):
-            kernels = 1 if large or tk * be // 64 < (8, 4)[p] else 2
+        kernels = 3 if large else 2
+        if D == 64 and p < 2 and tk * be // 64 < (8, 4)[p]:
+            kernels = 1
         assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == kernels
     q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
     k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
@@ -105,7 +105,7 @@ def test_small_fp16_probabilities_at_head_dim_64_are_as_precise_as_on_the_warp_l
     """One key 12 nats above 5000 others: their probabilities sit near the bottom of fp16, and the output is made of them."""
     from simple_vsa_b200 import _lib, ops
     g = torch.Generator().manual_seed(12)
-    be, qb, kb, D = 128, 2, 40, 64
+    be, qb, kb, D, H = 128, 2, 40, 64, 64
     q, k, v = (torch.randn(1, 1, n * be, D, generator=g) for n in (qb, kb, kb))
     k *= 0.5
     v += 1.0
@@ -113,9 +113,10 @@ def test_small_fp16_probabilities_at_head_dim_64_are_as_precise_as_on_the_warp_l
     k[0, 0, 5], v[0, 0, 5] = 0.0, 0.0
     k[0, 0, 5, 0] = 12.0 * D ** 0.5 / 4.0
     q, k, v = (x.half() for x in (q, k, v))
-    assert _lib.lib.vsa_sparse_pass_kernels(0, 1, qb * be, D, be, kb, _lib.VSA_F16) == 3
+    assert _lib.lib.vsa_sparse_pass_kernels(0, H, qb * be, D, be, kb, _lib.VSA_F16) == 3        # H equal heads
     want = (q[0, 0].double() @ k[0, 0].double().T * D ** -0.5).softmax(-1) @ v[0, 0].double()
-    selected = torch.arange(kb, dtype=torch.int32).expand(1, 1, qb, kb).contiguous().to(DEV)
+    q, k, v = (x.expand(1, H, -1, D).contiguous() for x in (q, k, v))
+    selected = torch.arange(kb, dtype=torch.int32).expand(1, H, qb, kb).contiguous().to(DEV)
     sizes = torch.full((kb,), be, dtype=torch.int32, device=DEV)
     error = {}
     for mode in ("auto", "mma"):
