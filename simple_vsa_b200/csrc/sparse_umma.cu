@@ -318,13 +318,20 @@ bool sparse_split64_pays(SparsePass pass, int64_t BH, int64_t L, int be, int top
 //   [1, 3, 4096], 192              dQ 4: 14.2 / 9.7, 8: 16.9 / 12.1, 32: 33.0 / 24.5;  dK/dV 16.7 / 15.1, 21.7 / 19.8, 40.6 / 42.6
 //   [1, 3, 8192], 384              dQ 4: 21.1 / 18.2, 8: 24.9 / 22.7, 32: 48.5 / 47.9;  dK/dV 24.3 / 21.9, 29.7 / 25.7, 62.8 / 62.8
 //   [1, 12, 16384], 3072           dQ 4: 156 / 118, 8: 178 / 137, 32: 358 / 296;  dK/dV 155 / 104, 199 / 137, 457 / 350
-// The forward takes 128 rows there too, although 64-row tiles are up to a tenth faster for short routes ([1, 12, 16384], 4 tiles:
-// 130 / 141).
+// The 64-row forward has two CTAs on an SM and less to set up: it is ahead for short routes, and on grids of three to five waves, where
+// 128-row CTAs leave half of their last wave empty, for longer ones.  With many waves the board's power limit decides; these are
+// times of 0.3 s of back-to-back calls:
+//   [1, 4, 4096], 256              forward 4: 13.9 / 14.3, 16: 19.1 / 19.4, 20: 20.9 / 20.5, 32: 26.1 / 25.2, 64: 40.0 / 37.0
+//   [1, 5, 8192], 640              forward 4: 33.6 / 36.5, 16: 46.5 / 51.1, 32: 64.7 / 68.7, 40: 75.3 / 76.8, 64: 107 / 104
+//   [1, 12, 8192], 1536            forward 16: 104 / 110, 24: 132 / 129, 64: 267 / 236
+//   [1, 12, 16384], 3072           forward 16: 198 / 199, 24: 252 / 237, 64: 512 / 449
+//   [1, 8, 92160], 11520           forward 16: 729 / 695, 24: 923 / 862, 64: 1883 / 1661
 bool sparse_wide_rows(SparsePass pass, int64_t BH, int64_t L, int D, int be, int topk, bool fused) {
   if (be % 128 != 0) return false;
   const int64_t tiles = BH * (L / kTile), n = (int64_t)topk * (be / kTile);
   if (D == 64) return sparse_wide64_pays(pass, tiles, n, fused);
-  return tiles > sm_count();
+  const int64_t sms = sm_count(), waves = (tiles + sms - 1) / sms;
+  return waves > 1 && (pass != kPassForward || n > (waves > 2 && waves <= 5 ? 40 : 16));
 }
 
 bool sparse_umma_eligible(int D, int be, int dtype, int topk) {

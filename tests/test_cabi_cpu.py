@@ -188,7 +188,11 @@ def test_kernels_of_a_pass():
             assert tuple(kernels(p, BH, n, 64, 128, tk) for p in range(3)) == passes, (BH, n, tk)
             if tk % 2 == 0:
                 assert tuple(kernels(p, BH, n, 64, 256, tk // 2) for p in range(3)) == passes, (BH, n, tk)
-    # and 128-row tiles for any route of dQ otherwise
+    # the forward: 64-row tiles up to 16 tiles a route, up to 40 where 148 SMs take three to five waves of them
+    for BH, n, line in ((4, 4096, 16), (3, 8192, 40), (5, 8192, 40), (6, 8192, 16), (12, 16384, 16)):
+        assert [kernels(0, BH, n, 128, 128, tk) for tk in (1, line // 2, line // 2 + 1)] == [2, 2, 3]
+        assert [kernels(0, BH, n, 128, 256, tk) for tk in (1, line // 4, line // 4 + 1)] == [2, 2, 3]
+    # 128-row tiles for any route of dQ
     assert [kernels(1, 3, 8192, 128, 128, tk) for tk in (1, 12, 32)] == [3, 3, 3]
     assert [kernels(1, 12, 16384, 128, 128, tk) for tk in (1, 4)] == [3, 3]
     assert [kernels(1, 80, 92160, 128, be, 1) for be in (128, 256)] == [3, 3]

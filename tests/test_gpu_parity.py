@@ -880,7 +880,7 @@ def test_forward_with_the_combine_folded_in_equals_the_two_step_form(kernels, wi
 
 
 @pytest.mark.parametrize("be,nb,tk,W,H", [(64, 16, 5, 2, 3), (64, 24, 6, 4, 3), (256, 8, 3, 2, 3), (128, 12, 4, 2, 3),
-                                          (256, 8, 3, 2, 18), (128, 12, 4, 2, 24)])       # enough rows for the 128-row kernels
+                                          (256, 8, 5, 2, 18), (128, 12, 9, 2, 24)])       # enough rows, and routes, for the 128-row kernels
 def test_shard_major_kv_layout_equals_the_ordinary_layout(be, nb, tk, W, H):
     """The kernels of the sequence-parallel mode read K/V (and write dK/dV) in the rank-major layout an all-gather
     leaves, ``[W,B,H,L/W,D]``.  One GPU, no collective: the same operator on the same numbers in both layouts, a

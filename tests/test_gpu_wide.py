@@ -25,6 +25,8 @@ def test_blocks_of_128_rows_match_the_oracle(be, qb, kb, tk, D, dtype, large):
         kernels = 3 if large else 2
         if D == 64 and p < 2 and tk * be // 64 < (8, 4)[p]:
             kernels = 1
+        if large and D == 128 and p == 0 and tk * be // 64 <= 16:
+            kernels = 2
         assert _lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == kernels
     q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
     k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
@@ -136,14 +138,15 @@ def test_one_half_of_a_tile_outside_the_shift_range_is_recomputed_exactly(be, qb
     before them.  Output, statistic and combined output match the oracle in both halves."""
     from simple_vsa_b200 import _lib, ops
     g = torch.Generator().manual_seed(be + D)
-    H, kb, tk, scale = 296 // (qb * be // 64), 8, 6, D ** -0.5
+    # routes long enough for the 128-row forward; blocks 8 and up are empty
+    H, (kb, tk), scale = 296 // (qb * be // 64), (8, 6) if be == 256 else (12, 10), D ** -0.5
     q, gate = (torch.randn(1, H, qb * be, D, generator=g) for _ in range(2))
     k, v = (torch.randn(1, H, kb * be, D, generator=g) for _ in range(2))
     out_c = torch.randn(1, H, qb, D, generator=g).to(dtype)
     q.view(1, H, -1, 128, D)[:, :, :, 64:] *= q_factor
     k.view(1, H, kb, be, D)[:, :, 3] *= k_factor
     q, k, v, gate = (x.to(dtype) for x in (q, k, v, gate))
-    sizes = torch.tensor([5, be, be, be - 3, be, 64, be, 1])
+    sizes = torch.tensor([5, be, be, be - 3, be, 64, be, 1] + [0] * (kb - 8))
     selected = torch.rand(1, H, qb, kb, generator=g)
     selected[..., 0], selected[..., 3] = 3.0, 2.0           # the block of 5 keys comes first, the high-scoring one second
     selected = selected.topk(tk, dim=-1).indices.to(torch.int32)
@@ -161,3 +164,38 @@ def test_one_half_of_a_tile_outside_the_shift_range_is_recomputed_exactly(be, qb
     assert _lib.device_status() == 0
     for got, ref, rtol in ((out, want, 2e-2), (total, want_total, 2e-2), (lse, want_lse, 1e-3)):
         torch.testing.assert_close(got.float().cpu(), ref.float(), atol=2e-2 if rtol == 2e-2 else 5e-2, rtol=rtol)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("live", [1, 2, 3, 4, 7])
+def test_the_128_row_forward_on_routes_with_few_live_tiles(live, D, dtype):
+    """Long routes of mostly empty blocks: one to seven live tiles, fewer than its softmax groups or its rings hold and more, and
+    query blocks without any."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator().manual_seed(live + D)
+    be, qb, kb, tk, H, scale = 128, 2, 10, 9, 74, D ** -0.5
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    assert _lib.lib.vsa_sparse_pass_kernels(0, H, qb * be, D, be, tk, code) == 3
+    q = torch.randn(1, H, qb * be, D, generator=g).to(dtype)
+    k, v = (torch.randn(1, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
+    sizes = torch.tensor(([be, 1, 63, 64, 65, be, 127])[:live] + [0] * (kb - live))
+    for x in (k, v):                                      # whatever lies in the padding rows must not reach a result
+        x.view(1, H, kb, be, D)[:, :, torch.arange(be)[None, :] >= sizes[:, None]] = float("nan")
+    clean = [torch.nan_to_num(x.float(), nan=0.0).to(dtype) for x in (k, v)]
+    selected = torch.rand(1, H, qb, kb, generator=g)
+    selected[..., 0] = 2.0                                # block 0 is full: every row has a live key ...
+    selected = selected.topk(tk, dim=-1).indices.to(torch.int32)
+    selected[:, ::2, 1] = kb - 1                          # ... but in these query blocks none has
+    want, want_lse = O.sparse_attention(q, *clean, selected, sizes, be, return_lse2=True)
+    out, lse = ops.sparse_forward(q.to(DEV), k.to(DEV), v.to(DEV), selected.to(DEV), sizes.to(DEV, torch.int32), be, scale, True)[:2]
+    assert _lib.device_status() == 0
+    out, lse = out.float().cpu().view(1, H, qb, be, D), lse.cpu().view(1, H, qb, be)
+    dead = torch.zeros(1, H, qb, dtype=torch.bool)
+    dead[:, ::2, 1] = True
+    assert torch.isnan(out[dead]).all()
+    want, want_lse = want.float().view_as(out)[~dead], want_lse.float().view_as(lse)[~dead]
+    bound = 4 * 2.0 ** (-9 if dtype == torch.bfloat16 else -12)         # as above
+    assert (out[~dead] - want).norm() <= bound * want.norm()
+    # a score is a sum of D <= 128 products in fp32: off by at most 128 * 2^-24 * sum |q k| * scale * log2 e, sum |q k| below 300
+    assert (lse[~dead] - want_lse).abs().max() <= 1e-3

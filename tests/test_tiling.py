@@ -149,12 +149,12 @@ def _two_step(V, meta, q, k, v, gate, topk, tile_size):
                                                   ((8, 9, 16), (2, 8, 8), torch.float16)])
 @pytest.mark.parametrize("with_gate", [False, True])
 def test_raster_order_operator_equals_the_two_step_form(grid, tile_size, dtype, with_gate):
-    """Clipped tiles on every axis, full tiles, blocks of 64 / 128 / 256 tokens (128 on 64-token and on 128-row tiles): out, dq and dgate bit for bit (same
+    """Clipped tiles on every axis, full tiles, blocks of 64 / 128 / 256 tokens (128 on 64-row and on 128-row tiles): out, dq and dgate bit for bit (same
     kernels, same arithmetic, other store addresses); dk/dv up to the order of the fp32 sums over CSR rows."""
     import simple_vsa_b200 as V
     dev = "cuda:0"
     torch.manual_seed(11)
-    B, H, D, topk = 2, 3, 128, 3
+    B, H, D, topk = 2, 3, 128, 9 if grid == (8, 9, 16) else 3       # 18 tiles of 64 a route: the 128-row forward
     S = grid[0] * grid[1] * grid[2]
     meta = V.build_vsa_metadata(grid, tile_size, device=dev)
     make = lambda: torch.randn(B, S, H, D, device=dev).to(dtype)
