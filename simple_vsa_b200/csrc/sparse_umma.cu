@@ -276,14 +276,15 @@ static int sm_count() {
 //   [1, 3, 8192, 64], 384              forward 12: 23.5 / 25.2 / 24.7, 24: 32.1 / 32.9 / 45.5;  dQ 4: 18.1 / 14.7 / 12.3, 6: 19.9 / 16.5 / 16.5;
 //                                      dK/dV 4: 20.5 / 18.2 / 26.9, 16: 36.6 / 37.4 / 62.9
 //   [1, 4, 8192, 64], 512              forward 8: 22.9 / 22.8 / 21.4, 10: 24.7 / 24.2 / 25.9, 16: 29.7 / 28.0 / 38.9
-//   [1, 12, 16384, 64], 3072           forward 12: 131 / 136 / 149, 24: 179 / 179 / 283;  dQ 4: 125 / 85 / 77, 6: 136 / 94 / 106;
+//   [1, 12, 16384, 64], 3072           forward, 0.2 s of back-to-back calls (power limit), 12: 136 / 140 / 151, 16: 153 / 154 / 195,
+//                                      24: 195 / 183 / 285;  dQ 4: 125 / 85 / 77, 6: 136 / 94 / 106;
 //                                      dK/dV 2: 103 / 66 / 61, 4: 132 / 89 / 100, 16: 241 / 190 / 329
 // With the pooled gradients (`fused`) dQ crosses earlier while the grid is small: 256 row tiles, 2: 12.9 / 7.7 / 10.4; 640, 4: 31.2 / 22.4 /
 // 24.1; 3072, 4: 138 / 92 / 85.
 static bool sparse_wide64_pays(SparsePass pass, int64_t tiles, int64_t n, bool fused) {
   const int64_t sms = sm_count(), waves = (tiles + sms - 1) / sms;
   if (waves == 1) return false;
-  if (pass == kPassForward) return n >= (waves == 2 ? 8 : waves == 4 ? 10 : 24);
+  if (pass == kPassForward) return n >= (waves == 2 ? 8 : waves == 4 ? 10 : 18);
   if (pass == kPassDkdv) return waves > 2 || n < 6;
   return n >= (waves == 2 ? 4 : 6) - (fused && waves <= 8 ? 2 : 0);
 }
