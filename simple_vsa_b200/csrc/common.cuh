@@ -105,7 +105,6 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
   return bits_pair(r);
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return Elem<__nv_bfloat16>::pack(lo, hi); }
 
 // Row of token `token` of slice `bh` in a K/V-shaped tensor.  Ordinary tensors are [BH][Lkv][D] (shard == Lkv).  A
 // sequence-parallel all-gather leaves the shards of the W ranks one after another, [W][BH][Lkv/W][D]; with
