@@ -1,7 +1,8 @@
 """The 64-row tcgen05 kernels that put a tile of the other side on each lane half (blocks of 64 tokens at head dims 64 and 128, larger
-blocks on small grids) at the edges of their tiles, against the CPU oracle: odd and single tile counts (one half without a tile),
-more pairs than any ring is deep, live sizes around 0, 1, 32 (a part of V) and the full tile, query and key lengths that differ,
-whatever bits the padding rows hold, and score gaps beyond the range of the softmax shift."""
+blocks on small grids; at head dim 64 the shortest routes run on mma.sync, as each test says) at the edges of their tiles, against
+the CPU oracle: odd and single tile counts (one half without a tile), more pairs than any ring is deep, live sizes around 0, 1, 32
+(a part of V) and the full tile, query and key lengths that differ, whatever bits the padding rows hold, and score gaps beyond the
+range of the softmax shift."""
 
 import pytest
 import torch
@@ -122,3 +123,75 @@ def test_a_key_that_nobody_attends_to_keeps_finite_gradients(D, qb):
         assert (got - ref).norm() <= bound * ref.norm()
     for x in leaves[1:]:
         assert (x.grad[:, :, [3, 40]] == 0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("live", [1, 2, 3, 4, 7])
+def test_routes_with_few_live_tiles(live, D, dtype):
+    """Routes long enough for the 64-row kernels at either head dim, of mostly empty blocks: one live tile, one pair, an odd tail, and
+    a query block without any; every key block is read by an odd number of query tiles."""
+    from simple_vsa_b200 import _lib, b200_sparse_attention
+    g = torch.Generator().manual_seed(live + D)
+    be, B, H, qb, kb, tk = 64, 1, 2, 4, 9, 8
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    assert all(_lib.lib.vsa_sparse_pass_kernels(p, B * H, n * be, D, be, tk, code) == 2 for p, n in enumerate((qb, qb, kb)))
+    q, dout = (torch.randn(B, H, qb * be, D, generator=g).to(dtype) for _ in range(2))
+    k, v = (torch.randn(B, H, kb * be, D, generator=g).to(dtype) for _ in range(2))
+    sizes = torch.tensor(([be, 1, 32, 33, be, 31, be - 1])[:live] + [0] * (kb - live))
+    for x in (k, v):
+        x.view(B, H, kb, be, D)[:, :, torch.arange(be)[None, :] >= sizes[:, None]] = float("nan")
+    clean = [torch.nan_to_num(x.float(), nan=0.0).to(dtype) for x in (k, v)]
+    selected = torch.arange(tk, dtype=torch.int32).expand(B, H, qb, tk).contiguous()
+    selected = selected[..., torch.randperm(tk, generator=g)].contiguous()
+    selected[:, :, 2] = kb - 1                            # an empty block only
+    rows = torch.arange(qb * be) // be != 2
+    want_in = [q.clone().requires_grad_()] + [x.clone().requires_grad_() for x in clean]
+    want = O.sparse_attention(want_in[0][:, :, rows], *want_in[1:], selected[:, :, [0, 1, 3]], sizes, be, q_blocks_per_chunk=8)
+    want.backward(dout[:, :, rows].float())
+    leaves = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    out = b200_sparse_attention(*leaves, selected.to(DEV), sizes, block_size=(1, 1, be))
+    out.backward(dout.to(DEV))
+    assert _lib.device_status() == 0
+    assert torch.isnan(out[:, :, (~rows).to(DEV)].float()).all()
+    assert (leaves[0].grad[:, :, (~rows).to(DEV)] == 0).all()
+    bound = 4 * 2.0 ** (-9 if dtype == torch.bfloat16 else -12)         # as above
+    for got, ref in zip([out[:, :, rows.to(DEV)], leaves[0].grad[:, :, rows.to(DEV)]] + [x.grad for x in leaves[1:]],
+                        [want, want_in[0].grad[:, :, rows]] + [x.grad for x in want_in[1:]]):
+        got, ref = got.detach().float().cpu(), ref.detach().float()
+        assert torch.isfinite(got).all()
+        assert (got - ref).norm() <= bound * ref.norm()
+
+
+@pytest.mark.parametrize("dtype,k_factor,q_factor", [(torch.bfloat16, 8.0, 40.0), (torch.float16, 1.5, 20.0)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_recomputed_tile_takes_the_combine_with_it(D, dtype, k_factor, q_factor):
+    """The rows that the exact kernel computes again reach the combined output too, gated, and their neighbours keep theirs."""
+    from simple_vsa_b200 import _lib, ops
+    g = torch.Generator().manual_seed(D)
+    be, H, qb, kb, tk, scale = 64, 2, 6, 9, 8, D ** -0.5
+    code = _lib.VSA_BF16 if dtype == torch.bfloat16 else _lib.VSA_F16
+    assert _lib.lib.vsa_sparse_pass_kernels(0, H, qb * be, D, be, tk, code) == 2
+    q, gate = (torch.randn(1, H, qb * be, D, generator=g) for _ in range(2))
+    k, v = (torch.randn(1, H, kb * be, D, generator=g) for _ in range(2))
+    out_c = torch.randn(1, H, qb, D, generator=g).to(dtype)
+    q.view(1, H, qb, be, D)[:, :, 1::2] *= q_factor
+    k.view(1, H, kb, be, D)[:, :, 3] *= k_factor
+    q, k, v, gate = (x.to(dtype) for x in (q, k, v, gate))
+    sizes = torch.tensor([5, 9, be, be, be - 3, be, 64, be, 1])
+    selected = torch.tensor([0, 1, 2, 3, 4, 5, 6, 8], dtype=torch.int32).expand(1, H, qb, tk).contiguous()
+    # the scores say which tiles leave the range: fp16 holds 2^16, bf16 2^127 above the shift (at head dim 128 fp16 is four binades above)
+    s = torch.einsum("bhtd,bhsd->bhts", q.float(), k.float()) * scale * 1.4427
+    s = s.view(1, H, qb, be, kb, be)
+    first = torch.cat([s[:, :, :, :, 0, :5], s[:, :, :, :, 1, :9]], -1).amax(-1)
+    above = (s[:, :, :, :, 3].amax(-1) - first).amax(-1)
+    limit = 127 if dtype == torch.bfloat16 else 20
+    assert (above[:, :, 1::2] > limit + 4).all() and (above[:, :, ::2] < (limit if dtype == torch.bfloat16 else 14)).all()
+    want, want_lse = O.sparse_attention(q, k, v, selected, sizes, be, return_lse2=True)
+    want_total = O.combine(want.to(dtype), out_c, gate, be, dtype)
+    out, lse, total = ops.sparse_forward(q.to(DEV), k.to(DEV), v.to(DEV), selected.to(DEV), sizes.to(DEV, torch.int32), be, scale,
+                                         True, combine_with=(out_c.to(DEV), gate.to(DEV)))
+    assert _lib.device_status() == 0
+    # the bounds of the test of the 128-row kernels' redo path
+    for got, ref, rtol in ((out, want, 2e-2), (total, want_total, 2e-2), (lse, want_lse, 1e-3)):
+        torch.testing.assert_close(got.float().cpu(), ref.float(), atol=2e-2 if rtol == 2e-2 else 5e-2, rtol=rtol)
