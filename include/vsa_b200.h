@@ -350,7 +350,8 @@ int vsa_sparse_kernel_family(int D, int be, int topk, int dtype);
 
 /* The kernels that one fine pass of an ordinary call (vsa_sparse_fwd with lse2, vsa_sparse_bwd_dq, vsa_sparse_bwd_dkdv) takes:
  * pass 0 = forward, 1 = dQ, 2 = dK/dV; L = Lq for the first two, Lkv for the third.  3 = tcgen05 on 128-row tiles, 2 = tcgen05
- * on 64-row tiles, 1 = warp-level mma.sync, 0 = CUDA cores; negative for bad arguments. */
+ * on 64-row tiles, 1 = warp-level mma.sync, 0 = CUDA cores; negative for bad arguments.  At D = 64 the gradient calls that add the
+ * pooled gradients (vsa_sparse_bwd_dq_fused, vsa_sparse_bwd_dkdv_fused) go over to tcgen05 at shorter routes than these. */
 int vsa_sparse_pass_kernels(int pass, int64_t BH, int64_t L, int D, int be, int topk, int dtype);
 
 /* ---- the whole operator in one call per direction ------------------------------------------------------------

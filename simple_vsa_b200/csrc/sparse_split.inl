@@ -12,9 +12,11 @@
 // statistics of the resident side are thread-local, and the two partial results are added once, in the epilogue.
 //
 // Why not the 128 x 64 products on transposed operands that these kernels replace: those read 6 KB of shared memory per 32 cycles
-// of tensor work and pass P / dS through it, 176 / 224 / 288 KB a pair at D = 128 (forward / dQ / dK/dV).  Here it is 136 / 160 /
-// 208 KB: operands in tensor memory cost no shared-memory reads, and one MMA (47 cycles for M64 x N128 x K16, 76 for N256)
-// reads 4 KB or 8 KB of B alone.
+// of tensor work and pass P / dS through it, 176 / 224 / 288 KB a pair at D = 128 (forward / dQ / dK/dV, 64 KB of TMA writes
+// among them).  Here it is 136 / 160 / 208 KB: operands in tensor memory cost no shared-memory reads, and one MMA (47 cycles for
+// M64 x N128 x K16, 76 for N256) reads 4 KB or 8 KB of B alone.  At 90 pairs a tile a pair takes 847 / 1318 / 1690 cycles, set-up
+// and drain included, with operand reads at 67 / 57 / 68 % of their peak and the tensor pipe at 60 / 58 / 61 % ([1, 8, 92160, 128],
+// topk 180): what bounds it is the chain product -> elementwise -> product, and 10,000 to 12,000 cycles of set-up and drain a tile.
 
 // Live 64-token key tiles of a query block in routing order: row of the tile in the K/V tensors (a multiple of 64) << 1 | live
 // tokens.  Called by the whole CTA; ends with a barrier.  Ids outside the key table and empty tiles are dropped.

@@ -1,6 +1,6 @@
 // Fine (block-sparse) attention on the Blackwell tensor path: TMA tile gathers by block id, tcgen05.mma with accumulators in tensor
 // memory, warp-specialised elementwise stages.  This file has the host side, the self-tests and the choice between the kernels:
-//   sparse_split.inl     64-row tiles, a tile of the other side per lane half (blocks of 64 tokens; larger ones on small grids)
+//   sparse_split.inl     64-row tiles, a tile of the other side per lane half (blocks of 64 tokens; larger ones on small grids or with short routes)
 //   sparse_wide.inl      128-row tiles (blocks of 128 and 256 tokens)
 //   sparse_umma_bwd.inl  the opt-in backward that forms dS once
 //   coarse_umma.inl      the pooled branch
