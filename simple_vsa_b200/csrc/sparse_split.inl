@@ -952,9 +952,6 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     for (int p = 0; p < n_pairs && ok; ++p) {
       const int s = p % Sm::q_stages;
       const uint32_t ph = p & 1;
-      // A padding key row: its scores come from whatever sits in K there.  A tile that does not exist has zero rows, which an
-      // infinite key turns into NaN before the infinite statistic can make the probability zero.
-      const bool keep = live && 2 * p + half < n_tiles;
       ok = VSA_WARP_WAIT2(bar(SK_Q_FULL + s), (p / Sm::q_stages) & 1, bar(SK_S_FULL), ph);
       if (!ok) break;
       tc_fence_after();
@@ -976,8 +973,9 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           const float2 y = fma2(word_pair(sv + 4 * i + 2), c2, make_float2(l4.z, l4.w));
           pf[2 * i] = make_float2(fast_exp2(-x.x), fast_exp2(-x.y));
           pf[2 * i + 1] = make_float2(fast_exp2(-y.x), fast_exp2(-y.y));
-          pk[2 * i] = keep ? Elem<elem_t>::pack(pf[2 * i].x, pf[2 * i].y) : 0u;
-          pk[2 * i + 1] = keep ? Elem<elem_t>::pack(pf[2 * i + 1].x, pf[2 * i + 1].y) : 0u;
+          // a padding key row: its scores come from whatever sits in K there
+          pk[2 * i] = live ? Elem<elem_t>::pack(pf[2 * i].x, pf[2 * i].y) : 0u;
+          pk[2 * i + 1] = live ? Elem<elem_t>::pack(pf[2 * i + 1].x, pf[2 * i + 1].y) : 0u;
         }
       }
       ok = VSA_WARP_WAIT(bar(SK_P_EMPTY), ph ^ 1);
@@ -1003,8 +1001,8 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           const float4 d4 = s_lse[16 + i];       // delta: 64 floats behind the statistics
           const float2 x = mul2(pf[2 * i], fma2(word_pair(dvv + 4 * i), m1, make_float2(d4.x, d4.y)));      // -dS
           const float2 y = mul2(pf[2 * i + 1], fma2(word_pair(dvv + 4 * i + 2), m1, make_float2(d4.z, d4.w)));
-          pk[2 * i] = keep ? Elem<elem_t>::pack(x.x, x.y) : 0u;
-          pk[2 * i + 1] = keep ? Elem<elem_t>::pack(y.x, y.y) : 0u;
+          pk[2 * i] = live ? Elem<elem_t>::pack(x.x, x.y) : 0u;
+          pk[2 * i + 1] = live ? Elem<elem_t>::pack(y.x, y.y) : 0u;
         }
       }
       ok = VSA_WARP_WAIT(bar(SK_DS_EMPTY), ph ^ 1);
@@ -1039,8 +1037,10 @@ sparse_dkdv_split_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   } else if (warp == 0) {   // Q pairs with the statistics of their rows; a lane per tile and 64 head dims
     for (int p = 0; p < n_pairs; ++p) {
       const int s = p % Sm::q_stages, h = lane >> 1;
-      const bool second = 2 * p + 1 < n_tiles;             // otherwise it lies outside the tensor: zeros, and P = 2^-inf = 0
-      const long long row_a = tile_row(2 * p), row_b = second ? tile_row(2 * p + 1) : BH * Lq;
+      // The second half of an odd tail is the first one's Q again, with statistics that make P = 2^-inf = 0 of any score that the
+      // first half has a probability for; zero rows would make NaN of an infinite key.  Its dO lies outside the tensor, i.e. is zero.
+      const bool second = 2 * p + 1 < n_tiles;
+      const long long row_a = tile_row(2 * p), row_b = second ? tile_row(2 * p + 1) : row_a;
       ok = VSA_WARP_WAIT(bar(SK_Q_EMPTY + s), ((p / Sm::q_stages) & 1) ^ 1);
       if (!ok) break;
       const uint32_t st = base + Sm::stats + s * 1024 + lane * 4;
